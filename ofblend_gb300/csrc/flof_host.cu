@@ -304,6 +304,24 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
               float4 *p, float4 *q, const GT *g, int maxIter, const float *i1 = nullptr) {
   const double gb = sizeof(GT) == 8 ? 8.0 : 16.0;  // bytes of g per cell
   const double gpc = i1 ? 4.0 : gb;                 // bytes of g or i1 per cell in update/direction
+  if (resident_cells_ok(d) && maxIter > 0) {
+    // one cooperative launch; its blocks wait on one another, so the lock is
+    // held until it has ended
+    std::lock_guard<std::mutex> lock(resident_mutex());
+    bool done = false;
+    KLP(c, KC_RESIDENT, d.x, nint(d) * 64,
+        done = launch_cg_resident(x, r, p, q, g, d, k, c->st, c->dpart, maxIter, c->dev_err,
+                                  c->stream));
+    if (done) {
+      CK(cudaMemcpyAsync(c->st_h, c->st, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream));
+      sync(c);
+      // the bytes of every iteration: p, g and r read, q kept, then p, x and r
+      // read and p, x and r written
+      if (c->profiling && !c->recs.empty())
+        c->recs.back().bytes = (double)nint(d) * (128 + gb) * c->st_h->iters;
+      return;
+    }
+  }
   int it = 0;
   int chunk = 4;
   for (;;) {

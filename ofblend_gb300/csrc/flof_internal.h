@@ -98,13 +98,13 @@ struct Pool {
 enum KClass {
   KC_OTHER = 0, KC_ASSEMBLE, KC_MATVEC, KC_UPDATE, KC_DIRECTION, KC_COPYBACK, KC_BLUR,
   KC_PROJECT, KC_EXPOL, KC_ADVECT, KC_RESAMPLE, KC_LSDIFF, KC_REDUCE, KC_ELEMWISE, KC_BORDER,
-  KC_LOOKUP, KC_DEFORM, KC_BLEND, KC_EXPOL_MASK, KC_MG, KC_COUNT
+  KC_LOOKUP, KC_DEFORM, KC_BLEND, KC_EXPOL_MASK, KC_MG, KC_RESIDENT, KC_COUNT
 };
 inline const char *kc_names[KC_COUNT] = {
     "other", "of_assemble_init", "cg_matvec", "cg_update", "cg_direction", "of_copy_back",
     "gauss_blur", "project_cells", "expol_sweep", "advect", "resample", "ls_diff", "reduce",
     "elementwise", "border", "lookup_slice", "deform_twoway", "blend_slices", "expol_mask",
-    "mg_vcycle"};
+    "mg_vcycle", "cg_resident"};
 
 struct ProfRec {
   int cls;
@@ -324,7 +324,9 @@ inline void check_device_errors(flof_ctx *c) {
     CK(cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream));
     CK(cudaStreamSynchronize(c->stream));
     fail(FLOF_E_TIMEOUT, std::string("a bounded wait on ") +
-                             (e == flof::FLOF_DEV_ERR_TC_TIMEOUT ? "tensor-core MMAs" : "a TMA copy") +
+                             (e == flof::FLOF_DEV_ERR_TC_TIMEOUT     ? "tensor-core MMAs"
+                              : e == flof::FLOF_DEV_ERR_GRID_TIMEOUT ? "a grid barrier"
+                                                                     : "a TMA copy") +
                              " gave up (device error " + std::to_string(e) + ")");
   }
 }

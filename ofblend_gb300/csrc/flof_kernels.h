@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <vector>
 
 #include "flof_common.cuh"
@@ -107,6 +108,7 @@ struct CGState {
   int iters;
   int xpend;        // 1: x += alpha p of the last update is still to be applied
   unsigned int counter[4];
+  unsigned int gbar;  // arrivals at the resident solve's grid barriers
 };
 enum { CG_RUNNING = 0, CG_CONVERGED = 1, CG_FAILED_SIGMA = 2, CG_EARLY = 3,
        CG_MAXITER = 4 };
@@ -164,6 +166,24 @@ void launch_cg_update(float4 *r, const float4 *q, const BF4 *g, Dims4 d, OFConst
 void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const BF4 *g, Dims4 d,
                          OFConsts c, CGState *st, cudaStream_t s,
                          const CGTune &tu = CGTune());
+// ---- resident PCG (flof_resident.cu) -------------------------------------------
+// The whole iteration of a level whose cells fit the SMs as one cooperative
+// launch, from the state that the assembly or launch_cg_init_r left; it ends
+// with st->done set.  r is read only at the start and q is scratch.  False
+// (nothing launched) for a larger level, maxIter <= 0, or when the device
+// refuses the launch: the caller then chains the kernels above.  Its blocks
+// wait on one another, so two of them must not run at once: hold
+// resident_mutex() from the launch until the stream has been waited for.
+// part holds at least 7 doubles per SM.
+constexpr size_t RESIDENT_SMEM = 220 * 1024;  // shared memory for its cells, per SM
+bool resident_cells_ok(Dims4 d);
+std::mutex &resident_mutex();
+bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
+                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        cudaStream_t s);
+bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
+                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        cudaStream_t s);
 // ---- strict arithmetic (flof_strict.cu, FLOF_OPT_STRICT) ----------------------
 // The reference's PCG arithmetic operation for operation: double alpha and
 // beta, double multiply-and-add updates rounded once to float, and dot
@@ -288,6 +308,8 @@ void launch_expol_slab(const float4 *in, float4 *out, const float *mark, Dims4 d
 constexpr int FLOF_DEV_ERR_TMA_TIMEOUT = 1;
 // a tensor-core convolution block whose bounded wait on its MMAs ran out
 constexpr int FLOF_DEV_ERR_TC_TIMEOUT = 2;
+// a block of the resident PCG whose bounded wait at a grid barrier ran out
+constexpr int FLOF_DEV_ERR_GRID_TIMEOUT = 3;
 bool launch_gauss_tma(const float4 *src, float4 *dst, Dims4 d, int s, const float *wtab,
                       const float *wsum_dev, int zero_border, int *err, cudaStream_t st);
 // The TMA extrapolation sweep writes only the cells it updates (unmarked
