@@ -408,6 +408,29 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Launches a kernel with programmatic stream serialisation, so that its blocks
+// are scheduled while the previous kernel of the stream drains (the kernel
+// starts with pdl_wait).  Falls back to an ordinary launch if the attribute is
+// refused.
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*k)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
+                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k, args...) != cudaSuccess) {
+    cudaGetLastError();
+    k<<<grid, block, 0, s>>>(args...);
+  }
+}
+
 // ---- reductions -----------------------------------------------------------
 
 __device__ __forceinline__ double warp_sum(double v) {

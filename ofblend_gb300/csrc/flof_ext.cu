@@ -88,18 +88,10 @@ FLOF_API int flof_extrap4dLsSimple(flof_grid *phi, int distance, int inside) {
     need(distance >= 0 && distance < (1 << 20), "distance out of range");
     flof_ctx *c = phi->ctx;
     set_ctx_device(c);
-    const float direction = inside ? -1.f : 1.f;
-    DBuf tmp(c, (size_t)d.cells() * sizeof(int));
-    const double cells = (double)d.cells();
-    KLP(c, KC_ELEMWISE, d.x, cells * 8,
-        launch_extrap_mark(phi->f(), (int *)tmp.p, d, inside ? 1 : 0, c->stream));
-    KLP(c, KC_ELEMWISE, d.x, cells * 4, launch_extrap_layer((int *)tmp.p, d, c->stream));
-    for (int dd = 2; dd < 1 + distance; ++dd)
-      KLP(c, KC_ELEMWISE, d.x, cells * 8,
-          launch_extrap_step(phi->f(), (int *)tmp.p, d, dd, direction, c->stream));
-    KLP(c, KC_ELEMWISE, d.x, cells * 8,
-        launch_extrap_remaining(phi->f(), (const int *)tmp.p, d,
-                                direction * (float)(distance + 2), c->stream));
+    DBuf scratch(c, extrap_scratch_bytes(d));
+    KLP(c, KC_ELEMWISE, d.x, (double)d.cells() * 12,
+        launch_extrap(phi->f(), d, distance, inside ? 1 : 0, scratch.p, c->stream));
+    c->launches += distance > 1 ? distance + 1 : 2;  // beyond the one counted
   });
 }
 

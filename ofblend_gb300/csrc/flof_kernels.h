@@ -355,11 +355,10 @@ void launch_expol_sweep(const float4 *in, float4 *out, const float *mark,
 // srct; `slice` is scratch of X*Y*Z floats.
 void launch_repeat_frame(float *phi, Dims4 d, float srct, int t0, int t1, int bnd, float *slice,
                          cudaStream_t s);
-// extrap4dLsSimple steps; tmp holds X*Y*Z*T ints.
-void launch_extrap_mark(const float *phi, int *tmp, Dims4 d, int inside, cudaStream_t s);
-void launch_extrap_layer(int *tmp, Dims4 d, cudaStream_t s);
-void launch_extrap_step(float *phi, int *tmp, Dims4 d, int dd, float direction, cudaStream_t s);
-void launch_extrap_remaining(float *phi, const int *tmp, Dims4 d, float value, cudaStream_t s);
+// extrap4dLsSimple (every extent at least 3): distance + 2 launches; scratch
+// holds extrap_scratch_bytes(d) bytes.
+size_t extrap_scratch_bytes(Dims4 d);
+void launch_extrap(float *phi, Dims4 d, int distance, int inside, void *scratch, cudaStream_t s);
 // one knSimpleBlurSpecial pass a -> tmp over a 3D (Z > 1) or 2D (Z == 1) grid
 void launch_simple_blur_special(const float *a, float *tmp, int X, int Y, int Z, float thresh,
                                 int bord, cudaStream_t s);

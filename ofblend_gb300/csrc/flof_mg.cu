@@ -811,29 +811,6 @@ k_mg_judge(const float4 *__restrict__ x, const float4 *__restrict__ b,
   }
 }
 
-// Launches an MG kernel with programmatic stream serialisation: its blocks
-// are scheduled while the previous kernel drains and wait in pdl_wait until
-// that kernel's writes are visible.  Falls back to an ordinary launch if the
-// attribute is refused.
-template <typename... KArgs, typename... Args>
-void mg_launch(void (*k)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
-               Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, k, args...) != cudaSuccess) {
-    cudaGetLastError();
-    k<<<grid, block, 0, s>>>(args...);
-  }
-}
-
 inline BoxDecoder interior_box(Dims4 d) { return make_decoder(d.x - 2, d.y - 2, d.z - 2, 1, 1, 1, 1); }
 inline uint32_t interior_n(Dims4 d) {
   if (d.x < 3 || d.y < 3 || d.z < 3 || d.t < 3) return 0;
@@ -861,10 +838,10 @@ std::vector<Dims4> mg_level_dims(Dims4 d) {
 void launch_mg_build(const float4 *g, Dims4 d, const MGLevelPtrs *L, int nl, const OFConsts &c,
                      const MGParams &mp, const CGState *st, cudaStream_t s) {
   if (nl <= 0) return;
-  mg_launch(k_mg_build1, grid_for(L[0].m.cells(), MT, 8), MT, s, g, d, L[0].m, L[0].G, L[0].cpl,
+  launch_pdl(k_mg_build1, grid_for(L[0].m.cells(), MT, 8), MT, s, g, d, L[0].m, L[0].G, L[0].cpl,
             L[0].dinv, c.wSmooth, c.wEnergy, mp.lambda, st);
   for (int l = 1; l < nl; ++l)
-    mg_launch(k_mg_build, grid_for(L[l].m.cells(), MT, 8), MT, s, L[l - 1].G, L[l - 1].cpl,
+    launch_pdl(k_mg_build, grid_for(L[l].m.cells(), MT, 8), MT, s, L[l - 1].G, L[l - 1].cpl,
               L[l - 1].m, L[l].m, L[l].G, L[l].cpl, L[l].dinv, mp.lambda, st);
 }
 
@@ -877,11 +854,11 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
   const float c0 = c.diag, wS = c.wSmooth;
   int nl_ = 0;
   if (!pre_done) {
-    mg_launch(k_mg0_pre, nb0, MT, s, b0, g, x0, d, bx, nint, c0, mp.omega0, st);
+    launch_pdl(k_mg0_pre, nb0, MT, s, b0, g, x0, d, bx, nint, c0, mp.omega0, st);
     ++nl_;
   }
   if (nl == 0) {
-    mg_launch(k_mg0_post, nb0, MT, s, b0, g, x0, z, d, bx, nint, c0, wS, mp.omega0, st, dpart,
+    launch_pdl(k_mg0_post, nb0, MT, s, b0, g, x0, z, d, bx, nint, c0, wS, mp.omega0, st, dpart,
               init);
     if (launches) *launches += nl_;  // the caller counts one
     return;
@@ -890,28 +867,28 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
     const int nbx = (d.x - 2 + 31) / 32;
     const int tchunks = (L[0].m.t + RR_TP - 1) / RR_TP;
     const long long nblk = (long long)nbx * L[0].m.y * L[0].m.z * tchunks;
-    mg_launch(k_mg0_resid_restrict, (unsigned)nblk, RR_NT, s, b0, g, x0, L[0].b, d, L[0].m, nbx,
+    launch_pdl(k_mg0_resid_restrict, (unsigned)nblk, RR_NT, s, b0, g, x0, L[0].b, d, L[0].m, nbx,
               c0, wS, st);
     ++nl_;
   }
   for (int l = 0; l + 1 < nl; ++l) {
     const uint32_t n = (uint32_t)L[l].m.cells();
     const int nb = grid_for(n, MT, 8);
-    mg_launch(k_mgc_pre, nb, MT, s, L[l].b, L[l].dinv, L[l].x, n, mp.omegac, st);
-    mg_launch(k_mgc_resid, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].x, L[l].r, L[l].m, st);
-    mg_launch(k_mgc_restrict, grid_for(L[l + 1].m.cells(), MT, 8), MT, s, L[l].r, L[l + 1].b,
+    launch_pdl(k_mgc_pre, nb, MT, s, L[l].b, L[l].dinv, L[l].x, n, mp.omegac, st);
+    launch_pdl(k_mgc_resid, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].x, L[l].r, L[l].m, st);
+    launch_pdl(k_mgc_restrict, grid_for(L[l + 1].m.cells(), MT, 8), MT, s, L[l].r, L[l + 1].b,
               L[l].m, L[l + 1].m, st);
     nl_ += 3;
   }
   const MGLevelPtrs &B = L[nl - 1];
-  mg_launch(k_mgc_coarsest, 1, MG_COARSEST, s, B.b, B.G, B.cpl, B.dinv, B.x, B.m, mp.omegac,
+  launch_pdl(k_mgc_coarsest, 1, MG_COARSEST, s, B.b, B.G, B.cpl, B.dinv, B.x, B.m, mp.omegac,
             mp.coarse_sweeps, st);
   ++nl_;
   for (int l = nl - 2; l >= 0; --l) {
     const uint32_t n = (uint32_t)L[l].m.cells();
     const int nb = grid_for(n, MT, 8);
-    mg_launch(k_mgc_prolong, nb, MT, s, L[l].x, L[l + 1].x, L[l].m, L[l + 1].m, st);
-    mg_launch(k_mgc_post, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].dinv, L[l].x, L[l].r, L[l].m,
+    launch_pdl(k_mgc_prolong, nb, MT, s, L[l].x, L[l + 1].x, L[l].m, L[l + 1].m, st);
+    launch_pdl(k_mgc_post, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].dinv, L[l].x, L[l].r, L[l].m,
               mp.omegac, st);
     // the post-smoothed iterate is in r; it becomes this level's x
     std::swap(L[l].x, L[l].r);
@@ -921,8 +898,8 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
     const BoxDecoder bxyz = make_decoder(d.x - 2, d.y - 2, d.z - 2, 1, 1, 1, 0);
     const uint32_t nxyz = (uint32_t)((long long)(d.x - 2) * (d.y - 2) * (d.z - 2));
     const int tchunks = (d.t - 2 + MG_TT - 1) / MG_TT;
-    mg_launch(k_mg0_prolong, nb0, MT, s, x0, L[0].x, d, bx, nint, L[0].m, st);
-    mg_launch(k_mg0_post_tw, grid_for((long long)nxyz * tchunks, MT, 8), MT, s, b0, g, x0, z, d,
+    launch_pdl(k_mg0_prolong, nb0, MT, s, x0, L[0].x, d, bx, nint, L[0].m, st);
+    launch_pdl(k_mg0_post_tw, grid_for((long long)nxyz * tchunks, MT, 8), MT, s, b0, g, x0, z, d,
               bxyz, nxyz, tchunks, c0, wS, mp.omega0, st, dpart, init);
     nl_ += 2;
   }
@@ -932,7 +909,7 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
 void launch_mgcg_update(float4 *x, float4 *r, const float4 *p, const float4 *q, Dims4 d,
                         CGState *st, float *fpart, int maxIter, cudaStream_t s) {
   const uint32_t nint = interior_n(d);
-  mg_launch(k_mgcg_update, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, r, p, q, d,
+  launch_pdl(k_mgcg_update, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, r, p, q, d,
             interior_box(d), nint, st, fpart, maxIter);
 }
 void launch_mgcg_update_pre(float4 *x, float4 *r, const float4 *p, const float4 *q,
@@ -942,11 +919,11 @@ void launch_mgcg_update_pre(float4 *x, float4 *r, const float4 *p, const float4 
   const uint32_t nint = interior_n(d);
   const int nb = grid_for(nint > 0 ? nint : 1, MT, 8);
   if (i1)
-    mg_launch(k_mgcg_update_pre<GradFromI1>, nb, MT, s, x, r, p, q,
+    launch_pdl(k_mgcg_update_pre<GradFromI1>, nb, MT, s, x, r, p, q,
               GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, x0, d, interior_box(d), nint, c.diag,
               mp.omega0, st, fpart, maxIter);
   else
-    mg_launch(k_mgcg_update_pre<GradLoad>, nb, MT, s, x, r, p, q, GradLoad{g}, x0, d,
+    launch_pdl(k_mgcg_update_pre<GradLoad>, nb, MT, s, x, r, p, q, GradLoad{g}, x0, d,
               interior_box(d), nint, c.diag, mp.omega0, st, fpart, maxIter);
 }
 
@@ -954,14 +931,14 @@ void launch_mg_judge(const float4 *x, const float4 *b, const float4 *g, float4 *
                      const OFConsts &c, float *fpart, unsigned int *counter, float *rmax,
                      cudaStream_t s) {
   const uint32_t nint = interior_n(d);
-  mg_launch(k_mg_judge, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, b, g, r, d, interior_box(d),
+  launch_pdl(k_mg_judge, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, b, g, r, d, interior_box(d),
             nint, c.diag, c.wSmooth, fpart, counter, rmax);
 }
 
 void launch_mgcg_direction(float4 *p, const float4 *z, Dims4 d, const CGState *st, int init,
                            cudaStream_t s) {
   const uint32_t nint = interior_n(d);
-  mg_launch(k_mgcg_direction, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, p, z, d, interior_box(d),
+  launch_pdl(k_mgcg_direction, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, p, z, d, interior_box(d),
             nint, st, init);
 }
 
