@@ -50,9 +50,8 @@ void interpol_grid(flof_ctx *c, float *target, Dims4 td, const float *source, Di
 float vec_max_norm(flof_ctx *c, const float4 *v, Dims4 d) {
   KLP(c, KC_REDUCE, d.x, d.cells() * 16,
       launch_reduce_minmax((const float *)v, d.cells(), 4, 0, c->fpart, c->counter + 4,
-                             c->fres + 0, c->stream));
-  const float m2 = read_f(c, c->fres + 0);
-  return sqrtf(m2);
+                             c->fres + 0, c->stream, next_post(c)));
+  return sqrtf(wait_value(c));
 }
 
 // advectCflTemplate<Grid4d<int>,...> (optflow4d.cpp:2170-2180) ->
@@ -93,14 +92,15 @@ void advect_cfl(flof_ctx *c, Dims4 d, float cfl, const float4 *vel, float *grid,
 // calcLsDiffTempl (optflow4d.cpp:895-927), synchronising.
 float ls_diff(flof_ctx *c, const float *i0, const float *i1, float *out, Dims4 d, float corr,
               int bnd) {
-  if (c->strict)
+  if (c->strict) {
     KLP(c, KC_LSDIFF, d.x, d.cells() * 8,
         launch_strict_ls_diff(i0, i1, out, d, corr, bnd, c->dres + 0, c->fres + 1, c->stream));
-  else
-    KLP(c, KC_LSDIFF, d.x, d.cells() * 8,
-        launch_ls_diff(i0, i1, out, d, corr, bnd, c->dpart, c->counter + 5, c->dres + 0,
-                         c->fres + 1, c->stream));
-  return read_f(c, c->fres + 1);
+    return read_f(c, c->fres + 1);
+  }
+  KLP(c, KC_LSDIFF, d.x, d.cells() * 8,
+      launch_ls_diff(i0, i1, out, d, corr, bnd, c->dpart, c->counter + 5, c->dres + 0, c->fres + 1,
+                     c->stream, next_post(c)));
+  return wait_value(c);
 }
 
 // In-bounds weight sums of knGaussianBlur by clipping pattern: per axis the
@@ -311,10 +311,14 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
     bool done = false;
     KLP(c, KC_RESIDENT, d.x, nint(d) * 64,
         done = launch_cg_resident(x, r, p, q, g, d, k, c->st, c->dpart, maxIter, c->dev_err,
-                                  c->stream));
+                                  next_post(c), c->stream));
     if (done) {
-      CK(cudaMemcpyAsync(c->st_h, c->st, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream));
-      sync(c);
+      wait_post(c, &c->hres->cg_seq);
+      c->st_h->done = c->hres->done;
+      c->st_h->iters = c->hres->iters;
+      c->st_h->resMax = c->hres->resMax;
+      c->st_h->retResidual = c->hres->retResidual;
+      c->st_h->resIni = c->hres->resIni;
       // the bytes of every iteration: p, g and r read, q kept, then p, x and r
       // read and p, x and r written
       if (c->profiling && !c->recs.empty())
@@ -906,10 +910,11 @@ FLOF_API int flof_ctx_create(int device, flof_ctx **out) {
       CK(cudaMallocHost(&c->st_h, sizeof(CGState)));
       CK(cudaMalloc(&c->dpart, sizeof(double) * maxBlocks));
       CK(cudaMalloc(&c->fpart, sizeof(float) * maxBlocks));
-      CK(cudaMalloc(&c->cfl_flag, sizeof(int)));
-      CK(cudaMemset(c->cfl_flag, 0, sizeof(int)));
-      CK(cudaMalloc(&c->dev_err, sizeof(int)));
-      CK(cudaMemset(c->dev_err, 0, sizeof(int)));
+      CK(cudaHostAlloc(&c->hres, sizeof(HostResult), cudaHostAllocMapped));
+      memset((void *)c->hres, 0, sizeof(HostResult));
+      CK(cudaHostGetDevicePointer((void **)&c->hres_d, c->hres, 0));
+      c->cfl_flag = &c->hres_d->cfl_flag;
+      c->dev_err = &c->hres_d->dev_err;
       CK(cudaMalloc(&c->counter, sizeof(unsigned int) * 8));
       CK(cudaMemset(c->counter, 0, sizeof(unsigned int) * 8));
       CK(cudaMalloc(&c->fres, sizeof(float) * 16));
@@ -951,8 +956,7 @@ FLOF_API int flof_ctx_destroy(flof_ctx *c) {
   cudaFree(c->dpart);
   cudaFree(c->fpart);
   cudaFree(c->counter);
-  cudaFree(c->cfl_flag);
-  cudaFree(c->dev_err);
+  cudaFreeHost(c->hres);
   cudaFree(c->fres);
   cudaFree(c->dres);
   cudaFreeHost(c->fres_h);
@@ -1415,15 +1419,12 @@ FLOF_API int flof_opticalFlowMultiscale4d(flof_ctx *c, flof_grid *vel, const flo
       // speculative pass: CFL substep counts checked on the device
       DBuf vel_in(c, vel->bytes());
       CK(cudaMemcpyAsync(vel_in.p, vel->d, vel->bytes(), cudaMemcpyDeviceToDevice, c->stream));
-      CK(cudaMemsetAsync(c->cfl_flag, 0, sizeof(int), c->stream));
+      volatile int *cfl_flag = &c->hres->cfl_flag;
+      *cfl_flag = 0;  // nothing in flight writes it
       c->cfl_sync = c->cfl_force_sync;
       e = multiscale(c, vel->D(), vel->v(), i0->f(), i1->f(), m, pp.level);
-      int flag = 0;
-      CK(cudaMemcpyAsync(c->fres_h + 8, c->cfl_flag, sizeof(int), cudaMemcpyDeviceToHost,
-                         c->stream));
       CK(cudaStreamSynchronize(c->stream));
-      memcpy(&flag, c->fres_h + 8, sizeof(int));
-      if (flag) {
+      if (*cfl_flag) {
         // some advection needed more than one CFL substep: redo the call
         // with host-side substep counts
         memset(&local, 0, sizeof(local));

@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include <array>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <new>
@@ -138,6 +139,9 @@ struct flof_ctx {
   float *fres = nullptr;            // 16 device scalars
   double *dres = nullptr;
   float *fres_h = nullptr;          // pinned
+  flof::HostResult *hres = nullptr;    // pinned, written by kernels
+  flof::HostResult *hres_d = nullptr;  // the device's address of it
+  unsigned int hseq = 0;               // the last result asked for
   double *dres_h = nullptr;
   long long launches = 0;
   int syncs = 0;
@@ -146,8 +150,8 @@ struct flof_ctx {
   // 0: CFL substep counts are checked on the device (one substep assumed,
   // exceptions flagged in cfl_flag); 1: the host reads max |v| each time.
   int cfl_sync = 0;
-  int *cfl_flag = nullptr;
-  int *dev_err = nullptr;  // device error word written by bounded waits
+  int *cfl_flag = nullptr;  // words of hres_d
+  int *dev_err = nullptr;   // written by bounded waits
   int cfl_force_sync = 0;
   int profiling = 0;
   std::map<std::pair<uint32_t, int>, float *> wsum_cache;  // (sigma bits, radius)
@@ -295,6 +299,32 @@ inline void sync(flof_ctx *c) {
   c->syncs++;
 }
 
+void check_device_errors(flof_ctx *c);
+
+// A place for the next result that a kernel posts to the host.
+inline flof::HostPost next_post(flof_ctx *c) { return flof::HostPost{c->hres_d, ++c->hseq}; }
+
+// Waits on the host for the result with sequence number c->hseq in *seq (a
+// member of c->hres).  A stream that ended or failed without posting it
+// raises the device error word or the CUDA error.
+inline void wait_post(flof_ctx *c, const unsigned int *seq) {
+  const volatile unsigned int *s = seq;
+  for (unsigned n = 1; *s != c->hseq; ++n) {
+    if (n % 1024) continue;
+    const cudaError_t e = cudaStreamQuery(c->stream);
+    if (e == cudaErrorNotReady) continue;
+    cuda_check(e, "waiting for a kernel's result");
+    if (*s == c->hseq) break;
+    check_device_errors(c);
+    fail(FLOF_E_CUDA, "a kernel ended without its result");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  c->syncs++;
+}
+inline float wait_value(flof_ctx *c) {
+  wait_post(c, &c->hres->seq);
+  return c->hres->value;
+}
 inline float read_f(flof_ctx *c, const float *dev) {
   CK(cudaMemcpyAsync(c->fres_h, dev, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   sync(c);
@@ -314,15 +344,13 @@ inline int trunc_d(double v) {
   return (int)v;
 }
 
-// Reads and clears the device error word (after the stream has drained).
+// Waits for the stream, then reads and clears the device error word.
 inline void check_device_errors(flof_ctx *c) {
-  CK(cudaMemcpyAsync(c->fres_h + 9, c->dev_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  int e = 0;
-  memcpy(&e, c->fres_h + 9, sizeof(int));
+  volatile int *w = &c->hres->dev_err;
+  const int e = *w;
   if (e) {
-    CK(cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    *w = 0;
     fail(FLOF_E_TIMEOUT, std::string("a bounded wait on ") +
                              (e == flof::FLOF_DEV_ERR_TC_TIMEOUT     ? "tensor-core MMAs"
                               : e == flof::FLOF_DEV_ERR_GRID_TIMEOUT ? "a grid barrier"

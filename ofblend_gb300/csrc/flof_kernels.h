@@ -37,18 +37,41 @@ void launch_set_bound_neumann(float *a, Dims4 d, int nc, int w, cudaStream_t s);
 // zero every cell outside isInBounds(resetBnd)
 void launch_reset_outside(float4 *a, Dims4 d, int resetBnd, cudaStream_t s);
 
+// ---- results for the host ------------------------------------------------------
+// Scalars that the host waits for, written by the kernel that forms them into
+// pinned host memory: the value first, then (after a system fence) the
+// sequence number that the host polls, so that no copy and no stream
+// synchronisation stands between the kernel and the host's next launch (a
+// copy and a synchronisation cost about 17 us, this about 5).  cfl_flag and
+// dev_err are plain words that kernels set when something is wrong.
+struct HostResult {
+  int cfl_flag;  // an advection needed more than one CFL substep
+  int dev_err;   // FLOF_DEV_ERR_* of a bounded wait that gave up
+  float value;   // a reduction's result
+  unsigned int seq;
+  int done, iters;  // the resident PCG's outcome (CGState)
+  float resMax, retResidual;
+  double resIni;
+  unsigned int cg_seq;
+};
+// Where a kernel sends a result; hr null: nowhere.
+struct HostPost {
+  HostResult *hr = nullptr;
+  unsigned int seq = 0;
+};
+
 // ---- reductions (result written to device memory) ---------------------------
 // which: 0 max, 1 min.  For nc == 4 the value is max/min |v|^2 (no sqrt).
 // `partials` holds grid_for(...) floats, `counter` one zeroed uint.
 void launch_reduce_minmax(const float *a, long long ncell, int nc, int which,
                           float *partials, unsigned int *counter, float *result,
-                          cudaStream_t s);
+                          cudaStream_t s, HostPost post = HostPost());
 // calcLsDiffTempl sum over the bnd box (double), scaled as the reference
 // does; result as double and as float.
 void launch_ls_diff(const float *i0, const float *i1, float *out, Dims4 d,
                     float correction, int bnd, double *partials,
                     unsigned int *counter, double *result_d, float *result_f,
-                    cudaStream_t s);
+                    cudaStream_t s, HostPost post = HostPost());
 int ls_diff_blocks(Dims4 d, int bnd);
 
 // ---- resampling / advection ---------------------------------------------------
@@ -169,7 +192,7 @@ void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const BF4 *g, Di
 // ---- resident PCG (flof_resident.cu) -------------------------------------------
 // The whole iteration of a level whose cells fit the SMs as one cooperative
 // launch, from the state that the assembly or launch_cg_init_r left; it ends
-// with st->done set.  r is read only at the start and q is scratch.  False
+// with st->done set and the outcome posted to the host.  r is read only at the start and q is scratch.  False
 // (nothing launched) for a larger level, maxIter <= 0, or when the device
 // refuses the launch: the caller then chains the kernels above.  Its blocks
 // wait on one another, so two of them must not run at once: hold
@@ -180,10 +203,10 @@ bool resident_cells_ok(Dims4 d);
 std::mutex &resident_mutex();
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        cudaStream_t s);
+                        HostPost post, cudaStream_t s);
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        cudaStream_t s);
+                        HostPost post, cudaStream_t s);
 // ---- strict arithmetic (flof_strict.cu, FLOF_OPT_STRICT) ----------------------
 // The reference's PCG arithmetic operation for operation: double alpha and
 // beta, double multiply-and-add updates rounded once to float, and dot

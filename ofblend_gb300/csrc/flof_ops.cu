@@ -206,10 +206,17 @@ void launch_reset_outside(float4 *a, Dims4 d, int resetBnd, cudaStream_t s) {
 // Reductions (grid4d.cpp:142-172, :263-285)
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ void post_value(const HostPost &post, float v) {
+  if (!post.hr) return;
+  post.hr->value = v;
+  __threadfence_system();
+  *(volatile unsigned int *)&post.hr->seq = post.seq;
+}
+
 template <int WHICH>
 __global__ void k_reduce_minmax(const float *__restrict__ a, long long n, int nc,
                                 float *partials, unsigned int *counter,
-                                float *result) {
+                                float *result, HostPost post) {
   __shared__ float sh[NT / 32];
   float acc = WHICH == 0 ? -FLT_MAX : FLT_MAX;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -237,40 +244,58 @@ __global__ void k_reduce_minmax(const float *__restrict__ a, long long n, int nc
     if (threadIdx.x == 0) {
       *result = m;
       *counter = 0;
+      post_value(post, m);
     }
   }
 }
 void launch_reduce_minmax(const float *a, long long ncell, int nc, int which,
                           float *partials, unsigned int *counter, float *result,
-                          cudaStream_t s) {
+                          cudaStream_t s, HostPost post) {
   const int nb = grid_for(ncell, NT, 4);
   if (which == 0)
-    k_reduce_minmax<0><<<nb, NT, 0, s>>>(a, ncell, nc, partials, counter, result);
+    k_reduce_minmax<0><<<nb, NT, 0, s>>>(a, ncell, nc, partials, counter, result, post);
   else
-    k_reduce_minmax<1><<<nb, NT, 0, s>>>(a, ncell, nc, partials, counter, result);
+    k_reduce_minmax<1><<<nb, NT, 0, s>>>(a, ncell, nc, partials, counter, result, post);
 }
 
-// calcLsDiffTempl (optflow4d.cpp:895-927)
-__global__ void k_ls_diff(const float *__restrict__ i0, const float *__restrict__ i1,
-                          float *out, Dims4 d, BoxDecoder bx, uint32_t nbox,
-                          float correction, double scale, double *partials,
-                          unsigned int *counter, double *result_d,
-                          float *result_f) {
+// calcLsDiffTempl (optflow4d.cpp:895-927).  Four cells per trip, all loads
+// first: a small grid then needs a quarter of the blocks, whose partials the
+// last block sums, and still has its loads in flight together.
+constexpr int LSD_CPT = 4;
+__global__ void __launch_bounds__(NT)
+k_ls_diff(const float *__restrict__ i0, const float *__restrict__ i1, float *out, Dims4 d,
+          BoxDecoder bx, uint32_t nbox, float correction, double scale, double *partials,
+          unsigned int *counter, double *result_d, float *result_f, HostPost post) {
   __shared__ double sh[NT / 32];
   double acc = 0.0;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nbox;
-       q += gridDim.x * blockDim.x) {
-    int i, j, k, l;
-    bx.decode(q, i, j, k, l);
-    const idx_t id = d.index(i, j, k, l);
-    const float a = __ldg(i0 + id), b = __ldg(i1 + id);
-    if ((a < 0.f && b < 0.f) || (a >= 0.f && b >= 0.f)) {
-      if (out) out[id] = 0.f;
-    } else {
-      float dd = fabsf(a - b) * correction;
-      if (dd > 1.f) dd = 1.f;
-      acc += (double)dd;
-      if (out) out[id] = dd;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nbox; q += LSD_CPT * stride) {
+    idx_t id[LSD_CPT];
+    float a[LSD_CPT], b[LSD_CPT];
+    // nbox + 3 stride stays far below 2^32
+#pragma unroll
+    for (int m = 0; m < LSD_CPT; ++m) {
+      const uint32_t n = q + m * stride;
+      id[m] = -1;
+      a[m] = b[m] = 0.f;  // equal signs: no contribution
+      if (n < nbox) {
+        int i, j, k, l;
+        bx.decode(n, i, j, k, l);
+        id[m] = d.index(i, j, k, l);
+        a[m] = __ldg(i0 + id[m]);
+        b[m] = __ldg(i1 + id[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < LSD_CPT; ++m) {
+      if ((a[m] < 0.f && b[m] < 0.f) || (a[m] >= 0.f && b[m] >= 0.f)) {
+        if (out && id[m] >= 0) out[id[m]] = 0.f;
+      } else {
+        float dd = fabsf(a[m] - b[m]) * correction;
+        if (dd > 1.f) dd = 1.f;
+        acc += (double)dd;
+        if (out) out[id[m]] = dd;
+      }
     }
   }
   double b = block_sum<NT>(acc, sh);
@@ -286,18 +311,19 @@ __global__ void k_ls_diff(const float *__restrict__ i0, const float *__restrict_
       *result_d = accu;
       *result_f = (float)accu;
       *counter = 0;
+      post_value(post, (float)accu);
     }
   }
 }
 int ls_diff_blocks(Dims4 d, int bnd) {
   const long long ex = d.x - 2 * bnd, ey = d.y - 2 * bnd, ez = d.z - 2 * bnd, et = d.t - 2 * bnd;
   const long long nb = (ex > 0 && ey > 0 && ez > 0 && et > 0) ? ex * ey * ez * et : 1;
-  return grid_for(nb, NT, 4);
+  return grid_for((nb + LSD_CPT - 1) / LSD_CPT, NT, 4);
 }
 void launch_ls_diff(const float *i0, const float *i1, float *out, Dims4 d,
                     float correction, int bnd, double *partials,
                     unsigned int *counter, double *result_d, float *result_f,
-                    cudaStream_t s) {
+                    cudaStream_t s, HostPost post) {
   const int ex = d.x - 2 * bnd, ey = d.y - 2 * bnd, ez = d.z - 2 * bnd, et = d.t - 2 * bnd;
   long long nbox = (ex > 0 && ey > 0 && ez > 0 && et > 0) ? (long long)ex * ey * ez * et : 0;
   BoxDecoder bx = make_decoder(ex > 0 ? ex : 1, ey > 0 ? ey : 1, ez > 0 ? ez : 1, bnd, bnd, bnd, bnd);
@@ -310,7 +336,7 @@ void launch_ls_diff(const float *i0, const float *i1, float *out, Dims4 d,
   const double scale = 1. / (double)cnt;
   k_ls_diff<<<ls_diff_blocks(d, bnd), NT, 0, s>>>(i0, i1, out, d, bx, (uint32_t)nbox,
                                                   correction, scale, partials, counter,
-                                                  result_d, result_f);
+                                                  result_d, result_f, post);
 }
 
 // ---------------------------------------------------------------------------

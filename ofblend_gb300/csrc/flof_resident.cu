@@ -86,20 +86,34 @@ __device__ __forceinline__ float quotient(double a, double b) {
   return (float)(a / b);
 }
 
+__device__ __forceinline__ void post_outcome(const HostPost &post, const CGState *st) {
+  HostResult *h = post.hr;
+  h->done = st->done;
+  h->iters = st->iters;
+  h->resMax = st->resMax;
+  h->retResidual = st->retResidual;
+  h->resIni = st->resIni;
+  __threadfence_system();
+  *(volatile unsigned int *)&h->cg_seq = post.seq;
+}
+
 // NTH threads; K cells per thread at most when QREG (A p in registers,
 // otherwise in qg); GS: the gradient is kept in shared memory too.
 template <int NTH, int K, bool QREG, bool GS, class GT>
 __global__ void __launch_bounds__(NTH, 1)
 k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
               const GT *__restrict__ g, Dims4 d, BoxDecoder bx, uint32_t nint, uint32_t per,
-              OFConsts c, CGState *st, double *part, int maxIter, int *err) {
+              OFConsts c, CGState *st, double *part, int maxIter, int *err, HostPost post) {
   extern __shared__ float4 res_sm[];
   __shared__ FF shff[3][NTH / 32];
   __shared__ float shm[NTH / 32];
   __shared__ double fin[5];
   __shared__ float ab[2];
   __shared__ int ok, stop;
-  if (st->done != CG_RUNNING) return;  // the same for every block
+  if (st->done != CG_RUNNING) {  // the same for every block
+    if (blockIdx.x == 0 && threadIdx.x == 0) post_outcome(post, st);
+    return;
+  }
   const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, nint);
   const int G = gridDim.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float4 *rs = res_sm, *gsm = res_sm + per;
@@ -185,7 +199,7 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
     }
     target += G;
     if (!grid_barrier(&st->gbar, target, &ok)) {
-      if (threadIdx.x == 0) atomicExch(err, FLOF_DEV_ERR_GRID_TIMEOUT);
+      if (threadIdx.x == 0) *(volatile int *)err = FLOF_DEV_ERR_GRID_TIMEOUT;
       return;
     }
     // the sums over the blocks: p.q, q.z, q.M^-1 q of this iteration, z.r and
@@ -227,6 +241,7 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
         st->iters = it;
         st->resMax = (float)fin[4];
         st->retResidual = (float)(fin[4] / st->resIni);
+        post_outcome(post, st);
       }
       return;
     }
@@ -284,7 +299,7 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
     }
     target += G;
     if (!grid_barrier(&st->gbar, target, &ok)) {
-      if (threadIdx.x == 0) atomicExch(err, FLOF_DEV_ERR_GRID_TIMEOUT);
+      if (threadIdx.x == 0) *(volatile int *)err = FLOF_DEV_ERR_GRID_TIMEOUT;
       return;
     }
   }
@@ -293,7 +308,7 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
 template <int NTH, int K, bool QREG, bool GS, class GT>
 bool launch_one(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d, uint32_t nint,
                 uint32_t per, OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                cudaStream_t s) {
+                HostPost post, cudaStream_t s) {
   auto k = k_cg_resident<NTH, K, QREG, GS, GT>;
   constexpr size_t per_cell = GS ? 32 : 16;
   // the largest dynamic shared memory that leaves one block per SM, asked for
@@ -317,7 +332,7 @@ bool launch_one(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d
   BoxDecoder bx = make_decoder(d.x - 2, d.y - 2, d.z - 2, 1, 1, 1, 1);
   const float4 *r0 = r;
   const unsigned grid = (nint + per - 1) / per;
-  void *args[] = {&x, &r0, &p, &q, &g, &d, &bx, &nint, &per, &c, &st, &part, &maxIter, &err};
+  void *args[] = {&x, &r0, &p, &q, &g, &d, &bx, &nint, &per, &c, &st, &part, &maxIter, &err, &post};
   if (cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(NTH), args, smem, s) !=
       cudaSuccess) {
     cudaGetLastError();
@@ -328,7 +343,7 @@ bool launch_one(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d
 
 template <class GT>
 bool launch_any(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d, OFConsts c,
-                CGState *st, double *part, int maxIter, int *err, cudaStream_t s) {
+                CGState *st, double *part, int maxIter, int *err, HostPost post, cudaStream_t s) {
   if (!resident_cells_ok(d) || maxIter <= 0) return false;
   const uint32_t n = (uint32_t)((long long)(d.x - 2) * (d.y - 2) * (d.z - 2) * (d.t - 2));
   const uint32_t sms = (uint32_t)sm_count();
@@ -338,12 +353,16 @@ bool launch_any(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d
   // then A p and the gradient out of registers and shared memory.
   uint32_t per = (n + sms - 1) / sms;
   if (per <= 256)
-    return launch_one<256, 1, true, true>(x, r, p, q, g, d, n, 256, c, st, part, maxIter, err, s);
+    return launch_one<256, 1, true, true>(x, r, p, q, g, d, n, 256,
+        c, st, part, maxIter, err, post, s);
   if (per <= 1024)
-    return launch_one<512, 2, true, true>(x, r, p, q, g, d, n, per, c, st, part, maxIter, err, s);
+    return launch_one<512, 2, true, true>(x, r, p, q, g, d, n, per,
+        c, st, part, maxIter, err, post, s);
   if (per <= 6144)
-    return launch_one<1024, 6, true, true>(x, r, p, q, g, d, n, per, c, st, part, maxIter, err, s);
-  return launch_one<1024, 1, false, false>(x, r, p, q, g, d, n, per, c, st, part, maxIter, err, s);
+    return launch_one<1024, 6, true, true>(x, r, p, q, g, d, n, per,
+        c, st, part, maxIter, err, post, s);
+  return launch_one<1024, 1, false, false>(x, r, p, q, g, d, n, per, c, st, part, maxIter, err,
+                                           post, s);
 }
 
 }  // namespace
@@ -361,13 +380,13 @@ std::mutex &resident_mutex() {
 
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        cudaStream_t s) {
-  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, s);
+                        HostPost post, cudaStream_t s) {
+  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, post, s);
 }
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        cudaStream_t s) {
-  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, s);
+                        HostPost post, cudaStream_t s) {
+  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, post, s);
 }
 
 }  // namespace flof

@@ -166,7 +166,7 @@ k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
     const bool ok = mbar_wait_bounded(&bar[p % NS], (p / NS) & 1);
     if (__syncthreads_or(!ok)) {
       if (threadIdx.x == 0) {
-        atomicExch(err, FLOF_DEV_ERR_TMA_TIMEOUT);
+        *(volatile int *)err = FLOF_DEV_ERR_TMA_TIMEOUT;
         // let the copies in flight land before the block's shared memory goes
         for (int r = p; r < NP && r < p + NS; ++r) mbar_wait_bounded(&bar[r % NS], (r / NS) & 1);
       }
@@ -364,7 +364,7 @@ k_expol_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
       }
       if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) {
-          atomicExch(err, FLOF_DEV_ERR_TMA_TIMEOUT);
+          *(volatile int *)err = FLOF_DEV_ERR_TMA_TIMEOUT;
           for (int r = p; r < NP && r < p + NS; ++r) mbar_wait_bounded(&bar[r % NS], (r / NS) & 1);
         }
         __syncthreads();
@@ -519,7 +519,7 @@ k_expol_sep_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst
       }
       if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) {
-          atomicExch(err, FLOF_DEV_ERR_TMA_TIMEOUT);
+          *(volatile int *)err = FLOF_DEV_ERR_TMA_TIMEOUT;
           for (int r = p; r < NP && r < p + NS; ++r) mbar_wait_bounded(&bar[r % NS], (r / NS) & 1);
         }
         __syncthreads();
