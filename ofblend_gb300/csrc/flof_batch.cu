@@ -131,6 +131,7 @@ FLOF_API int flof_opticalFlowMultiscale4d_batch(flof_ctx *c, int n, flof_grid *c
     std::vector<flof_ctx *> ws(nw);
     for (int q = 0; q < nw; ++q) {
       ws[q] = worker(c, q);
+      ws[q]->beside = nw > 1;
       CK(cudaStreamWaitEvent(ws[q]->stream, ready, 0));
     }
     CK(cudaEventDestroy(ready));

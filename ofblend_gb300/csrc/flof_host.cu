@@ -305,13 +305,13 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
   const double gb = sizeof(GT) == 8 ? 8.0 : 16.0;  // bytes of g per cell
   const double gpc = i1 ? 4.0 : gb;                 // bytes of g or i1 per cell in update/direction
   if (resident_cells_ok(d) && maxIter > 0) {
-    // one cooperative launch; its blocks wait on one another, so the lock is
-    // held until it has ended
-    std::lock_guard<std::mutex> lock(resident_mutex());
+    // one cooperative launch; its blocks wait on one another, so its share of
+    // the SMs is held until it has ended
+    ResidentShare share;
     bool done = false;
     KLP(c, KC_RESIDENT, d.x, nint(d) * 64,
         done = launch_cg_resident(x, r, p, q, g, d, k, c->st, c->dpart, maxIter, c->dev_err,
-                                  next_post(c), c->stream));
+                                  next_post(c), c->beside, share, c->stream));
     if (done) {
       wait_post(c, &c->hres->cg_seq);
       c->st_h->done = c->hres->done;

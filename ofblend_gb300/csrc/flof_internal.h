@@ -170,6 +170,7 @@ struct flof_ctx {
   std::map<std::array<int, 4>, flof::CGTune> tunes;
   std::mutex tune_mu;
   flof_ctx *tune_owner = nullptr;
+  bool beside = false;  // a worker of a batch: other solves run beside its own
   // worker contexts of the batched solve (created on demand)
   std::vector<flof_ctx *> workers;
   // live grids of this context: destroying the context frees their storage

@@ -6,7 +6,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <mutex>
 #include <vector>
 
 #include "flof_common.cuh"
@@ -195,18 +194,28 @@ void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const BF4 *g, Di
 // with st->done set and the outcome posted to the host.  r is read only at the start and q is scratch.  False
 // (nothing launched) for a larger level, maxIter <= 0, or when the device
 // refuses the launch: the caller then chains the kernels above.  Its blocks
-// wait on one another, so two of them must not run at once: hold
-// resident_mutex() from the launch until the stream has been waited for.
+// wait on one another, so those of all launches in flight are counted and the
+// call waits for room; `share` gives its part back when it goes out of scope,
+// after the stream has been waited for.  shared: other solves run beside this
+// one (the same result, on a quarter of the SMs where the level is small).
 // part holds at least 7 doubles per SM.
 constexpr size_t RESIDENT_SMEM = 220 * 1024;  // shared memory for its cells, per SM
 bool resident_cells_ok(Dims4 d);
-std::mutex &resident_mutex();
+struct ResidentShare {
+  int blocks = 0;
+  ResidentShare() {}
+  ResidentShare(const ResidentShare &) = delete;
+  ResidentShare &operator=(const ResidentShare &) = delete;
+  ~ResidentShare() { give(); }
+  void take(int n);
+  void give();
+};
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        HostPost post, cudaStream_t s);
+                        HostPost post, bool shared, ResidentShare &share, cudaStream_t s);
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        HostPost post, cudaStream_t s);
+                        HostPost post, bool shared, ResidentShare &share, cudaStream_t s);
 // ---- strict arithmetic (flof_strict.cu, FLOF_OPT_STRICT) ----------------------
 // The reference's PCG arithmetic operation for operation: double alpha and
 // beta, double multiply-and-add updates rounded once to float, and dot

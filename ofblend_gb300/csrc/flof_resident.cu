@@ -26,10 +26,19 @@
 //   16^4          38k        17.0 / 7.2 us      45x38x41x30 1.7M  68 / 47 us
 //   24^3 x 16    149k        22.6 / 9.2 us
 //
-// The blocks wait on one another, so the launch is cooperative and one at a
-// time per process (the caller holds resident_mutex() until the kernel has
-// ended); every wait is bounded, and a block that gives up records
-// FLOF_DEV_ERR_GRID_TIMEOUT and returns, and the others after it.
+// The blocks wait on one another, so the launch is cooperative and the blocks
+// of all launches in flight are counted (resident_share): they never exceed
+// the SMs, so all of them can be resident whatever else runs, as ordinary
+// kernels end by themselves.  Every wait is bounded; a block that gives up
+// records FLOF_DEV_ERR_GRID_TIMEOUT and returns, and the others after it.
+//
+// The sums are formed per work group of `per` cells and then over the groups
+// in order, and a block holds M groups, so the result does not depend on M:
+// one solve alone spreads its groups over the SMs (M = 1), the solves of a
+// batch take a quarter of the SMs each (M = 4) and run side by side.
+#include <condition_variable>
+#include <mutex>
+
 #include "flof_kernels.h"
 
 namespace flof {
@@ -97,13 +106,14 @@ __device__ __forceinline__ void post_outcome(const HostPost &post, const CGState
   *(volatile unsigned int *)&h->cg_seq = post.seq;
 }
 
-// NTH threads; K cells per thread at most when QREG (A p in registers,
-// otherwise in qg); GS: the gradient is kept in shared memory too.
-template <int NTH, int K, bool QREG, bool GS, class GT>
+// NTH threads; M groups per block, K cells of a group per thread at most when
+// QREG (A p in registers, otherwise in qg); GS: the gradient is kept in shared
+// memory too.  GV groups in all.
+template <int NTH, int M, int K, bool QREG, bool GS, class GT>
 __global__ void __launch_bounds__(NTH, 1)
 k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
               const GT *__restrict__ g, Dims4 d, BoxDecoder bx, uint32_t nint, uint32_t per,
-              OFConsts c, CGState *st, double *part, int maxIter, int *err, HostPost post) {
+              int GV, OFConsts c, CGState *st, double *part, int maxIter, int *err, HostPost post) {
   extern __shared__ float4 res_sm[];
   __shared__ FF shff[3][NTH / 32];
   __shared__ float shm[NTH / 32];
@@ -114,42 +124,49 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
     if (blockIdx.x == 0 && threadIdx.x == 0) post_outcome(post, st);
     return;
   }
-  const uint32_t c0 = blockIdx.x * per, c1 = min(c0 + per, nint);
-  const int G = gridDim.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float4 *rs = res_sm, *gsm = res_sm + per;
+  // the block's cells are contiguous; group v of it covers per cells from
+  // first(v)
+  const uint32_t b0 = blockIdx.x * (M * per);
+  auto first = [&](int v) { return min(b0 + v * per, nint); };
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float4 *rs = res_sm, *gsm = res_sm + M * per;
   const idx_t sY = d.x, sZ = d.sz(), sT = d.st();
-  double *pA = part, *pB = part + 3 * G;  // [dot][block]; [parity][z.r, max r][block]
+  double *pA = part, *pB = part + 3 * GV;  // [dot][group]; [parity][z.r, max r][group]
   const double acc = st->acc, sigma0 = st->sigma;
   auto addr = [&](uint32_t n) {
     int i, j, k, l;
     bx.decode(n, i, j, k, l);
     return d.index(i, j, k, l);
   };
-  int ids[QREG ? K : 1];
-  float4 q[QREG ? K : 1];
-  for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
-    const idx_t id = addr(n);
-    rs[n - c0] = __ldg(r0 + id);
-    if (GS) gsm[n - c0] = ld_g(g, id);
-  }
-  if (QREG) {
+  int ids[QREG ? M * K : 1];
+  float4 q[QREG ? M * K : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const uint32_t n = c0 + threadIdx.x + k * NTH;
-      ids[k] = n < c1 ? (int)addr(n) : 0;
+  for (int v = 0; v < M; ++v) {
+    const uint32_t c0 = first(v), c1 = first(v + 1);
+    for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
+      const idx_t id = addr(n);
+      rs[n - b0] = __ldg(r0 + id);
+      if (GS) gsm[n - b0] = ld_g(g, id);
+    }
+    if (QREG) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const uint32_t n = c0 + threadIdx.x + k * NTH;
+        ids[v * K + k] = n < c1 ? (int)addr(n) : 0;
+      }
     }
   }
   // (each thread reads back only the shared cells that it wrote)
 
   unsigned int target = 0;
   for (int it = 0;; ++it) {
-    FF d0 = {0.f, 0.f}, d1 = {0.f, 0.f}, d2 = {0.f, 0.f};
+    FF d0, d1, d2;
     auto phase1 = [&](uint32_t n, idx_t id) {
       const float4 pc = p[id];
       const float4 tm = p[id - sT], zm = p[id - sZ], ym = p[id - sY], xm = p[id - 1];
       const float4 xp = p[id + 1], yp = p[id + sY], zp = p[id + sZ], tp = p[id + sT];
-      const float4 gg = GS ? gsm[n - c0] : ld_g(g, id);
-      const float4 r = rs[n - c0];
+      const float4 gg = GS ? gsm[n - b0] : ld_g(g, id);
+      const float4 r = rs[n - b0];
       const float gp = __fmaf_rn(gg.w, pc.w, __fmaf_rn(gg.z, pc.z, __fmaf_rn(gg.y, pc.y, gg.x * pc.x)));
       auto row = [&](float gc, float p0, float a0, float a1, float a2, float a3, float a4, float a5,
                      float a6, float a7) {
@@ -171,51 +188,57 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
       ff_add(d2, (ux * qq.x + uy * qq.y) + (uz * qq.z + uw * qq.w));
       return qq;
     };
-    if (QREG) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const uint32_t n = c0 + threadIdx.x + k * NTH;
-        if (n < c1) q[k] = phase1(n, ids[k]);
-      }
-    } else {
+    for (int v = 0; v < M; ++v) {
+      const uint32_t c0 = first(v), c1 = first(v + 1);
+      d0 = d1 = d2 = FF{0.f, 0.f};
+      if (QREG) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const uint32_t n = c0 + threadIdx.x + k * NTH;
+          if (n < c1) q[v * K + k] = phase1(n, ids[v * K + k]);
+        }
+      } else {
 #pragma unroll 2
-      for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
-        const idx_t id = addr(n);
-        qg[id] = phase1(n, id);
+        for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
+          const idx_t id = addr(n);
+          qg[id] = phase1(n, id);
+        }
+      }
+      d0 = warp_sum_ff(d0);
+      d1 = warp_sum_ff(d1);
+      d2 = warp_sum_ff(d2);
+      if (v > 0) __syncthreads();  // the last group's sums have been read
+      if (lane == 0) {
+        shff[0][w] = d0;
+        shff[1][w] = d1;
+        shff[2][w] = d2;
+      }
+      __syncthreads();
+      if (w < 3 && c0 < nint) {
+        const FF t = warp_sum_ff(lane < NTH / 32 ? shff[w][lane] : FF{0.f, 0.f});
+        if (lane == 0) __stcg(pA + w * GV + blockIdx.x * M + v, ff_value(t));
       }
     }
-    d0 = warp_sum_ff(d0);
-    d1 = warp_sum_ff(d1);
-    d2 = warp_sum_ff(d2);
-    if (lane == 0) {
-      shff[0][w] = d0;
-      shff[1][w] = d1;
-      shff[2][w] = d2;
-    }
-    __syncthreads();
-    if (w < 3) {
-      const FF v = warp_sum_ff(lane < NTH / 32 ? shff[w][lane] : FF{0.f, 0.f});
-      if (lane == 0) __stcg(pA + w * G + blockIdx.x, ff_value(v));
-    }
-    target += G;
+    target += gridDim.x;
     if (!grid_barrier(&st->gbar, target, &ok)) {
       if (threadIdx.x == 0) *(volatile int *)err = FLOF_DEV_ERR_GRID_TIMEOUT;
       return;
     }
-    // the sums over the blocks: p.q, q.z, q.M^-1 q of this iteration, z.r and
+    // the sums over the groups: p.q, q.z, q.M^-1 q of this iteration, z.r and
     // max r of the iterate that the last phase 2 left
     const int par = it & 1;
     if (w < 5) {
-      const double *src = w < 3 ? pA + w * G : pB + (2 * par + (w - 3)) * G;
+      const double *src = w < 3 ? pA + w * GV : pB + (2 * par + (w - 3)) * GV;
       double s = 0.0;
       if (w < 4) {
         if (w < 3 || it > 0)
-          for (int b = lane; b < G; b += 32) s += __ldcg(src + b);
+          for (int b = lane; b < GV; b += 32) s += __ldcg(src + b);
         s = warp_sum(s);
       } else {
         float m = 0.f;  // border rows hold r = 0
         if (it > 0)
-          for (int b = lane; b < G; b += 32) m = fmaxf(m, (float)__ldcg(src + b));
+          for (int b = lane; b < GV; b += 32) m = fmaxf(m, (float)__ldcg(src + b));
         s = (double)warp_max(m);
       }
       if (lane == 0) fin[w] = s;
@@ -246,11 +269,11 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
       return;
     }
     const float a = ab[0], b = ab[1];
-    FF rz = {0.f, 0.f};
-    float mx = 0.f;
+    FF rz;
+    float mx;
     auto phase2 = [&](uint32_t n, idx_t id, const float4 qq) {
-      float4 r = rs[n - c0];
-      const float4 gg = GS ? gsm[n - c0] : ld_g(g, id);
+      float4 r = rs[n - b0];
+      const float4 gg = GS ? gsm[n - b0] : ld_g(g, id);
       const float4 pc = p[id];
       float4 xx = x[id], pn;
       const float4 pre = res_precond(gg, c.diag);
@@ -266,38 +289,47 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
       one(r.y, xx.y, pn.y, pc.y, qq.y, pre.y);
       one(r.z, xx.z, pn.z, pc.z, qq.z, pre.z);
       one(r.w, xx.w, pn.w, pc.w, qq.w, pre.w);
-      rs[n - c0] = r;
+      rs[n - b0] = r;
       x[id] = xx;
       p[id] = pn;
     };
-    if (QREG) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const uint32_t n = c0 + threadIdx.x + k * NTH;
-        if (n < c1) phase2(n, ids[k], q[k]);
-      }
-    } else {
+    for (int v = 0; v < M; ++v) {
+      const uint32_t c0 = first(v), c1 = first(v + 1);
+      rz = FF{0.f, 0.f};
+      mx = 0.f;
+      if (QREG) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const uint32_t n = c0 + threadIdx.x + k * NTH;
+          if (n < c1) phase2(n, ids[v * K + k], q[v * K + k]);
+        }
+      } else {
 #pragma unroll 2
-      for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
-        const idx_t id = addr(n);
-        phase2(n, id, qg[id]);
+        for (uint32_t n = c0 + threadIdx.x; n < c1; n += NTH) {
+          const idx_t id = addr(n);
+          phase2(n, id, qg[id]);
+        }
+      }
+      rz = warp_sum_ff(rz);
+      mx = warp_max(mx);
+      if (v > 0) __syncthreads();
+      if (lane == 0) {
+        shff[0][w] = rz;
+        shm[w] = mx;
+      }
+      __syncthreads();
+      if (c0 < nint) {
+        if (w == 0) {
+          const FF t = warp_sum_ff(lane < NTH / 32 ? shff[0][lane] : FF{0.f, 0.f});
+          if (lane == 0) __stcg(pB + 2 * (par ^ 1) * GV + blockIdx.x * M + v, ff_value(t));
+        } else if (w == 1) {
+          const float t = warp_max(lane < NTH / 32 ? shm[lane] : 0.f);
+          if (lane == 0) __stcg(pB + (2 * (par ^ 1) + 1) * GV + blockIdx.x * M + v, (double)t);
+        }
       }
     }
-    rz = warp_sum_ff(rz);
-    mx = warp_max(mx);
-    if (lane == 0) {
-      shff[0][w] = rz;
-      shm[w] = mx;
-    }
-    __syncthreads();
-    if (w == 0) {
-      const FF v = warp_sum_ff(lane < NTH / 32 ? shff[0][lane] : FF{0.f, 0.f});
-      if (lane == 0) __stcg(pB + 2 * (par ^ 1) * G + blockIdx.x, ff_value(v));
-    } else if (w == 1) {
-      const float m = warp_max(lane < NTH / 32 ? shm[lane] : 0.f);
-      if (lane == 0) __stcg(pB + (2 * (par ^ 1) + 1) * G + blockIdx.x, (double)m);
-    }
-    target += G;
+    target += gridDim.x;
     if (!grid_barrier(&st->gbar, target, &ok)) {
       if (threadIdx.x == 0) *(volatile int *)err = FLOF_DEV_ERR_GRID_TIMEOUT;
       return;
@@ -305,64 +337,103 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
   }
 }
 
-template <int NTH, int K, bool QREG, bool GS, class GT>
-bool launch_one(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d, uint32_t nint,
-                uint32_t per, OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                HostPost post, cudaStream_t s) {
-  auto k = k_cg_resident<NTH, K, QREG, GS, GT>;
-  constexpr size_t per_cell = GS ? 32 : 16;
-  // the largest dynamic shared memory that leaves one block per SM, asked for
-  // once (thread-safe static init); 0 when the device refuses it
-  static const size_t smem_max = [&]() -> size_t {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RESIDENT_SMEM) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return 0;
+struct ResidentArgs {
+  float4 *x, *r, *p, *q;
+  Dims4 d;
+  uint32_t n, per;  // interior cells, cells per group
+  OFConsts c;
+  CGState *st;
+  double *part;
+  int maxIter;
+  int *err;
+  HostPost post;
+  cudaStream_t s;
+};
+
+// The blocks of all launches in flight, at most one per SM in sum; waits in
+// the order of arrival.
+struct SmShares {
+  std::mutex mu;
+  std::condition_variable cv;
+  int used = 0;
+  unsigned long long next = 0, serving = 0;
+  void acquire(int n) {
+    std::unique_lock<std::mutex> lk(mu);
+    const unsigned long long mine = next++;
+    cv.wait(lk, [&] { return serving == mine && used + n <= sm_count(); });
+    ++serving;
+    used += n;
+    cv.notify_all();
+  }
+  void release(int n) {
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      used -= n;
     }
+    cv.notify_all();
+  }
+};
+SmShares &sm_shares() {
+  static SmShares s;
+  return s;
+}
+
+template <int NTH, int M, int K, bool QREG, bool GS, class GT>
+bool launch_one(ResidentArgs a, const GT *g, ResidentShare &share) {
+  auto k = k_cg_resident<NTH, M, K, QREG, GS, GT>;
+  constexpr size_t per_cell = GS ? 32 : 16;
+  // the shared memory that the kernel may use, asked for once (thread-safe
+  // static init); 0 when the device refuses it
+  static const size_t smem_max = [&]() -> size_t {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, NTH, RESIDENT_SMEM) != cudaSuccess ||
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RESIDENT_SMEM) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, NTH, RESIDENT_SMEM) != cudaSuccess ||
         n < 1) {
       cudaGetLastError();
       return 0;
     }
     return RESIDENT_SMEM;
   }();
-  const size_t smem = per_cell * per;
+  const size_t smem = per_cell * a.per * M;
   if (smem > smem_max) return false;
-  BoxDecoder bx = make_decoder(d.x - 2, d.y - 2, d.z - 2, 1, 1, 1, 1);
-  const float4 *r0 = r;
-  const unsigned grid = (nint + per - 1) / per;
-  void *args[] = {&x, &r0, &p, &q, &g, &d, &bx, &nint, &per, &c, &st, &part, &maxIter, &err, &post};
-  if (cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(NTH), args, smem, s) !=
+  BoxDecoder bx = make_decoder(a.d.x - 2, a.d.y - 2, a.d.z - 2, 1, 1, 1, 1);
+  const float4 *r0 = a.r;
+  int groups = (int)((a.n + a.per - 1) / a.per);
+  const int grid = (groups + M - 1) / M;
+  void *args[] = {&a.x, &r0,  &a.p, &a.q,  &g,    &a.d,       &bx,    &a.n,   &a.per,
+                  &groups, &a.c, &a.st, &a.part, &a.maxIter, &a.err, &a.post};
+  share.take(grid);
+  if (cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(NTH), args, smem, a.s) !=
       cudaSuccess) {
     cudaGetLastError();
+    share.give();
     return false;
   }
   return true;
 }
 
 template <class GT>
-bool launch_any(float4 *x, float4 *r, float4 *p, float4 *q, const GT *g, Dims4 d, OFConsts c,
-                CGState *st, double *part, int maxIter, int *err, HostPost post, cudaStream_t s) {
-  if (!resident_cells_ok(d) || maxIter <= 0) return false;
-  const uint32_t n = (uint32_t)((long long)(d.x - 2) * (d.y - 2) * (d.z - 2) * (d.t - 2));
+bool launch_any(ResidentArgs a, const GT *g, bool shared, ResidentShare &share) {
+  if (!resident_cells_ok(a.d) || a.maxIter <= 0) return false;
+  a.n = (uint32_t)((long long)(a.d.x - 2) * (a.d.y - 2) * (a.d.z - 2) * (a.d.t - 2));
   const uint32_t sms = (uint32_t)sm_count();
-  // 256 cells per block until every SM has one (fewer blocks make the barriers
-  // and the sums over the blocks cheaper: 6.2 against 6.9 us for 6000 cells),
-  // then two cells for each of 512 threads, then up to six for each of 1024,
-  // then A p and the gradient out of registers and shared memory.
-  uint32_t per = (n + sms - 1) / sms;
-  if (per <= 256)
-    return launch_one<256, 1, true, true>(x, r, p, q, g, d, n, 256,
-        c, st, part, maxIter, err, post, s);
-  if (per <= 1024)
-    return launch_one<512, 2, true, true>(x, r, p, q, g, d, n, per,
-        c, st, part, maxIter, err, post, s);
-  if (per <= 6144)
-    return launch_one<1024, 6, true, true>(x, r, p, q, g, d, n, per,
-        c, st, part, maxIter, err, post, s);
-  return launch_one<1024, 1, false, false>(x, r, p, q, g, d, n, per, c, st, part, maxIter, err,
-                                           post, s);
+  // 256 cells per group until every SM has one (fewer groups make the barriers
+  // and the sums over them cheaper: 6.2 against 6.9 us for 6000 cells), then
+  // two cells for each of 512 threads, then up to six for each of 1024, then
+  // A p and the gradient out of registers and shared memory.  The larger
+  // levels fill the SMs alone and are not shared out.
+  a.per = (a.n + sms - 1) / sms;
+  if (a.per <= 256) {
+    a.per = 256;
+    return shared ? launch_one<256, 4, 1, true, true>(a, g, share)
+                  : launch_one<256, 1, 1, true, true>(a, g, share);
+  }
+  if (a.per <= 1024)
+    return shared ? launch_one<512, 4, 2, true, true>(a, g, share)
+                  : launch_one<512, 1, 2, true, true>(a, g, share);
+  if (a.per <= 6144) return launch_one<1024, 1, 6, true, true>(a, g, share);
+  return launch_one<1024, 1, 1, false, false>(a, g, share);
 }
 
 }  // namespace
@@ -373,20 +444,26 @@ bool resident_cells_ok(Dims4 d) {
   return n <= (long long)sm_count() * (long long)(RESIDENT_SMEM / 16);
 }
 
-std::mutex &resident_mutex() {
-  static std::mutex mu;
-  return mu;
+void ResidentShare::take(int n) {
+  sm_shares().acquire(n);
+  blocks = n;
+}
+void ResidentShare::give() {
+  if (blocks) sm_shares().release(blocks);
+  blocks = 0;
 }
 
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        HostPost post, cudaStream_t s) {
-  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, post, s);
+                        HostPost post, bool shared, ResidentShare &share, cudaStream_t s) {
+  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, err, post, s}, g,
+                    shared, share);
 }
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
                         OFConsts c, CGState *st, double *part, int maxIter, int *err,
-                        HostPost post, cudaStream_t s) {
-  return launch_any(x, r, p, q, g, d, c, st, part, maxIter, err, post, s);
+                        HostPost post, bool shared, ResidentShare &share, cudaStream_t s) {
+  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, err, post, s}, g,
+                    shared, share);
 }
 
 }  // namespace flof
