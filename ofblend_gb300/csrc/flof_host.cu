@@ -612,6 +612,8 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
   DBuf mask(c, expol_mask_words(d) * sizeof(uint16_t));
   // the projection's queue of cells that need a search, and its two counters
   DBuf pqueue(c, project_queue_bytes(d)), pcount(c, 2 * sizeof(unsigned int));
+  DBuf reach(c, expol_reach_bytes(d));  // the tiles' distances from the marked cells
+  const int *dist = nullptr;
   DBuf s2;  // the separable sweep's (x,y) box sums (blurType 2)
   int singleStep = 0;
   if (postVelBlur < blurThreshold) singleStep = 1;
@@ -629,9 +631,13 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
       // The sweeps only rewrite unmarked interior cells; both buffers carry
       // the projected values everywhere else (the reference's tmp copy).
       CK(cudaMemcpyAsync(B, A, vec_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
-      if (c->slab_tma)  // the plain-load sweeps read the marker
+      if (c->slab_tma) {  // the plain-load sweeps read the marker
         KLP(c, KC_EXPOL_MASK, d.x, d.cells() * 4,
             launch_expol_mask(marker.f(), (uint16_t *)mask.p, d, c->stream));
+        KLP(c, KC_EXPOL_MASK, d.x, d.cells() * 4,
+            dist = launch_expol_reach(marker.f(), reach.p, d, c->stream));
+        c->launches++;  // two kernels
+      }
     }
     const uint16_t *keep = (const uint16_t *)mask.p;
     for (int s = 0; s < doCvExtrapol; ++s) {
@@ -639,7 +645,7 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
       if (blurType == FLOF_BLUR_GAUSS_SEPARABLE) {
         if (c->slab_tma)
           KLP(c, KC_EXPOL, d.x, d.cells() * 32,
-              tma = launch_expol_sep_tw(A, B, keep, d, c->dev_err, c->stream));
+              tma = launch_expol_sep_tw(A, B, keep, dist, s + 1, d, c->dev_err, c->stream));
         if (!tma) {
           if (!s2.p) s2 = DBuf(c, vec_bytes(d));
           KLP(c, KC_EXPOL, d.x, d.cells() * 68,
@@ -648,7 +654,7 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
       } else {
         if (c->slab_tma)
           KLP(c, KC_EXPOL, d.x, d.cells() * 32,
-              tma = launch_expol_tw(A, B, keep, d, c->dev_err, c->stream));
+              tma = launch_expol_tw(A, B, keep, dist, s + 1, d, c->dev_err, c->stream));
         if (!tma)
           KLP(c, KC_EXPOL, d.x, d.cells() * 36,
               launch_expol_slab(A, B, marker.f(), d, c->stream));

@@ -354,8 +354,14 @@ void launch_expol_mask(const float *mark, uint16_t *mask, Dims4 d, cudaStream_t 
 // The sweep walking t with three output planes' running sums in registers
 // (every output adds its 81 taps in the reference's order); false when TMA
 // is unavailable (the caller then uses launch_expol_slab).
-bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, Dims4 d, int *err,
-                     cudaStream_t st);
+// `dist` (from launch_expol_reach on the round's marker, expol_reach_bytes(d)
+// bytes of scratch) bounds each tile's distance from the marked cells: sweep
+// number `sweep` (from 1) of the round leaves the tiles beyond it alone.  This
+// needs every unmarked cell of both buffers to hold +0 before the first sweep.
+size_t expol_reach_bytes(Dims4 d);
+const int *launch_expol_reach(const float *mark, void *scratch, Dims4 d, cudaStream_t st);
+bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, const int *dist,
+                     int sweep, Dims4 d, int *err, cudaStream_t st);
 // The sweep with its 3^4 box sum formed separably (blurType 2, flof_mg.cu):
 // s2 (a Vec4 grid of d's size) receives the 3x3 (x,y) sums, out the 1/81 of
 // their 3x3 (z,t) sums at unmarked interior cells.  Equal to the reference's
@@ -364,8 +370,8 @@ void launch_expol_sep(const float4 *in, float4 *out, float4 *s2, const float *ma
                       cudaStream_t s);
 // The separable sweep in one TMA pass walking t, with the same sums in the
 // same order as launch_expol_sep (equal bits); false when TMA is unavailable.
-bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, Dims4 d, int *err,
-                         cudaStream_t st);
+bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, const int *dist,
+                         int sweep, Dims4 d, int *err, cudaStream_t st);
 
 // ---- projection correction ------------------------------------------------------
 // knProjectCells in two kernels: the normals and the cells that finish

@@ -268,12 +268,29 @@ constexpr int ETW_KZ = ETW_DZ + 2;  // slabs per t plane
 static_assert(ETW_RY == ExpolGeom::RY && ETW_DZ == ExpolGeom::DZ,
               "the keep mask groups rows and z planes as the sweep does");
 
+// Tiles that a sweep cannot reach.  Before the first sweep every unmarked cell
+// holds +0 (knProjectCells leaves it so), and a sweep gives an unmarked cell
+// the mean of its 3^4 neighbourhood, so after s sweeps an unmarked cell
+// further than s cells (in the maximum norm) from every marked one still holds
+// +0: all of its 81 taps were +0, and so is their sum over 81.  dist holds per
+// tile a lower bound of that distance; a tile beyond it has nothing to read
+// and nothing to write, since both sweep buffers hold +0 there.  The surface
+// band is a few cells thick, so the first sweeps of a round touch a part of
+// the grid only.
+__device__ __forceinline__ bool tile_unreached(const int *__restrict__ dist, int sweep) {
+  const size_t tile =
+      ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  return __ldg(dist + tile) > sweep;
+}
+
 // Four blocks per SM (64 registers, a few bytes spilled) beat three
 // (80 registers): 0.221 against 0.229 ms per 64^4 sweep; copies of two z
 // slabs, two copies in flight (one barrier per two slabs), 0.217 ms.
 __global__ void __launch_bounds__(32 * ETW_NW, 4)
 k_expol_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Dims4 d,
-           int tiles_x, const uint16_t *__restrict__ fixed, int *err) {
+           int tiles_x, const uint16_t *__restrict__ fixed, const int *__restrict__ dist, int sweep,
+           int *err) {
+  if (tile_unreached(dist, sweep)) return;
   extern __shared__ __align__(128) unsigned char raw[];
   __shared__ __align__(8) uint64_t bar[ETW_NS];
   constexpr int RY = ETW_RY, DZ = ETW_DZ, KZ = ETW_KZ, NS = ETW_NS;
@@ -411,6 +428,73 @@ k_expol_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
   plane(ETW_TC + 1, T_(), F_(), F_());
 }
 
+// Per brick of BRICK_X x 8 x 8 x 8 cells, the bounds of its marked cells in
+// x, y, z, t (lo > hi: none).
+constexpr int BRICK_X = 16, BRICK = 8;
+struct BrickBounds {
+  int lo[4], hi[4];
+};
+__global__ void __launch_bounds__(128)
+k_expol_bricks(const float *__restrict__ mark, BrickBounds *__restrict__ out, Dims4 d, int bx,
+               int by, int bz) {
+  __shared__ int sh[8];
+  if (threadIdx.x < 8) sh[threadIdx.x] = threadIdx.x < 4 ? 0x7fffffff : -1;
+  __syncthreads();
+  const int xb = blockIdx.x % bx, r = blockIdx.x / bx, yb = r % by, r2 = r / by;
+  const int zb = r2 % bz, tb = r2 / bz;
+  const int x = xb * BRICK_X + (threadIdx.x & 15), y = yb * BRICK + (threadIdx.x >> 4);
+  int lo[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[4] = {-1, -1, -1, -1};
+  if (x < d.x && y < d.y)
+    for (int t = tb * BRICK; t < min(tb * BRICK + BRICK, d.t); ++t)
+      for (int z = zb * BRICK; z < min(zb * BRICK + BRICK, d.z); ++z)
+        if (__ldg(mark + d.index(x, y, z, t)) != 0.f) {
+          const int c[4] = {x, y, z, t};
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            lo[a] = min(lo[a], c[a]);
+            hi[a] = max(hi[a], c[a]);
+          }
+        }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
+    hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(&sh[a], lo[a]);
+      atomicMax(&sh[4 + a], hi[a]);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 8) ((int *)(out + blockIdx.x))[threadIdx.x] = sh[threadIdx.x];
+}
+
+// dist[tile]: the least distance in the maximum norm between the tile's
+// outputs and a brick's bounds (marked cells lie within those).
+__global__ void __launch_bounds__(128)
+k_expol_dist(const BrickBounds *__restrict__ b, int nb, int *__restrict__ dist, int tiles_x) {
+  __shared__ int best;
+  if (threadIdx.x == 0) best = 0x7fffffff;
+  __syncthreads();
+  const int lo[4] = {(int)(blockIdx.x % tiles_x) * TX, (int)(blockIdx.x / tiles_x) * ETW_TY,
+                     (int)blockIdx.y * ETW_DZ, (int)blockIdx.z * ETW_TC};
+  const int hi[4] = {lo[0] + TX - 1, lo[1] + ETW_TY - 1, lo[2] + ETW_DZ - 1, lo[3] + ETW_TC - 1};
+  int mine = 0x7fffffff;
+  for (int k = threadIdx.x; k < nb; k += 128) {
+    const int4 l = __ldg((const int4 *)(b + k)), h = __ldg((const int4 *)(b + k) + 1);
+    if (h.x < 0) continue;
+    int g = max(l.x - hi[0], lo[0] - h.x);
+    g = max(g, max(l.y - hi[1], lo[1] - h.y));
+    g = max(g, max(l.z - hi[2], lo[2] - h.z));
+    g = max(g, max(l.w - hi[3], lo[3] - h.w));
+    mine = min(mine, g);
+  }
+  mine = __reduce_min_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0) atomicMin(&best, mine);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    dist[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = best;
+}
+
 // The separable extrapolation sweep (blurType 2) walking t.  It takes
 // k_expol_tw's slabs in k_expol_tw's order but forms each output's 3^4 sum as
 // box sums: per slab the x sums of the rows a thread needs and the y sums of
@@ -426,6 +510,7 @@ k_expol_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
 // pipelines did not help.  A copy brings two z slabs (one block barrier per
 // two slabs): 0.165 ms.
 constexpr int ESW_RY = 2, ESW_NW = ETW_TY / ESW_RY, ESW_TC = 8, ESW_NS = 3, ESW_MINB = 3;
+static_assert(ESW_TC == ETW_TC, "both sweeps have the tiles that k_expol_dist measures");
 constexpr int ESW_SPC = 2;  // z slabs per copy: one barrier step per two slabs
 constexpr int ESW_CBYTES = ESW_SPC * ETW_BYTES;  // one copy, its slabs back to back
 constexpr int ESW_CSTRIDE = (ESW_CBYTES + 127) / 128 * 128;
@@ -434,7 +519,9 @@ static_assert(ETW_KZ % ESW_SPC == 0, "whole copies per plane");
 
 __global__ void __launch_bounds__(32 * ESW_NW, ESW_MINB)
 k_expol_sep_tw(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Dims4 d,
-               int tiles_x, const uint16_t *__restrict__ fixed, int *err) {
+               int tiles_x, const uint16_t *__restrict__ fixed, const int *__restrict__ dist,
+               int sweep, int *err) {
+  if (tile_unreached(dist, sweep)) return;
   extern __shared__ __align__(128) unsigned char raw[];
   __shared__ __align__(8) uint64_t bar[ESW_NS];
   constexpr int RY = ESW_RY, DZ = ETW_DZ, KZ = ETW_KZ, NS = ESW_NS;
@@ -676,10 +763,42 @@ void launch_expol_mask(const float *mark, uint16_t *mask, Dims4 d, cudaStream_t 
   k_expol_mask<<<grid_for(n, 256), 256, 0, st>>>(mark, mask, d, ygroups, zgroups, n);
 }
 
-bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, Dims4 d, int *err,
-                     cudaStream_t st) {
-  const int zgroups = (d.z + ETW_DZ - 1) / ETW_DZ, tgroups = (d.t + ETW_TC - 1) / ETW_TC;
-  if (zgroups > 65535 || tgroups > 65535) return false;
+namespace {
+dim3 sweep_grid(Dims4 d) {
+  const int tiles_x = (d.x + TX - 1) / TX, tiles_y = (d.y + ETW_TY - 1) / ETW_TY;
+  return dim3(tiles_x * tiles_y, (d.z + ETW_DZ - 1) / ETW_DZ, (d.t + ETW_TC - 1) / ETW_TC);
+}
+int brick_count(Dims4 d, int *bx, int *by, int *bz) {
+  *bx = (d.x + BRICK_X - 1) / BRICK_X;
+  *by = (d.y + BRICK - 1) / BRICK;
+  *bz = (d.z + BRICK - 1) / BRICK;
+  return *bx * *by * *bz * ((d.t + BRICK - 1) / BRICK);
+}
+}  // namespace
+
+size_t expol_reach_bytes(Dims4 d) {
+  int bx, by, bz;
+  const dim3 g = sweep_grid(d);
+  return sizeof(BrickBounds) * (size_t)brick_count(d, &bx, &by, &bz) +
+         sizeof(int) * (size_t)g.x * g.y * g.z;
+}
+
+const int *launch_expol_reach(const float *mark, void *scratch, Dims4 d, cudaStream_t st) {
+  int bx, by, bz;
+  const int nb = brick_count(d, &bx, &by, &bz);
+  const dim3 g = sweep_grid(d);
+  BrickBounds *b = (BrickBounds *)scratch;
+  int *dist = (int *)(b + nb);
+  if (g.y > 65535 || g.z > 65535) return dist;  // the sweeps refuse such a grid too
+  k_expol_bricks<<<nb, 128, 0, st>>>(mark, b, d, bx, by, bz);
+  k_expol_dist<<<g, 128, 0, st>>>(b, nb, dist, (d.x + TX - 1) / TX);
+  return dist;
+}
+
+bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, const int *dist,
+                     int sweep, Dims4 d, int *err, cudaStream_t st) {
+  const dim3 grid = sweep_grid(d);
+  if (grid.y > 65535 || grid.z > 65535) return false;
   CUtensorMap map;
   if (!encode_slab_map(&map, in, d, ETW_W, ETW_H, ETW_SPC)) return false;
   static const bool attr = [] {
@@ -691,16 +810,15 @@ bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, Dims4 
     return true;
   }();
   if (!attr) return false;
-  const int tiles_x = (d.x + TX - 1) / TX, tiles_y = (d.y + ETW_TY - 1) / ETW_TY;
-  dim3 grid(tiles_x * tiles_y, zgroups, tgroups);
-  k_expol_tw<<<grid, 32 * ETW_NW, ETW_SMEM, st>>>(map, out, d, tiles_x, mask, err);
+  k_expol_tw<<<grid, 32 * ETW_NW, ETW_SMEM, st>>>(map, out, d, (d.x + TX - 1) / TX, mask, dist,
+                                                  sweep, err);
   return true;
 }
 
-bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, Dims4 d, int *err,
-                         cudaStream_t st) {
-  const int zgroups = (d.z + ETW_DZ - 1) / ETW_DZ, tgroups = (d.t + ESW_TC - 1) / ESW_TC;
-  if (zgroups > 65535 || tgroups > 65535) return false;
+bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, const int *dist,
+                         int sweep, Dims4 d, int *err, cudaStream_t st) {
+  const dim3 grid = sweep_grid(d);
+  if (grid.y > 65535 || grid.z > 65535) return false;
   CUtensorMap map;
   if (!encode_slab_map(&map, in, d, ETW_W, ETW_H, ESW_SPC)) return false;
   static const bool attr = [] {
@@ -712,9 +830,8 @@ bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, Di
     return true;
   }();
   if (!attr) return false;
-  const int tiles_x = (d.x + TX - 1) / TX, tiles_y = (d.y + ETW_TY - 1) / ETW_TY;
-  dim3 grid(tiles_x * tiles_y, zgroups, tgroups);
-  k_expol_sep_tw<<<grid, 32 * ESW_NW, ESW_SMEM, st>>>(map, out, d, tiles_x, mask, err);
+  k_expol_sep_tw<<<grid, 32 * ESW_NW, ESW_SMEM, st>>>(map, out, d, (d.x + TX - 1) / TX, mask,
+                                                      dist, sweep, err);
   return true;
 }
 
