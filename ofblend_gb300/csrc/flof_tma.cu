@@ -37,33 +37,23 @@ namespace {
 
 constexpr int TX = 32;                // tile width: one column per lane
 
-// Tile geometry: NW warps, RY rows per thread, DT consecutive t planes and DZ
-// consecutive z planes per block, NSTAGE slab buffers in flight.
-template <int S, int NW_, int RY_, int DT_, int DZ_, int NSTAGE_, int MINB_ = 1>
-struct TG {
-  static constexpr int NW = NW_, RY = RY_, DT = DT_, DZ = DZ_, NSTAGE = NSTAGE_, MINB = MINB_;
-  static constexpr int NTHR = 32 * NW;
-  static constexpr int TY = NW * RY;
-  static constexpr int W = TX + 2 * S, H = TY + 2 * S, N = W * H;
-  static constexpr int BYTES = N * 16;                   // one slab
-  static constexpr int STRIDE = (BYTES + 127) / 128 * 128;  // slab start spacing
-  static constexpr int SMEM = NSTAGE * STRIDE;
+// The sweeps' keep-mask layout: a 16-bit word per thread for RY = 2 rows,
+// DZ = 2 z planes and DT = 4 t planes.
+struct ExpolGeom {
+  static constexpr int RY = 2, DT = 4, DZ = 2;
   static_assert(DZ * DT * RY <= 16, "the keep mask holds 16 cells per thread");
 };
-// The blur (S = 1, 2) is bound by its multiply-adds: one (z, t) plane per
-// block, 32 rows.  ExpolGeom fixes the sweeps' keep-mask layout: a 16-bit
-// word per thread for RY = 2 rows, DZ = 2 z planes and DT = 4 t planes.
-template <int S> using BlurGeom = TG<S, 4, 8, 1, 1, 2>;
-using ExpolGeom = TG<1, 8, 2, 4, 2, 4, 3>;
 
 // The extrapolation sweeps and the blur add with sm_100-family packed
 // `add.rn.f32x2`: a float4 is two float pairs (x,y), (z,w), each lane rounded
 // like the scalar add, so the sums are bit for bit the scalar ones in the
-// same order at half the instruction count (4M random pairs on GB300: no
-// difference).  The blur's products stay scalar multiplies: the packed
-// `mul.rn.f32x2` gave results different from the scalar multiply in about
-// 15% of 4M random cases on GB300, and a blur built on it failed the bitwise
-// comparisons with the reference's separately rounded products.
+// same order at half the instruction count (the FP32 pipe takes the same
+// cycles).  The blur's products are packed too, as fma(w, a, -0): the packed
+// `mul.rn.f32x2` may be contracted with the add that follows (results differed
+// from the separately rounded product in 15% of 4M random cases), while an fma
+// whose addend the compiler cannot see cannot; adding -0 leaves the rounded
+// product, zeros' signs included.  The -0 is a kernel argument: as a constant
+// the fma became a multiply and was contracted after all.
 struct __align__(16) P4 {
   unsigned long long lo, hi;
 };
@@ -80,14 +70,16 @@ __device__ __forceinline__ float4 unpack4(const P4 &v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.z), "=f"(r.w) : "l"(v.hi));
   return r;
 }
-// w times a float4 by scalar multiplies, the products packed as two float
-// pairs for the packed adds
-__device__ __forceinline__ P4 mulp4(float w, const float4 &a) {
-  const float4 m = make_float4(__fmul_rn(w, a.x), __fmul_rn(w, a.y), __fmul_rn(w, a.z),
-                               __fmul_rn(w, a.w));
-  P4 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.lo) : "f"(m.x), "f"(m.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.hi) : "f"(m.z), "f"(m.w));
+__device__ __forceinline__ unsigned long long pair2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+// the products of two float pairs, each rounded once; nz is the pair (-0, -0)
+__device__ __forceinline__ unsigned long long mul2_rn(unsigned long long a, unsigned long long b,
+                                                      unsigned long long nz) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
   return r;
 }
 
@@ -106,143 +98,131 @@ struct WTabT {
   float w[40];
 };
 
-// The Gaussian blur pass.  A block computes the outputs of DZ x DT
-// consecutive (z, t) planes.  It walks the input slabs (tt, zz) of the union
-// of their neighbourhoods in lexicographic order; for a fixed output plane
-// (z_o, t_o) that order is the reference's (vt, zk) order with
-// vt = tt - t_o, zk = zz - z_o, so every output still adds its taps in the
-// reference's sequence while each slab is fetched once for all planes.
-template <int S, class G>
-__global__ void __launch_bounds__(G::NTHR, G::MINB)
-k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Dims4 d,
-           int tiles_x, const float *__restrict__ wsum, WTabT wt, int zero_border, int *err) {
-  constexpr int RY = G::RY, DT = G::DT, DZ = G::DZ, NS = G::NSTAGE;
+// The Gaussian blur pass (S = 1, 2).  A block owns an LW-wide (x,y) tile of
+// one (z, t) plane and takes the (x,y) slabs of its neighbourhood in the
+// reference's (t, z) order; a thread computes RY consecutive rows of one
+// column, so every output adds its taps in the reference's sequence.  Slabs
+// outside the grid would add products of zero, which leave a running sum
+// unchanged, and are not visited.
+// Bound by the FP32 pipe: 625 ordered adds per component, plus the products
+// w * a, each rounded once as in the reference (mul2_rn) and formed once per
+// |yj| for the two rows that use it.  Keeping five output planes' sums, so that
+// the products are shared along t too, needs a loop body of 2000 instructions
+// and waits for them (no_instruction 2.5 of 4.6 cycles per issue): 2.12 ms at
+// 64^4, no faster than this form.
+constexpr int BW_NS = 3, BW_MAXW = 4;
+template <int LW, int RY>
+struct BW {
+  static constexpr int RG = 32 / LW;      // row groups of a warp
+  static constexpr int UNIT = RG * RY;    // rows of a warp
+};
+__host__ __device__ constexpr int blur_stride(int w, int h) { return (w * h * 16 + 127) / 128 * 128; }
+
+template <int S, int LW, int RY>
+__global__ void __launch_bounds__(32 * BW_MAXW)
+k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Dims4 d, int tiles_x,
+           const float *__restrict__ wsum, WTabT wt, unsigned long long nz, int zero_border,
+           int *err) {
+  using G = BW<LW, RY>;
+  constexpr int NS = BW_NS, NV = 2 * S + 1, W = LW + 2 * S;
   extern __shared__ __align__(128) unsigned char raw[];
   __shared__ __align__(8) uint64_t bar[NS];
-  __shared__ float wsh[40];
-
-  const int tile = blockIdx.x;
-  const int x0 = (tile % tiles_x) * TX, y0 = (tile / tiles_x) * G::TY;
-  const int z0 = blockIdx.y * DZ, t0 = blockIdx.z * DT;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int x = x0 + tx;
-
+  __shared__ unsigned long long wsh[40];  // (w, w) pairs
+  const int ty_rows = (int)(blockDim.x >> 5) * G::UNIT, h = ty_rows + 2 * S;
+  const int stride = blur_stride(W, h);
+  const int x0 = (int)(blockIdx.x % tiles_x) * LW, y0 = (int)(blockIdx.x / tiles_x) * ty_rows;
+  const int z = blockIdx.y, t = blockIdx.z;
+  const int lane = threadIdx.x & 31, lx = lane % LW, x = x0 + lx;
+  const int row0 = ((int)(threadIdx.x >> 5) * G::RG + lane / LW) * RY;
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int b = 0; b < NS; ++b) mbar_init(&bar[b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (threadIdx.x < 40) wsh[threadIdx.x] = wt.w[threadIdx.x];
+  for (int i = threadIdx.x; i < 40; i += blockDim.x) wsh[i] = pair2(wt.w[i], wt.w[i]);
   __syncthreads();
-
-  constexpr int KZ = DZ + 2 * S;
-  constexpr int NP = (DT + 2 * S) * KZ;  // slabs (tt, zz), tt-major
-  // slab p lives in buffer p % NS; its barrier completes phase (p / NS) & 1
+  // the slabs inside the grid, t-major
+  const int ta = max(t - S, 0), tb = min(t + S, d.t - 1);
+  const int za = max(z - S, 0), zb = min(z + S, d.z - 1);
+  const int np = (tb - ta + 1) * (zb - za + 1);
+  int it = ta, iz = za;  // the next slab to fetch
   auto issue = [&](int p) {
     uint64_t *b = &bar[p % NS];
-    mbar_expect_tx(b, G::BYTES);
-    tma_load_slab(raw + (p % NS) * G::STRIDE, &map, x0 - S, y0 - S, z0 - S + p % KZ,
-                  t0 - S + p / KZ, b);
-  };
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int p = 0; p < NS - 1; ++p)
-      if (p < NP) issue(p);
-  }
-
-  typedef float4 V4;
-  P4 val[DZ][DT][RY];  // running sums as two float pairs for the packed adds
-#pragma unroll
-  for (int oz = 0; oz < DZ; ++oz)
-#pragma unroll
-    for (int o = 0; o < DT; ++o)
-#pragma unroll
-      for (int q = 0; q < RY; ++q) memset(&val[oz][o][q], 0, sizeof(P4));
-
-  for (int p = 0; p < NP; ++p) {
-    const int vt0 = p / KZ - S, zk0 = p % KZ - S;  // offsets seen by plane (0, 0)
-    // buffer (p - 1) % NS was released by the barrier that ended step p - 1
-    if (threadIdx.x == 0 && p + NS - 1 < NP) issue(p + NS - 1);
-    const bool ok = mbar_wait_bounded(&bar[p % NS], (p / NS) & 1);
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) {
-        *(volatile int *)err = FLOF_DEV_ERR_TMA_TIMEOUT;
-        // let the copies in flight land before the block's shared memory goes
-        for (int r = p; r < NP && r < p + NS; ++r) mbar_wait_bounded(&bar[r % NS], (r / NS) & 1);
-      }
-      __syncthreads();
-      return;
+    mbar_expect_tx(b, (uint32_t)(W * h * 16));
+    tma_load_slab(raw + (p % NS) * stride, &map, x0 - S, y0 - S, iz, it, b);
+    if (++iz > zb) {
+      iz = za;
+      ++it;
     }
-    const V4 *cur = (const V4 *)(raw + (p % NS) * G::STRIDE);
-    // slab rows RY*ty .. RY*ty+RY-1+2S feed output rows RY*ty+q via yj = k-q-S
+  };
+  if (threadIdx.x == 0)
+    for (int p = 0; p < NS - 1 && p < np; ++p) issue(p);
+
+  P4 acc[RY];
 #pragma unroll
-    for (int k = 0; k < RY + 2 * S; ++k) {
-      const V4 *row = cur + (RY * ty + k) * G::W + tx;
-      V4 a[2 * S + 1];
+  for (int q = 0; q < RY; ++q) acc[q] = P4{0ull, 0ull};
+  int p = 0;
+  for (int tt = ta; tt <= tb; ++tt)
+    for (int zz = za; zz <= zb; ++zz, ++p) {
+      // buffer (p - 1) % NS was released by the barrier that ended step p - 1
+      if (threadIdx.x == 0 && p + NS - 1 < np) issue(p + NS - 1);
+      const bool ok = mbar_wait_bounded(&bar[p % NS], (p / NS) & 1);
+      // a thread whose wait gave up reads stale values, in bounds; the barrier
+      // that ends the step then ends the block
+      const P4 *cur = (const P4 *)(raw + (p % NS) * stride) + row0 * W + lx;
+      const unsigned long long *wz = wsh + (tt - t) * (tt - t) + (zz - z) * (zz - z);
+      // slab row row0 + k feeds output row q via yj = k - q - S
 #pragma unroll
-      for (int m = 0; m <= 2 * S; ++m) a[m] = row[m];
+      for (int k = 0; k < RY + 2 * S; ++k) {
+        P4 a[NV];
 #pragma unroll
-      for (int oz = 0; oz < DZ; ++oz) {
-        const int zk = zk0 - oz;
-        if (zk < -S || zk > S) continue;
+        for (int i = 0; i < NV; ++i) a[i] = cur[k * W + i];
 #pragma unroll
-        for (int o = 0; o < DT; ++o) {
-          const int vt = vt0 - o;
-          if (vt < -S || vt > S) continue;
-          // Output rows at y offsets +-ay use the same weights, so the
-          // rounded products w * a are formed once per |yj| and added to
-          // each of those rows in the usual xi order.
+        for (int ay = 0; ay <= S; ++ay) {
+          // output rows at y offsets +-ay use the same weights
+          const int qm = k - S - ay, qp = k - S + ay;
+          if (!((qm >= 0 && qm < RY) || (qp >= 0 && qp < RY))) continue;
+          P4 prod[NV];
 #pragma unroll
-          for (int ay = 0; ay <= S; ++ay) {
-            bool used = false;
-#pragma unroll
-            for (int q = 0; q < RY; ++q) used |= (k - q - S == ay) || (k - q - S == -ay);
-            if (!used) continue;
-            const int base = vt * vt + zk * zk + ay * ay;
-            P4 prod[2 * S + 1];
-#pragma unroll
-            for (int xi = -S; xi <= S; ++xi) prod[xi + S] = mulp4(wsh[base + xi * xi], a[xi + S]);
-#pragma unroll
-            for (int q = 0; q < RY; ++q) {
-              const int yj = k - q - S;
-              if (yj != ay && yj != -ay) continue;
-#pragma unroll
-              for (int xi = -S; xi <= S; ++xi) acc4(val[oz][o][q], prod[xi + S]);
-            }
+          for (int i = 0; i < NV; ++i) {
+            const unsigned long long w2 = wz[ay * ay + (i - S) * (i - S)];
+            prod[i] = P4{mul2_rn(w2, a[i].lo, nz), mul2_rn(w2, a[i].hi, nz)};
           }
+          if (qm >= 0 && qm < RY)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) acc4(acc[qm], prod[i]);
+          if (ay > 0 && qp >= 0 && qp < RY)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) acc4(acc[qp], prod[i]);
         }
       }
+      if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) {
+          *(volatile int *)err = FLOF_DEV_ERR_TMA_TIMEOUT;
+          // let the copies in flight land before the block's shared memory goes
+          for (int r = p; r < np && r < p + NS; ++r) mbar_wait_bounded(&bar[r % NS], (r / NS) & 1);
+        }
+        __syncthreads();
+        return;
+      }
     }
-    __syncthreads();
-  }
 
   if (x >= d.x) return;
   constexpr int P1 = (S + 1) * (S + 1);
+  const bool zt_inner = z >= 1 && z < d.z - 1 && t >= 1 && t < d.t - 1;
+  const int code_zt = (clip_code_t<S>(t, d.t) * P1 + clip_code_t<S>(z, d.z)) * P1;
 #pragma unroll
-  for (int oz = 0; oz < DZ; ++oz) {
-    const int z = z0 + oz;
-    if (z >= d.z) break;
-#pragma unroll
-    for (int o = 0; o < DT; ++o) {
-      const int t = t0 + o;
-      if (t >= d.t) break;
-      const bool zt_inner = z >= 1 && z < d.z - 1 && t >= 1 && t < d.t - 1;
-      const int code_zt = (clip_code_t<S>(t, d.t) * P1 + clip_code_t<S>(z, d.z)) * P1;
-#pragma unroll
-      for (int q = 0; q < RY; ++q) {
-        const int y = y0 + RY * ty + q;
-        if (y >= d.y) continue;
-        const idx_t id = d.index(x, y, z, t);
-        const float4 v = unpack4(val[oz][o][q]);
-        if (!(zt_inner && x >= 1 && x < d.x - 1 && y >= 1 && y < d.y - 1)) {
-          if (zero_border) dst[id] = make_float4(0.f, 0.f, 0.f, 0.f);
-          continue;
-        }
-        const float ws =
-            __ldg(wsum + (code_zt + clip_code_t<S>(y, d.y)) * P1 + clip_code_t<S>(x, d.x));
-        dst[id] = make_float4(v.x / ws, v.y / ws, v.z / ws, v.w / ws);
-      }
+  for (int q = 0; q < RY; ++q) {
+    const int y = y0 + row0 + q;
+    if (y >= d.y) continue;
+    const idx_t id = d.index(x, y, z, t);
+    if (!(zt_inner && x >= 1 && x < d.x - 1 && y >= 1 && y < d.y - 1)) {
+      if (zero_border) dst[id] = make_float4(0.f, 0.f, 0.f, 0.f);
+      continue;
     }
+    const float4 v = unpack4(acc[q]);
+    const float ws = __ldg(wsum + (code_zt + clip_code_t<S>(y, d.y)) * P1 + clip_code_t<S>(x, d.x));
+    dst[id] = make_float4(v.x / ws, v.y / ws, v.z / ws, v.w / ws);
   }
 }
 
@@ -680,37 +660,82 @@ bool encode_slab_map(CUtensorMap *m, const float4 *base, Dims4 d, int W, int H, 
 
 namespace {
 
-template <int S, class G>
-bool launch_blur(const float4 *src, float4 *dst, Dims4 d, const float *wsum, const float *w,
-                 int zero_border, int *err, cudaStream_t st) {
-  const int tgroups = (d.t + G::DT - 1) / G::DT, zgroups = (d.z + G::DZ - 1) / G::DZ;
-  if (zgroups > 65535 || tgroups > 65535) return false;
+// The shape of a blur launch: tile width, rows per thread, warps per block.
+struct BlurShape {
+  int lw, ry, nw, ny;
+};
+// Of 32, 16 and 8 columns and 8 or 4 rows a thread, the tile that computes the
+// least: cells beyond the grid are computed like the others (tiles of 32 x 32
+// computed 1.8 times the cells at 48^4, 2.6 times at 40^3), and the products
+// shared between rows make a row of 8 cheaper than one of 4 (175 against 190
+// pipe cycles a slab).  A grid with fewer than three warps per SM partition at
+// 8 rows takes 4, for more warps.
+BlurShape blur_shape(Dims4 d) {
+  BlurShape best = {32, 8, 4, 1};
+  double bt = 0.0;
+  for (int ry : {8, 4})
+    for (int lw : {32, 16, 8}) {
+      const int unit = 32 / lw * ry;
+      const int ny = (d.y + BW_MAXW * unit - 1) / (BW_MAXW * unit);
+      const int nw = ((d.y + ny - 1) / ny + unit - 1) / unit;
+      const double warps = (double)((d.x + lw - 1) / lw) * ny * nw * d.z * d.t;
+      const double slots = 4.0 * sm_count(), row = ry == 8 ? 175.0 : 190.0;
+      // with few warps per partition their latency shows
+      const double per = warps / slots, t = row * ry * (per < 3.0 ? 1.0 + per * 2.0 / 3.0 : per);
+      if (bt == 0.0 || t < bt) {
+        bt = t;
+        best = BlurShape{lw, ry, nw, ny};
+      }
+    }
+  return best;
+}
+
+template <int S, int LW, int RY>
+bool launch_blur_shape(const float4 *src, float4 *dst, Dims4 d, const float *wsum, const WTabT &wt,
+                       int zero_border, int *err, cudaStream_t st, const BlurShape &b) {
+  constexpr int W = LW + 2 * S, UNIT = BW<LW, RY>::UNIT;
+  const int tiles_x = (d.x + LW - 1) / LW, h = b.nw * UNIT + 2 * S;
   CUtensorMap map;
-  if (!encode_slab_map(&map, src, d, G::W, G::H)) return false;
-  const int tiles_x = (d.x + TX - 1) / TX, tiles_y = (d.y + G::TY - 1) / G::TY;
-  dim3 grid(tiles_x * tiles_y, zgroups, tgroups);
+  if (!encode_slab_map(&map, src, d, W, h)) return false;
   static const bool attr = [] {
-    if (cudaFuncSetAttribute(k_blur_tma<S, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)G::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_blur_tma<S, LW, RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             BW_NS * blur_stride(W, BW_MAXW * UNIT + 2 * S)) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
     return true;
   }();
   if (!attr) return false;
+  k_blur_tma<S, LW, RY><<<dim3(tiles_x * b.ny, d.z, d.t), 32 * b.nw, BW_NS * blur_stride(W, h), st>>>(
+      map, dst, d, tiles_x, wsum, wt, 0x8000000080000000ull, zero_border, err);
+  return true;
+}
+
+template <int S>
+bool launch_blur(const float4 *src, float4 *dst, Dims4 d, const float *wsum, const float *w,
+                 int zero_border, int *err, cudaStream_t st) {
+  if (d.z > 65535 || d.t > 65535) return false;
   WTabT wt;
   for (int i = 0; i < 40; ++i) wt.w[i] = (w && i <= 4 * S * S) ? w[i] : 0.f;
-  k_blur_tma<S, G><<<grid, G::NTHR, G::SMEM, st>>>(map, dst, d, tiles_x, wsum, wt, zero_border,
-                                                   err);
-  return true;
+  const BlurShape b = blur_shape(d);
+#define FLOF_BLUR(LW, RY) \
+  if (b.lw == LW && b.ry == RY) return launch_blur_shape<S, LW, RY>(src, dst, d, wsum, wt, zero_border, err, st, b)
+  FLOF_BLUR(32, 8);
+  FLOF_BLUR(16, 8);
+  FLOF_BLUR(8, 8);
+  FLOF_BLUR(32, 4);
+  FLOF_BLUR(16, 4);
+  FLOF_BLUR(8, 4);
+#undef FLOF_BLUR
+  return false;
 }
 
 }  // namespace
 
 bool launch_gauss_tma(const float4 *src, float4 *dst, Dims4 d, int s, const float *wtab,
                       const float *wsum_dev, int zero_border, int *err, cudaStream_t st) {
-  if (s == 1) return launch_blur<1, BlurGeom<1>>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
-  if (s == 2) return launch_blur<2, BlurGeom<2>>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
+  if (s == 1) return launch_blur<1>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
+  if (s == 2) return launch_blur<2>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
   return false;
 }
 
