@@ -141,8 +141,11 @@ const float *wsum_table(flof_ctx *c, float sigma, int s, const float *wtab) {
   return dptr;
 }
 
-// gaussianBlurGeneric(a, sigma, iter = 1) (optflow4d.cpp:160-174).
-void gauss_blur(flof_ctx *c, float *a, Dims4 d, int nc, float sigma, int blurType) {
+// gaussianBlurGeneric(a, sigma, iter = 1) (optflow4d.cpp:160-174).  Only the
+// cells of `keep` are wanted: the caller overwrites the others, which may hold
+// anything afterwards.
+void gauss_blur(flof_ctx *c, float *a, Dims4 d, int nc, float sigma, int blurType,
+                const CellBox &keep) {
   int s = trunc_d(1. * (double)sigma + 0.5);
   if (s == 0) s = 1;
   if (s > 6 || s < 0) fail(FLOF_E_ARG, "Gaussian blur radius above 6 cells is not supported");
@@ -160,10 +163,11 @@ void gauss_blur(flof_ctx *c, float *a, Dims4 d, int nc, float sigma, int blurTyp
         const float *src = pass == 0 ? a : tmp.f();
         float *dst = pass == 0 ? tmp.f() : a;
         const int zb = pass == 0 ? 1 : 0;
+        const CellBox box = pass == 0 ? grow_box(keep, d, s) : keep;
         bool tma = false;
         if (nc == 4 && c->slab_tma)
-          KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
-              tma = launch_gauss_tma((const float4 *)src, (float4 *)dst, d, s, wtab, ws, zb,
+          KLP(c, KC_BLUR, d.x, box.cells() * nc * 8,
+              tma = launch_gauss_tma((const float4 *)src, (float4 *)dst, d, s, wtab, ws, zb, box,
                                      c->dev_err, c->stream));
         if (!tma)
           KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
@@ -179,17 +183,32 @@ void gauss_blur(flof_ctx *c, float *a, Dims4 d, int nc, float sigma, int blurTyp
     float w1[8];
     for (int q = 0; q <= s; ++q)
       w1[q] = (float)exp((double)(-(float)(q * q)) / (2. * (double)sigma * (double)sigma));
-    // the reference's two passes: a -> t2 (zero ring), t2 -> a (ring kept)
+    // the reference's two passes: a -> t2 (zero ring), t2 -> a (ring kept); each
+    // kernel's box is what the next one's taps reach
     DBuf t1(c, nb), t2(c, nb);
-    KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
-        launch_gauss_sep_pair(a, t1.f(), d, nc, 0, s, w1, 0, c->stream));
-    KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
-        launch_gauss_sep_pair(t1.f(), t2.f(), d, nc, 1, s, w1, 1, c->stream));
-    KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
-        launch_gauss_sep_pair(t2.f(), t1.f(), d, nc, 0, s, w1, 0, c->stream));
-    KLP(c, KC_BLUR, d.x, d.cells() * nc * 8,
-        launch_gauss_sep_pair(t1.f(), a, d, nc, 1, s, w1, 2, c->stream));
+    const CellBox b2 = grow_box(keep, d, s, 12u), b1 = grow_box(keep, d, s);
+    const CellBox b0 = grow_box(b1, d, s, 12u);
+    KLP(c, KC_BLUR, d.x, b0.cells() * nc * 8,
+        launch_gauss_sep_pair(a, t1.f(), d, nc, 0, s, w1, 0, b0, c->stream));
+    KLP(c, KC_BLUR, d.x, b1.cells() * nc * 8,
+        launch_gauss_sep_pair(t1.f(), t2.f(), d, nc, 1, s, w1, 1, b1, c->stream));
+    KLP(c, KC_BLUR, d.x, b2.cells() * nc * 8,
+        launch_gauss_sep_pair(t2.f(), t1.f(), d, nc, 0, s, w1, 0, b2, c->stream));
+    KLP(c, KC_BLUR, d.x, keep.cells() * nc * 8,
+        launch_gauss_sep_pair(t1.f(), a, d, nc, 1, s, w1, 2, keep, c->stream));
   }
+}
+
+// The cells that isInBounds(b) keeps (b <= c < n - b on every axis).
+CellBox inner_box(Dims4 d, long long b) {
+  CellBox k = whole_box(d);
+  if (b < 0) return k;  // a width past the int range
+  for (int a = 0; a < 4; ++a) {
+    const int n = k.hi[a];
+    k.lo[a] = b < n ? (int)b : n;
+    k.hi[a] = n - b > k.lo[a] ? (int)(n - b) : k.lo[a];
+  }
+  return k;
 }
 
 struct OFArgs {
@@ -584,13 +603,14 @@ void optical_flow_dim(flof_ctx *c, Dims4 d, float4 *velOut, const float4 *velIn,
 
   KLP(c, KC_COPYBACK, d.x, d.cells() * 32,
       launch_of_copy_back(x.v(), velOut, d.cells(), k.mDx, c->st, c->stream));
+  const int rb = a.resetBndWidth > 0.f ? trunc_f(a.resetBndWidth * (float)d.x) + 1 : 0;
   if (a.postVelBlur > 0.f) {
     if (a.blurType != 1 && a.blurType != FLOF_BLUR_GAUSS_SEPARABLE)
       fail(FLOF_E_ARG, "blurType must be 1 (Gaussian) or 2 (separable Gaussian)");
-    gauss_blur(c, (float *)velOut, d, 4, (float)(0.5 * a.postVelBlur), a.blurType);
+    gauss_blur(c, (float *)velOut, d, 4, (float)(0.5 * a.postVelBlur), a.blurType,
+               a.resetBndWidth > 0.f ? inner_box(d, rb) : whole_box(d));
   }
   if (a.resetBndWidth > 0.f) {
-    const int rb = trunc_f(a.resetBndWidth * (float)d.x) + 1;
     KLP(c, KC_BORDER, d.x, 0, launch_reset_outside(velOut, d, rb, c->stream));
   }
 }
@@ -661,8 +681,10 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
       }
       std::swap(A, B);
     }
-    if (postVelBlur > 1e-6f) gauss_blur(c, (float *)A, d, 4, (float)(0.5 * postVelBlur), blurType);
     const int resetBnd = trunc_f(resetBndWidth * (float)d.x) + 1;
+    if (postVelBlur > 1e-6f)  // setBound zeroes c <= resetBnd and c >= n - 1 - resetBnd
+      gauss_blur(c, (float *)A, d, 4, (float)(0.5 * postVelBlur), blurType,
+                 resetBndWidth > 0.f ? inner_box(d, (long long)resetBnd + 1) : whole_box(d));
     if (resetBndWidth > 0.f)
       KLP(c, KC_BORDER, d.x, 0,
           launch_set_bound((float *)A, d, 4, make_float4(0.f, 0.f, 0.f, 0.f), resetBnd,
@@ -1525,7 +1547,7 @@ FLOF_API int flof_gaussianBlur4d(flof_ctx *c, flof_grid *a, float sigma, int blu
     need_4d(a, "grid");
     need(blurType == 1 || blurType == 2, "blurType must be 1 or 2");
     set_ctx_device(c);
-    gauss_blur(c, a->f(), a->D(), a->nc(), sigma, blurType);
+    gauss_blur(c, a->f(), a->D(), a->nc(), sigma, blurType, whole_box(a->D()));
     check_device_errors(c);
   });
 }

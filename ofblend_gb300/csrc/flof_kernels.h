@@ -310,6 +310,29 @@ void launch_of_copy_back(const float4 *x, float4 *vel, long long cells,
                          float mDx, const CGState *st, cudaStream_t s);
 
 // ---- Gaussian blur (gaussianBlurGeneric, strict 4D stencil) -----------------
+// The cells lo <= c < hi that a pass has to compute; others are left as they
+// are.  The velocity blurs are followed by a border reset that zeroes a tenth
+// of the extent on every side (at 64^4 only 37% of the cells survive it), so
+// the passes before it compute what the surviving cells depend on.
+struct CellBox {
+  int lo[4], hi[4];
+  long long cells() const {
+    long long n = 1;
+    for (int a = 0; a < 4; ++a) n *= hi[a] > lo[a] ? hi[a] - lo[a] : 0;
+    return n;
+  }
+};
+inline CellBox whole_box(Dims4 d) { return CellBox{{0, 0, 0, 0}, {d.x, d.y, d.z, d.t}}; }
+// the box grown by g cells along the axes of `axes` (bit a), within the grid
+inline CellBox grow_box(CellBox b, Dims4 d, int g, unsigned axes = 15u) {
+  const int n[4] = {d.x, d.y, d.z, d.t};
+  for (int a = 0; a < 4; ++a)
+    if (axes >> a & 1u) {
+      b.lo[a] = b.lo[a] - g > 0 ? b.lo[a] - g : 0;
+      b.hi[a] = b.hi[a] + g < n[a] ? b.hi[a] + g : n[a];
+    }
+  return b;
+}
 // One pass of knGaussianBlur over bnd=1 cells; when zero_border, the border
 // ring of dst is written with zeros.  wtab holds exp weights by squared
 // distance (host-computed, as the reference's float(exp(double))).
@@ -320,7 +343,8 @@ void launch_gauss_pass(const float *src, float *dst, Dims4 d, int nc, int s,
 // interior cells; border_mode 1 zeros the one-cell ring, 2 leaves it alone);
 // equal to the reference's blur up to rounding.
 void launch_gauss_sep_pair(const float *src, float *dst, Dims4 d, int nc, int zt, int s,
-                           const float *w1d, int border_mode, cudaStream_t st);
+                           const float *w1d, int border_mode, const CellBox &box,
+                           cudaStream_t st);
 
 // Shared-memory slab versions (flof_stencil.cu) of the blur pass for radius
 // 1 and 2 and of the extrapolation sweep; same results bit for bit.
@@ -343,7 +367,8 @@ constexpr int FLOF_DEV_ERR_TC_TIMEOUT = 2;
 // a block of the resident PCG whose bounded wait at a grid barrier ran out
 constexpr int FLOF_DEV_ERR_GRID_TIMEOUT = 3;
 bool launch_gauss_tma(const float4 *src, float4 *dst, Dims4 d, int s, const float *wtab,
-                      const float *wsum_dev, int zero_border, int *err, cudaStream_t st);
+                      const float *wsum_dev, int zero_border, const CellBox &box, int *err,
+                      cudaStream_t st);
 // The TMA extrapolation sweep writes only the cells it updates (unmarked
 // interior cells), so its output buffer must already hold the input's values
 // at every other cell (a copy of the input made once per projection round).

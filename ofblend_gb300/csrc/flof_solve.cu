@@ -768,21 +768,22 @@ __device__ __forceinline__ float4 sum_taps(const W1 &w, const float4 (&a)[2 * S 
   return scale4(v, inv);
 }
 
-// dst(x, y, z, t) = the y sum of the x sums, every cell.  A thread walks a
+// dst(x, y, z, t) = the y sum of the x sums, every cell of the box.  A thread walks a
 // run of y rows; the taps of the next row are loaded before the current
 // row's sums are formed.
 template <int NC, int S>
 __global__ void __launch_bounds__(NT)
-k_blur_sep_xy(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W1 w,
+k_blur_sep_xy(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W1 w, CellBox box,
               uint32_t n) {
   const idx_t sY = d.x;
+  const uint32_t ex = box.hi[0] - box.lo[0], ez = box.hi[2] - box.lo[2], et = box.hi[3] - box.lo[3];
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int x = (int)(q % (uint32_t)d.x);
-    uint32_t r = q / (uint32_t)d.x;
-    const int z = (int)(r % (uint32_t)d.z);
-    r /= (uint32_t)d.z;
-    const int t = (int)(r % (uint32_t)d.t);
-    const int ya = (int)(r / (uint32_t)d.t) * SEP_RUN, yb = min(ya + SEP_RUN, d.y);
+    const int x = box.lo[0] + (int)(q % ex);
+    uint32_t r = q / ex;
+    const int z = box.lo[2] + (int)(r % ez);
+    r /= ez;
+    const int t = box.lo[3] + (int)(r % et);
+    const int ya = box.lo[1] + (int)(r / et) * SEP_RUN, yb = min(ya + SEP_RUN, box.hi[1]);
     const idx_t plane = d.index(x, 0, z, t);
     const float ix = sep_inv<S>(w, x, d.x);
     float4 ring[2 * S + 1], a[2 * S + 1];
@@ -807,7 +808,7 @@ k_blur_sep_xy(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W
   }
 }
 
-// dst(x, y, z, t) = the t sum of the z sums at interior cells; border_mode 1
+// dst(x, y, z, t) = the t sum of the z sums at the box's interior cells; border_mode 1
 // writes zeros on the one-cell ring, 2 leaves it alone.  A block is 32 x
 // columns by SEP_ZB z planes at one y, so the z taps of a thread are mostly
 // its neighbours' cells, read through L1; each thread walks a run of t
@@ -815,19 +816,20 @@ k_blur_sep_xy(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W
 template <int NC, int S>
 __global__ void __launch_bounds__(NT)
 k_blur_sep_zt(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W1 w,
-              int border_mode, int xtiles, int ztiles, uint32_t nblocks) {
+              int border_mode, CellBox box, int xtiles, int ztiles, uint32_t nblocks) {
   const idx_t sZ = d.sz(), sT = d.st();
+  const uint32_t ey = box.hi[1] - box.lo[1];
   const int tx = threadIdx.x & 31, tz = threadIdx.x >> 5;
   for (uint32_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
     uint32_t r = b;
     const int xt = (int)(r % (uint32_t)xtiles);
     r /= (uint32_t)xtiles;
-    const int y = (int)(r % (uint32_t)d.y);
-    r /= (uint32_t)d.y;
+    const int y = box.lo[1] + (int)(r % ey);
+    r /= ey;
     const int zt = (int)(r % (uint32_t)ztiles);
-    const int ta = (int)(r / (uint32_t)ztiles) * SEP_RUN, tb = min(ta + SEP_RUN, d.t);
-    const int x = xt * 32 + tx, z = zt * SEP_ZB + tz;
-    if (x >= d.x || z >= d.z) continue;
+    const int ta = box.lo[3] + (int)(r / (uint32_t)ztiles) * SEP_RUN, tb = min(ta + SEP_RUN, box.hi[3]);
+    const int x = box.lo[0] + xt * 32 + tx, z = box.lo[2] + zt * SEP_ZB + tz;
+    if (x >= box.hi[0] || z >= box.hi[2]) continue;
     const idx_t col = d.index(x, y, z, 0);
     const bool ring_xyz = x < 1 || x >= d.x - 1 || y < 1 || y >= d.y - 1 || z < 1 || z >= d.z - 1;
     if (ring_xyz) {
@@ -863,38 +865,41 @@ k_blur_sep_zt(const float *__restrict__ src, float *__restrict__ dst, Dims4 d, W
 
 template <int NC, int S>
 void launch_sep_pair(const float *src, float *dst, Dims4 d, int zt, const W1 &w, int border_mode,
-                     cudaStream_t st) {
+                     const CellBox &box, cudaStream_t st) {
+  const long long ex = box.hi[0] - box.lo[0], ey = box.hi[1] - box.lo[1],
+                  ez = box.hi[2] - box.lo[2], et = box.hi[3] - box.lo[3];
   if (!zt) {
-    const uint32_t n = (uint32_t)((long long)d.x * d.z * d.t * ((d.y + SEP_RUN - 1) / SEP_RUN));
-    k_blur_sep_xy<NC, S><<<grid_for(n, NT, 8), NT, 0, st>>>(src, dst, d, w, n);
+    const uint32_t n = (uint32_t)(ex * ez * et * ((ey + SEP_RUN - 1) / SEP_RUN));
+    k_blur_sep_xy<NC, S><<<grid_for(n, NT, 8), NT, 0, st>>>(src, dst, d, w, box, n);
   } else {
-    const int xtiles = (d.x + 31) / 32, ztiles = (d.z + SEP_ZB - 1) / SEP_ZB;
-    const uint32_t nb =
-        (uint32_t)((long long)xtiles * d.y * ztiles * ((d.t + SEP_RUN - 1) / SEP_RUN));
+    const int xtiles = (int)(ex + 31) / 32, ztiles = (int)(ez + SEP_ZB - 1) / SEP_ZB;
+    const uint32_t nb = (uint32_t)(xtiles * ey * ztiles * ((et + SEP_RUN - 1) / SEP_RUN));
     const int grid = (int)std::min<long long>(nb, (long long)sm_count() * 8);
-    k_blur_sep_zt<NC, S><<<grid, 32 * SEP_ZB, 0, st>>>(src, dst, d, w, border_mode, xtiles, ztiles,
-                                                       nb);
+    k_blur_sep_zt<NC, S><<<grid, 32 * SEP_ZB, 0, st>>>(src, dst, d, w, border_mode, box, xtiles,
+                                                       ztiles, nb);
   }
 }
 template <int NC>
 void launch_sep_pair_nc(const float *src, float *dst, Dims4 d, int zt, int s, const W1 &w,
-                        int border_mode, cudaStream_t st) {
+                        int border_mode, const CellBox &box, cudaStream_t st) {
   switch (s) {
-    case 1: launch_sep_pair<NC, 1>(src, dst, d, zt, w, border_mode, st); break;
-    case 2: launch_sep_pair<NC, 2>(src, dst, d, zt, w, border_mode, st); break;
-    case 3: launch_sep_pair<NC, 3>(src, dst, d, zt, w, border_mode, st); break;
-    case 4: launch_sep_pair<NC, 4>(src, dst, d, zt, w, border_mode, st); break;
-    case 5: launch_sep_pair<NC, 5>(src, dst, d, zt, w, border_mode, st); break;
-    default: launch_sep_pair<NC, 6>(src, dst, d, zt, w, border_mode, st); break;
+    case 1: launch_sep_pair<NC, 1>(src, dst, d, zt, w, border_mode, box, st); break;
+    case 2: launch_sep_pair<NC, 2>(src, dst, d, zt, w, border_mode, box, st); break;
+    case 3: launch_sep_pair<NC, 3>(src, dst, d, zt, w, border_mode, box, st); break;
+    case 4: launch_sep_pair<NC, 4>(src, dst, d, zt, w, border_mode, box, st); break;
+    case 5: launch_sep_pair<NC, 5>(src, dst, d, zt, w, border_mode, box, st); break;
+    default: launch_sep_pair<NC, 6>(src, dst, d, zt, w, border_mode, box, st); break;
   }
 }
 
 void launch_gauss_sep_pair(const float *src, float *dst, Dims4 d, int nc, int zt, int s,
-                           const float *w1d, int border_mode, cudaStream_t st) {
+                           const float *w1d, int border_mode, const CellBox &box,
+                           cudaStream_t st) {
+  if (box.cells() == 0) return;
   W1 w;
   for (int q = 0; q < 7; ++q) w.w[q] = q <= s ? w1d[q] : 0.f;
-  if (nc == 4) launch_sep_pair_nc<4>(src, dst, d, zt, s, w, border_mode, st);
-  else launch_sep_pair_nc<1>(src, dst, d, zt, s, w, border_mode, st);
+  if (nc == 4) launch_sep_pair_nc<4>(src, dst, d, zt, s, w, border_mode, box, st);
+  else launch_sep_pair_nc<1>(src, dst, d, zt, s, w, border_mode, box, st);
 }
 
 // ---------------------------------------------------------------------------

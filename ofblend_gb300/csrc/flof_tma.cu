@@ -103,7 +103,7 @@ struct WTabT {
 // reference's (t, z) order; a thread computes RY consecutive rows of one
 // column, so every output adds its taps in the reference's sequence.  Slabs
 // outside the grid would add products of zero, which leave a running sum
-// unchanged, and are not visited.
+// unchanged, and are not visited.  The tiles cover the output box only.
 // Bound by the FP32 pipe: 625 ordered adds per component, plus the products
 // w * a, each rounded once as in the reference (mul2_rn) and formed once per
 // |yj| for the two rows that use it.  Keeping five output planes' sums, so that
@@ -122,7 +122,7 @@ template <int S, int LW, int RY>
 __global__ void __launch_bounds__(32 * BW_MAXW)
 k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Dims4 d, int tiles_x,
            const float *__restrict__ wsum, WTabT wt, unsigned long long nz, int zero_border,
-           int *err) {
+           CellBox box, int *err) {
   using G = BW<LW, RY>;
   constexpr int NS = BW_NS, NV = 2 * S + 1, W = LW + 2 * S;
   extern __shared__ __align__(128) unsigned char raw[];
@@ -130,8 +130,9 @@ k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
   __shared__ unsigned long long wsh[40];  // (w, w) pairs
   const int ty_rows = (int)(blockDim.x >> 5) * G::UNIT, h = ty_rows + 2 * S;
   const int stride = blur_stride(W, h);
-  const int x0 = (int)(blockIdx.x % tiles_x) * LW, y0 = (int)(blockIdx.x / tiles_x) * ty_rows;
-  const int z = blockIdx.y, t = blockIdx.z;
+  const int x0 = box.lo[0] + (int)(blockIdx.x % tiles_x) * LW;
+  const int y0 = box.lo[1] + (int)(blockIdx.x / tiles_x) * ty_rows;
+  const int z = box.lo[2] + (int)blockIdx.y, t = box.lo[3] + (int)blockIdx.z;
   const int lane = threadIdx.x & 31, lx = lane % LW, x = x0 + lx;
   const int row0 = ((int)(threadIdx.x >> 5) * G::RG + lane / LW) * RY;
   if (threadIdx.x == 0) {
@@ -207,14 +208,14 @@ k_blur_tma(const __grid_constant__ CUtensorMap map, float4 *__restrict__ dst, Di
       }
     }
 
-  if (x >= d.x) return;
+  if (x >= box.hi[0]) return;
   constexpr int P1 = (S + 1) * (S + 1);
   const bool zt_inner = z >= 1 && z < d.z - 1 && t >= 1 && t < d.t - 1;
   const int code_zt = (clip_code_t<S>(t, d.t) * P1 + clip_code_t<S>(z, d.z)) * P1;
 #pragma unroll
   for (int q = 0; q < RY; ++q) {
     const int y = y0 + row0 + q;
-    if (y >= d.y) continue;
+    if (y >= box.hi[1]) continue;
     const idx_t id = d.index(x, y, z, t);
     if (!(zt_inner && x >= 1 && x < d.x - 1 && y >= 1 && y < d.y - 1)) {
       if (zero_border) dst[id] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -665,12 +666,14 @@ struct BlurShape {
   int lw, ry, nw, ny;
 };
 // Of 32, 16 and 8 columns and 8 or 4 rows a thread, the tile that computes the
-// least: cells beyond the grid are computed like the others (tiles of 32 x 32
+// least: cells beyond the box are computed like the others (tiles of 32 x 32
 // computed 1.8 times the cells at 48^4, 2.6 times at 40^3), and the products
 // shared between rows make a row of 8 cheaper than one of 4 (175 against 190
 // pipe cycles a slab).  A grid with fewer than three warps per SM partition at
 // 8 rows takes 4, for more warps.
-BlurShape blur_shape(Dims4 d) {
+BlurShape blur_shape(const CellBox &box) {
+  const Dims4 d{box.hi[0] - box.lo[0], box.hi[1] - box.lo[1], box.hi[2] - box.lo[2],
+                box.hi[3] - box.lo[3]};
   BlurShape best = {32, 8, 4, 1};
   double bt = 0.0;
   for (int ry : {8, 4})
@@ -692,9 +695,10 @@ BlurShape blur_shape(Dims4 d) {
 
 template <int S, int LW, int RY>
 bool launch_blur_shape(const float4 *src, float4 *dst, Dims4 d, const float *wsum, const WTabT &wt,
-                       int zero_border, int *err, cudaStream_t st, const BlurShape &b) {
+                       int zero_border, const CellBox &box, int *err, cudaStream_t st,
+                       const BlurShape &b) {
   constexpr int W = LW + 2 * S, UNIT = BW<LW, RY>::UNIT;
-  const int tiles_x = (d.x + LW - 1) / LW, h = b.nw * UNIT + 2 * S;
+  const int tiles_x = (box.hi[0] - box.lo[0] + LW - 1) / LW, h = b.nw * UNIT + 2 * S;
   CUtensorMap map;
   if (!encode_slab_map(&map, src, d, W, h)) return false;
   static const bool attr = [] {
@@ -706,20 +710,22 @@ bool launch_blur_shape(const float4 *src, float4 *dst, Dims4 d, const float *wsu
     return true;
   }();
   if (!attr) return false;
-  k_blur_tma<S, LW, RY><<<dim3(tiles_x * b.ny, d.z, d.t), 32 * b.nw, BW_NS * blur_stride(W, h), st>>>(
-      map, dst, d, tiles_x, wsum, wt, 0x8000000080000000ull, zero_border, err);
+  const dim3 grid(tiles_x * b.ny, box.hi[2] - box.lo[2], box.hi[3] - box.lo[3]);
+  k_blur_tma<S, LW, RY><<<grid, 32 * b.nw, BW_NS * blur_stride(W, h), st>>>(
+      map, dst, d, tiles_x, wsum, wt, 0x8000000080000000ull, zero_border, box, err);
   return true;
 }
 
 template <int S>
 bool launch_blur(const float4 *src, float4 *dst, Dims4 d, const float *wsum, const float *w,
-                 int zero_border, int *err, cudaStream_t st) {
+                 int zero_border, const CellBox &box, int *err, cudaStream_t st) {
   if (d.z > 65535 || d.t > 65535) return false;
+  if (box.cells() == 0) return true;
   WTabT wt;
   for (int i = 0; i < 40; ++i) wt.w[i] = (w && i <= 4 * S * S) ? w[i] : 0.f;
-  const BlurShape b = blur_shape(d);
+  const BlurShape b = blur_shape(box);
 #define FLOF_BLUR(LW, RY) \
-  if (b.lw == LW && b.ry == RY) return launch_blur_shape<S, LW, RY>(src, dst, d, wsum, wt, zero_border, err, st, b)
+  if (b.lw == LW && b.ry == RY) return launch_blur_shape<S, LW, RY>(src, dst, d, wsum, wt, zero_border, box, err, st, b)
   FLOF_BLUR(32, 8);
   FLOF_BLUR(16, 8);
   FLOF_BLUR(8, 8);
@@ -733,9 +739,10 @@ bool launch_blur(const float4 *src, float4 *dst, Dims4 d, const float *wsum, con
 }  // namespace
 
 bool launch_gauss_tma(const float4 *src, float4 *dst, Dims4 d, int s, const float *wtab,
-                      const float *wsum_dev, int zero_border, int *err, cudaStream_t st) {
-  if (s == 1) return launch_blur<1>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
-  if (s == 2) return launch_blur<2>(src, dst, d, wsum_dev, wtab, zero_border, err, st);
+                      const float *wsum_dev, int zero_border, const CellBox &box, int *err,
+                      cudaStream_t st) {
+  if (s == 1) return launch_blur<1>(src, dst, d, wsum_dev, wtab, zero_border, box, err, st);
+  if (s == 2) return launch_blur<2>(src, dst, d, wsum_dev, wtab, zero_border, box, err, st);
   return false;
 }
 
