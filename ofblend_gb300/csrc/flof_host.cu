@@ -33,8 +33,8 @@ namespace {
 
 // interpolGridTempl (optflow4d.cpp:40-57): factor = Real(src)/target per
 // axis, offset = factor * 0.5.
-void interpol_grid(flof_ctx *c, float *target, Dims4 td, const float *source, Dims4 sd,
-                   int nc) {
+void interpol_grid(flof_ctx *c, float *target, Dims4 td, const float *source, Dims4 sd, int nc,
+                   float mul = 1.f) {
   const int sa[4] = {sd.x, sd.y, sd.z, sd.t}, ta[4] = {td.x, td.y, td.z, td.t};
   float fac[4], off[4];
   for (int q = 0; q < 4; ++q) {
@@ -43,7 +43,7 @@ void interpol_grid(flof_ctx *c, float *target, Dims4 td, const float *source, Di
   }
   KLP(c, KC_RESAMPLE, td.x, (td.cells() + sd.cells()) * nc * 4,
       launch_resample(target, td, source, sd, nc, make_float4(fac[0], fac[1], fac[2], fac[3]),
-                        make_float4(off[0], off[1], off[2], off[3]), c->stream));
+                        make_float4(off[0], off[1], off[2], off[3]), c->stream, mul));
 }
 
 // max |v| of a Vec4 grid (getMaxValue, grid4d.cpp:274-277), synchronising.
@@ -54,14 +54,19 @@ float vec_max_norm(flof_ctx *c, const float4 *v, Dims4 d) {
   return sqrtf(wait_value(c));
 }
 
+// max |v|^2 into c->fres[0], on the device
+void reduce_max(flof_ctx *c, const float4 *v, Dims4 d) {
+  KLP(c, KC_REDUCE, d.x, d.cells() * 16,
+      launch_reduce_minmax((const float *)v, d.cells(), 4, 0, c->fpart, c->counter + 4, c->fres + 0,
+                           c->stream));
+}
+
 // advectCflTemplate<Grid4d<int>,...> (optflow4d.cpp:2170-2180) ->
 // advectCflHelper4d (:1309-1321) with the solver dt = 1 and velFactor = 1
 // (a multiplication by 1 is exact, so the velocity copy is skipped).
 void advect_cfl(flof_ctx *c, Dims4 d, float cfl, const float4 *vel, float *grid, int nc) {
   if (!c->cfl_sync) {
-    KLP(c, KC_REDUCE, d.x, d.cells() * 16,
-        launch_reduce_minmax((const float *)vel, d.cells(), 4, 0, c->fpart, c->counter + 4,
-                             c->fres + 0, c->stream));
+    reduce_max(c, vel, d);
     DBuf tmp(c, (size_t)d.cells() * nc * sizeof(float));
     KLP(c, KC_ADVECT, d.x, d.cells() * (16 + 8 * nc),
         launch_advect_cfl1(vel, grid, tmp.f(), d, nc, c->fres + 0, cfl, c->cfl_flag, c->stream));
@@ -89,6 +94,22 @@ void advect_cfl(flof_ctx *c, Dims4 d, float cfl, const float4 *vel, float *grid,
                        cudaMemcpyDeviceToDevice, c->stream));
 }
 
+// dst = advect_cfl of src (which stays as it is).  max_ready: c->fres[0] holds
+// max |vel|^2 already.
+void advect_into(flof_ctx *c, Dims4 d, float cfl, const float4 *vel, const float *src, DBuf &dst,
+                 int nc, bool max_ready) {
+  const size_t nb = (size_t)d.cells() * nc * sizeof(float);
+  if (!dst.p) dst = DBuf(c, nb);
+  if (c->cfl_sync) {
+    CK(cudaMemcpyAsync(dst.p, src, nb, cudaMemcpyDeviceToDevice, c->stream));
+    advect_cfl(c, d, cfl, vel, dst.f(), nc);
+    return;
+  }
+  if (!max_ready) reduce_max(c, vel, d);
+  KLP(c, KC_ADVECT, d.x, d.cells() * (16 + 8 * nc),
+      launch_advect_cfl1(vel, src, dst.f(), d, nc, c->fres + 0, cfl, c->cfl_flag, c->stream));
+}
+
 // calcLsDiffTempl (optflow4d.cpp:895-927), synchronising.
 float ls_diff(flof_ctx *c, const float *i0, const float *i1, float *out, Dims4 d, float corr,
               int bnd) {
@@ -101,6 +122,26 @@ float ls_diff(flof_ctx *c, const float *i0, const float *i1, float *out, Dims4 d
       launch_ls_diff(i0, i1, out, d, corr, bnd, c->dpart, c->counter + 5, c->dres + 0, c->fres + 1,
                      c->stream, next_post(c)));
   return wait_value(c);
+}
+
+// The driver's warp and its error: dst = advect_cfl of src by vel, its Neumann
+// border, and calcLsDiff4d against i1; synchronising.
+float warp_error(flof_ctx *c, Dims4 d, float cfl, const float4 *vel, const float *src, DBuf &dst,
+                 const float *i1, float corr, int bnd, bool max_ready) {
+  if (!dst.p) dst = DBuf(c, real_bytes(d));
+  if (!c->cfl_sync && !c->strict) {
+    if (!max_ready) reduce_max(c, vel, d);
+    max_ready = true;
+    bool done = false;
+    KLP(c, KC_ADVECT, d.x, d.cells() * 28,
+        done = launch_warp_error(vel, src, dst.f(), i1, d, c->fres + 0, cfl, c->cfl_flag, corr, bnd,
+                                 c->dpart, c->counter + 5, c->dres + 0, c->fres + 1, c->stream,
+                                 next_post(c)));
+    if (done) return wait_value(c);
+  }
+  advect_into(c, d, cfl, vel, src, dst, 1, max_ready);
+  KLP(c, KC_BORDER, d.x, 0, launch_set_bound_neumann(dst.f(), d, 1, 0, c->stream));
+  return ls_diff(c, dst.f(), i1, nullptr, d, corr, bnd);
 }
 
 // In-bounds weight sums of knGaussianBlur by clipping pattern: per axis the
@@ -729,20 +770,15 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
   oa.solver = p.solver;
 
   DBuf i0warped(c, real_bytes(d));
-  CK(cudaMemcpyAsync(i0warped.p, i0, real_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
 
   if (d.x > p.minGridSize) {
     Dims4 sd{d.x / 2, d.y / 2, d.z / 2, d.t / 2};
     DBuf velSm(c, vec_bytes(sd)), i0Sm(c, real_bytes(sd)), i1Sm(c, real_bytes(sd));
     interpol_grid(c, i0Sm.f(), sd, i0, d, 1);
     interpol_grid(c, i1Sm.f(), sd, i1, d, 1);
-    interpol_grid(c, velSm.f(), sd, (const float *)vel, d, 4);
-    KL(c, launch_mult_const(velSm.f(), sd.cells(), 4, make_float4(0.5f, 0.5f, 0.5f, 0.5f),
-                            c->stream));
+    interpol_grid(c, velSm.f(), sd, (const float *)vel, d, 4, 0.5f);
     multiscale(c, sd, velSm.v(), i0Sm.f(), i1Sm.f(), p, level + 1);
-    interpol_grid(c, (float *)vel, d, velSm.f(), sd, 4);
-    KL(c, launch_mult_const((float *)vel, d.cells(), 4, make_float4(2.f, 2.f, 2.f, 2.f),
-                            c->stream));
+    interpol_grid(c, (float *)vel, d, velSm.f(), sd, 4, 2.f);
   }
 
   if (p.warmStart && !(d.x > p.minGridSize) && c->model) {
@@ -754,12 +790,8 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
       model_predict_raw(c->model, i0, i1, pred.v());
       float err[2];
       const float4 *cand[2] = {vel, pred.v()};
-      for (int q = 0; q < 2; ++q) {
-        CK(cudaMemcpyAsync(tmp.p, i0, real_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
-        advect_cfl(c, d, p.cfl, cand[q], tmp.f(), 1);
-        KLP(c, KC_BORDER, d.x, 0, launch_set_bound_neumann(tmp.f(), d, 1, 0, c->stream));
-        err[q] = ls_diff(c, tmp.f(), i1, nullptr, d, lsDiffFac, resetBnd);
-      }
+      for (int q = 0; q < 2; ++q)
+        err[q] = warp_error(c, d, p.cfl, cand[q], i0, tmp, i1, lsDiffFac, resetBnd, false);
       const bool use = err[1] < err[0];
       if (use) CK(cudaMemcpyAsync(vel, pred.p, vec_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
       if (c->stats) {
@@ -770,9 +802,7 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
     }
   }
 
-  advect_cfl(c, d, p.cfl, vel, i0warped.f(), 1);
-  KLP(c, KC_BORDER, d.x, 0, launch_set_bound_neumann(i0warped.f(), d, 1, 0, c->stream));
-  float errCurr = ls_diff(c, i0warped.f(), i1, nullptr, d, lsDiffFac, resetBnd);
+  float errCurr = warp_error(c, d, p.cfl, vel, i0, i0warped, i1, lsDiffFac, resetBnd, false);
 
   bool doProject = false;
   int multiStep = p.multiStep;
@@ -785,9 +815,11 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
   if (multiStep >= 10) fail(FLOF_E_ARG, "Too many of substeps!");
 
   if (multiStep > 1) {
+    // vs2[k] is the step k's velocity carried through the later steps; a step
+    // that nothing has carried yet is read from vs[k] itself
     std::vector<DBuf> vs(multiStep), vs2(multiStep);
-    for (int of = 0; of < multiStep; ++of) vs2[of] = DBuf(c, vec_bytes(d));
-    DBuf tmpVel(c, vec_bytes(d)), i0warp2(c, real_bytes(d));
+    std::vector<const float4 *> cur(multiStep), terms(multiStep);
+    DBuf tmpVel(c, vec_bytes(d)), i0warp2(c, real_bytes(d)), carried;
     float velBlur = p.postVelBlur;
     float errLast = errCurr;
     int ofStepsCurr = multiStep;
@@ -798,20 +830,21 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
       optical_flow_dim(c, d, vs[of].v(), nullptr, i0warped.f(), i1, oa, nullptr, nullptr);
       velBlur = (float)((double)velBlur * (3. / 4.));
       if (velBlur < 2.f) velBlur = 2.f;
-      for (int k = of; k >= 0; --k)
-        CK(cudaMemcpyAsync(vs2[k].p, vs[k].p, vec_bytes(d), cudaMemcpyDeviceToDevice,
-                           c->stream));
+      for (int k = of; k >= 0; --k) cur[k] = vs[k].v();
       for (int k = of - 1; k >= 0; --k)
-        for (int l = 0; l < k; ++l) advect_cfl(c, d, p.cfl, vs2[k].v(), vs2[l].f(), 4);
-      CK(cudaMemcpyAsync(tmpVel.p, vel, vec_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
-      for (int k = of; k >= 0; --k)
-        KLP(c, KC_ELEMWISE, d.x, n4 * 12, launch_add(tmpVel.f(), vs2[k].f(), n4, c->stream));
-      CK(cudaMemcpyAsync(i0warp2.p, i0, real_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
-      advect_cfl(c, d, p.cfl, tmpVel.v(), i0warp2.f(), 1);
-      KLP(c, KC_BORDER, d.x, 0, launch_set_bound_neumann(i0warp2.f(), d, 1, 0, c->stream));
-      const float errC = ls_diff(c, i0warp2.f(), i1, nullptr, d, lsDiffFac, resetBnd);
-      CK(cudaMemcpyAsync(i0warped.p, i0warp2.p, real_bytes(d), cudaMemcpyDeviceToDevice,
-                         c->stream));
+        for (int l = 0; l < k; ++l) {
+          advect_into(c, d, p.cfl, cur[k], (const float *)cur[l], carried, 4, l > 0);
+          std::swap(vs2[l], carried);
+          cur[l] = vs2[l].v();
+        }
+      // tmpVel = vel + vs2[of] + ... + vs2[0] and its maximum norm
+      for (int k = of; k >= 0; --k) terms[of - k] = cur[k];
+      KLP(c, KC_ELEMWISE, d.x, d.cells() * 16 * (of + 3),
+          launch_vec_sum(tmpVel.v(), vel, terms.data(), of + 1, d.cells(), c->fpart, c->counter + 4,
+                         c->fres + 0, c->stream));
+      const float errC =
+          warp_error(c, d, p.cfl, tmpVel.v(), i0, i0warp2, i1, lsDiffFac, resetBnd, true);
+      std::swap(i0warped, i0warp2);
       if (of > 0 && (double)(errC / errLast) > 0.95) {
         CK(cudaMemsetAsync(vs[of].p, 0, vec_bytes(d), c->stream));
         ofStepsCurr = of + 1;
@@ -819,9 +852,14 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
       errLast = errC;
     }
     for (int of = ofStepsCurr - 1; of >= 0; --of)
-      for (int l = 0; l < of; ++l) advect_cfl(c, d, p.cfl, vs[of].v(), vs[l].f(), 4);
-    for (int of = 0; of < ofStepsCurr; ++of)
-      KLP(c, KC_ELEMWISE, d.x, n4 * 12, launch_add((float *)vel, vs[of].f(), n4, c->stream));
+      for (int l = 0; l < of; ++l) {
+        advect_into(c, d, p.cfl, vs[of].v(), vs[l].f(), carried, 4, l > 0);
+        std::swap(vs[l], carried);
+      }
+    for (int of = 0; of < ofStepsCurr; ++of) terms[of] = vs[of].v();
+    KLP(c, KC_ELEMWISE, d.x, d.cells() * 16 * (ofStepsCurr + 2),
+        launch_vec_sum(vel, vel, terms.data(), ofStepsCurr, d.cells(), c->fpart, c->counter + 4,
+                       nullptr, c->stream));
   } else {
     DBuf velCurr(c, vec_bytes(d));
     if (!doProject) {
@@ -847,12 +885,8 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
                  projMaxIter, p.blurType);
   }
 
-  if (level == 0) {
-    CK(cudaMemcpyAsync(i0warped.p, i0, real_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
-    advect_cfl(c, d, p.cfl, vel, i0warped.f(), 1);
-    KLP(c, KC_BORDER, d.x, 0, launch_set_bound_neumann(i0warped.f(), d, 1, 0, c->stream));
-    errCurr = ls_diff(c, i0warped.f(), i1, nullptr, d, lsDiffFac, resetBnd);
-  }
+  if (level == 0)
+    errCurr = warp_error(c, d, p.cfl, vel, i0, i0warped, i1, lsDiffFac, resetBnd, false);
   return errCurr;
 }
 

@@ -65,6 +65,12 @@ struct HostPost {
 void launch_reduce_minmax(const float *a, long long ncell, int nc, int which,
                           float *partials, unsigned int *counter, float *result,
                           cudaStream_t s, HostPost post = HostPost());
+// out = ((base + terms[0]) + terms[1]) + ... over ncell Vec4 cells (out may be
+// base); result (nullable): max |out|^2.
+constexpr int VEC_SUM_MAX = 9;
+void launch_vec_sum(float4 *out, const float4 *base, const float4 *const *terms, int nt,
+                    long long ncell, float *partials, unsigned int *counter, float *result,
+                    cudaStream_t s);
 // calcLsDiffTempl sum over the bnd box (double), scaled as the reference
 // does; result as double and as float.
 void launch_ls_diff(const float *i0, const float *i1, float *out, Dims4 d,
@@ -74,8 +80,9 @@ void launch_ls_diff(const float *i0, const float *i1, float *out, Dims4 d,
 int ls_diff_blocks(Dims4 d, int bnd);
 
 // ---- resampling / advection ---------------------------------------------------
+// (target times mul, rounded after the sample)
 void launch_resample(float *target, Dims4 td, const float *source, Dims4 sd,
-                     int nc, float4 fac, float4 off, cudaStream_t s);
+                     int nc, float4 fac, float4 off, cudaStream_t s, float mul = 1.f);
 // dst (fresh) = src sampled at ijkt+0.5 - vel*dt over bnd=1 cells; the
 // border ring of dst is written with zeros.
 void launch_advect(const float4 *vel, const float *src, float *dst, Dims4 d,
@@ -85,6 +92,14 @@ void launch_advect(const float4 *vel, const float *src, float *dst, Dims4 d,
 // int(maxVel/cfl)+1 != 1.
 void launch_advect_cfl1(const float4 *vel, const float *src, float *dst, Dims4 d, int nc,
                         const float *maxn2, float cfl, int *flag, cudaStream_t s);
+// dst = advection (one substep, as launch_advect_cfl1), setBoundNeumann(0) and
+// calcLsDiff4d against i1 over the bnd box, in one pass; dst must not be src.
+// False when an extent is below 3 (the ring's source cells would not lie inside
+// it): the caller then runs the three in turn.
+bool launch_warp_error(const float4 *vel, const float *src, float *dst, const float *i1, Dims4 d,
+                       const float *maxn2, float cfl, int *flag, float correction, int bnd,
+                       double *partials, unsigned int *counter, double *result_d, float *result_f,
+                       cudaStream_t s, HostPost post);
 // Two-way blend of deform4d (scenes/flof.py:603-610) in one pass:
 // out = (advect(vel,i0,a) * (1-a)) + a * advect(velInv,i1,1-a).
 void launch_deform_twoway(const float4 *vel, const float4 *velInv,

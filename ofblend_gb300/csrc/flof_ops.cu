@@ -264,6 +264,54 @@ void launch_reduce_minmax(const float *a, long long ncell, int nc, int which,
     k_reduce_minmax<1><<<nb, NT, 0, s>>>(a, ncell, nc, partials, counter, result, post);
 }
 
+// out = ((base + t[0]) + t[1]) + ..., each add rounded on its own, in one pass;
+// with `result`, max |out|^2 as k_reduce_minmax<0> forms it.  out may be base.
+struct VecTerms {
+  const float4 *t[VEC_SUM_MAX];
+};
+__global__ void __launch_bounds__(NT)
+k_vec_sum(float4 *out, const float4 *base, VecTerms terms, int nt, long long n, float *partials,
+          unsigned int *counter, float *result) {
+  __shared__ float sh[NT / 32];
+  float acc = -FLT_MAX;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    float4 v = base[i];
+    for (int k = 0; k < nt; ++k) {
+      const float4 y = __ldg(terms.t[k] + i);
+      v.x += y.x;
+      v.y += y.y;
+      v.z += y.z;
+      v.w += y.w;
+    }
+    out[i] = v;
+    const float m = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;  // normSquare
+    if (m > acc) acc = m;
+  }
+  if (!result) return;
+  const float b = block_max<NT>(acc, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = b;
+  if (last_block_arrives(counter)) {
+    float m = -FLT_MAX;
+    for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
+      const float v = __ldcg(partials + q);
+      if (v > m) m = v;
+    }
+    m = block_max<NT>(m, sh);
+    if (threadIdx.x == 0) {
+      *result = m;
+      *counter = 0;
+    }
+  }
+}
+void launch_vec_sum(float4 *out, const float4 *base, const float4 *const *terms, int nt,
+                    long long ncell, float *partials, unsigned int *counter, float *result,
+                    cudaStream_t s) {
+  VecTerms v;
+  for (int k = 0; k < VEC_SUM_MAX; ++k) v.t[k] = k < nt ? terms[k] : nullptr;
+  k_vec_sum<<<grid_for(ncell, NT), NT, 0, s>>>(out, base, v, nt, ncell, partials, counter, result);
+}
+
 // calcLsDiffTempl (optflow4d.cpp:895-927).  Four cells per trip, all loads
 // first: a small grid then needs a quarter of the blocks, whose partials the
 // last block sums, and still has its loads in flight together.
@@ -367,7 +415,7 @@ static int planes_per_thread(long long cells, int most) {
 template <int NC>
 __global__ void __launch_bounds__(NT, 6)
 k_resample(float *__restrict__ target, Dims4 td, BoxDecoder bx, uint32_t n, int tt,
-           const float *__restrict__ source, Dims4 sd, float4 fac, float4 off) {
+           const float *__restrict__ source, Dims4 sd, float4 fac, float4 off, float mul) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   int i, j, k, tc;
@@ -391,7 +439,9 @@ k_resample(float *__restrict__ target, Dims4 td, BoxDecoder bx, uint32_t n, int 
         b = plane_vec(src, c, p + (uint32_t)c.sT, ax, ay, az);
         have = at.b;
       }
-      ((float4 *)target)[id] = weigh2(a, b, at);
+      float4 v = weigh2(a, b, at);
+      if (mul != 1.f) v = make_float4(v.x * mul, v.y * mul, v.z * mul, v.w * mul);
+      ((float4 *)target)[id] = v;
     }
   } else {
     const Corner c = corner_of(sd, ax.b, ay.b, az.b, 0);
@@ -404,20 +454,21 @@ k_resample(float *__restrict__ target, Dims4 td, BoxDecoder bx, uint32_t n, int 
         b = plane_real(source, c, p + (uint32_t)c.sT, ax, ay, az);
         have = at.b;
       }
-      target[id] = a * at.w0 + b * at.w1;
+      const float v = a * at.w0 + b * at.w1;
+      target[id] = mul != 1.f ? v * mul : v;
     }
   }
 }
 void launch_resample(float *target, Dims4 td, const float *source, Dims4 sd,
-                     int nc, float4 fac, float4 off, cudaStream_t s) {
+                     int nc, float4 fac, float4 off, cudaStream_t s, float mul) {
   if (td.cells() <= 0) return;
   BoxDecoder bx = make_decoder(td.x, td.y, td.z, 0, 0, 0, 0);
   const int tt = planes_per_thread(td.cells(), RS_TT);
   const uint32_t n = (uint32_t)(td.st() * ((td.t + tt - 1) / tt));
   if (nc == 4)
-    k_resample<4><<<grid_all(n), NT, 0, s>>>(target, td, bx, n, tt, source, sd, fac, off);
+    k_resample<4><<<grid_all(n), NT, 0, s>>>(target, td, bx, n, tt, source, sd, fac, off, mul);
   else
-    k_resample<1><<<grid_all(n), NT, 0, s>>>(target, td, bx, n, tt, source, sd, fac, off);
+    k_resample<1><<<grid_all(n), NT, 0, s>>>(target, td, bx, n, tt, source, sd, fac, off, mul);
 }
 
 // ---------------------------------------------------------------------------
@@ -475,6 +526,87 @@ void launch_advect(const float4 *vel, const float *src, float *dst, Dims4 d,
 void launch_advect_cfl1(const float4 *vel, const float *src, float *dst, Dims4 d, int nc,
                         const float *maxn2, float cfl, int *flag, cudaStream_t s) {
   advect_any(vel, src, dst, d, nc, (1.0f / (float)1) * 1.0f, maxn2, cfl, flag, s);
+}
+
+// The driver's warp in one pass: dst = the single-substep advection of src
+// (k_advect with maxn2), setBoundNeumann(0) of it, and calcLsDiff4d of the
+// result against i1 over the bnd box.  A cell of the outermost ring takes the
+// value of its source cell, which lies inside it (every extent at least 3), by
+// advecting that cell itself: the same operations, so the same bits as copying
+// it afterwards.  One pass instead of four over the
+// grid and, for a small level, one launch instead of four.
+__global__ void __launch_bounds__(NT)
+k_warp_error(const float4 *__restrict__ vel, const float *__restrict__ src, float *__restrict__ dst,
+             const float *__restrict__ i1, Dims4 d, BoxDecoder bx, const float *maxn2, float cfl,
+             int *flag, float correction, int bnd, double scale, double *partials,
+             unsigned int *counter, double *result_d, float *result_f, HostPost post) {
+  __shared__ double sh[NT / 32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const float maxVel = sqrtf(*maxn2) * 1.0f;
+    const int steps = trunc_i(maxVel / cfl) + 1;
+    if (steps != 1) *flag = 1;
+  }
+  double acc = 0.0;
+  const uint32_t n = (uint32_t)d.cells();
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    int c[4];
+    bx.decode(q, c[0], c[1], c[2], c[3]);
+    const bool box = in_bounds(d, c[0], c[1], c[2], c[3], bnd);
+    const int ext[4] = {d.x, d.y, d.z, d.t};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int o = c[a];
+      if (o <= 0) c[a] = 1;
+      if (o >= ext[a] - 1) c[a] = ext[a] - 2;
+    }
+    const float4 v = __ldg(vel + d.index(c[0], c[1], c[2], c[3]));
+    const float dt = 1.0f;
+    const float w = interp4_real(src, d, (float)(c[0] + 0.5f) - v.x * dt,
+                                 (float)(c[1] + 0.5f) - v.y * dt, (float)(c[2] + 0.5f) - v.z * dt,
+                                 (float)(c[3] + 0.5f) - v.w * dt);
+    dst[q] = w;
+    if (box) {
+      const float b = __ldg(i1 + q);
+      if (!((w < 0.f && b < 0.f) || (w >= 0.f && b >= 0.f))) {
+        float dd = fabsf(w - b) * correction;
+        if (dd > 1.f) dd = 1.f;
+        acc += (double)dd;
+      }
+    }
+  }
+  double b = block_sum<NT>(acc, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = b;
+  if (last_block_arrives(counter)) {
+    double m = 0.0;
+    for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) m += __ldcg(partials + q);
+    m = block_sum<NT>(m, sh);
+    if (threadIdx.x == 0) {
+      double accu = m * 1000.;
+      if (d.t > 1) accu *= 1000.;
+      accu *= scale;
+      *result_d = accu;
+      *result_f = (float)accu;
+      *counter = 0;
+      post_value(post, (float)accu);
+    }
+  }
+}
+bool launch_warp_error(const float4 *vel, const float *src, float *dst, const float *i1, Dims4 d,
+                       const float *maxn2, float cfl, int *flag, float correction, int bnd,
+                       double *partials, unsigned int *counter, double *result_d, float *result_f,
+                       cudaStream_t s, HostPost post) {
+  if (d.x < 3 || d.y < 3 || d.z < 3 || d.t < 3) return false;
+  static const int per_sm = [] {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_warp_error, NT, 0);
+    return n < 1 ? 1 : n;
+  }();
+  const int ex = d.x - 2 * bnd, ey = d.y - 2 * bnd, ez = d.z - 2 * bnd, et = d.t - 2 * bnd;
+  const int cnt = ex * ey * ez * et;  // as launch_ls_diff
+  k_warp_error<<<grid_for(d.cells(), NT, per_sm), NT, 0, s>>>(
+      vel, src, dst, i1, d, make_decoder(d.x, d.y, d.z, 0, 0, 0, 0), maxn2, cfl, flag, correction,
+      bnd, 1. / (double)cnt, partials, counter, result_d, result_f, post);
+  return true;
 }
 
 // Bound by instruction issue (about 330 per cell, most of them index and
