@@ -477,7 +477,10 @@ int mg_pcg(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, const OFAr
                        c->stream, &vl));
   KLP(c, KC_DIRECTION, d.x, nb * 32, launch_mgcg_direction(p, z.v(), d, c->st, 1, c->stream));
   const int cap = a.cgMaxIter < mp.max_iter ? a.cgMaxIter : mp.max_iter;
-  int it = 0, chunk = 2;
+  // An iteration past the last one is some twenty launches that return at once
+  // (50 us at 64^4), so after a first chunk the next one is what the reduction so
+  // far asks for: 7 or 8 iterations are queued for 7, where doubling queued 14.
+  int it = 0, chunk = 4;
   for (;;) {
     const int n = (cap - it) < chunk ? (cap - it) : chunk;
     for (int s = 0; s < n; ++s) {
@@ -494,7 +497,11 @@ int mg_pcg(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, const OFAr
     CK(cudaMemcpyAsync(c->st_h, c->st, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream));
     sync(c);
     if (c->st_h->done != CG_RUNNING || it >= cap) break;
-    chunk = chunk * 2 > 16 ? 16 : chunk * 2;
+    const double ratio = (double)c->st_h->resMax / c->st_h->resIni;
+    const double target = c->st_h->acc / c->st_h->resIni;
+    const double rate = ratio > 0 && ratio < 1 && target > 0 ? log(ratio) / it : 0.0;
+    const double est = rate < 0 ? (log(target) - log(ratio)) / rate + 0.8 : 2.0 * chunk;
+    chunk = est < 1 ? 1 : est > 16 ? 16 : (int)est;
   }
   c->launches += vl;
   int status = c->st_h->done;
