@@ -160,7 +160,6 @@ struct OFConsts {
   float diag;       // 8 wSmooth mDx2Inv + wEnergy
 };
 
-int cg_blocks(Dims4 d);
 // Launch shapes of the PCG kernels, chosen per grid size by the autotuner
 // (defaults otherwise): t planes per matvec work item (4, 8 or 16) and
 // resident blocks per SM of the update / direction kernels.

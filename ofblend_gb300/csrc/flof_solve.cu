@@ -23,11 +23,6 @@ constexpr int NT = 256;
 // Assembly + PCG initialisation
 // ---------------------------------------------------------------------------
 
-int cg_blocks(Dims4 d) {
-  long long n = (long long)(d.x - 2) * (d.y - 2) * (d.z - 2) * (d.t - 2);
-  return grid_for(n > 0 ? n : 1, NT, 8);
-}
-
 static inline BoxDecoder interior_decoder(Dims4 d) {
   return make_decoder(d.x - 2 > 0 ? d.x - 2 : 1, d.y - 2 > 0 ? d.y - 2 : 1,
                       d.z - 2 > 0 ? d.z - 2 : 1, 1, 1, 1, 1);
@@ -160,7 +155,9 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
                              float4 *p, float4 *x, Dims4 d, OFConsts c,
                              float accuracy, CGState *st, double *dpart,
                              float *fpart, cudaStream_t s) {
-  k_of_assemble_init<<<cg_blocks(d), NT, 0, s>>>(
+  // five blocks per SM are resident: a single wave (mean over the levels of a
+  // 64^4 solve 82 us; 8 per SM 95, 10 per SM 90, one trip per thread 172)
+  k_of_assemble_init<<<grid_for(d.cells(), NT, 5), NT, 0, s>>>(
       i0w, i1, vel, g, r, p, x, d, make_decoder(d.x, d.y, d.z, 0, 0, 0, 0),
       (uint32_t)d.cells(), c, accuracy, st, dpart, fpart);
 }
@@ -998,7 +995,11 @@ __device__ __forceinline__ void project_write(float4 *__restrict__ dst, float *_
 // and the start of the search.  Cells with a zero normal (flat, clamped phi)
 // finish here; the others are appended to `queue` (warp-aggregated, in no
 // fixed order) for k_project_search.
-__global__ void __launch_bounds__(128, 5)
+// One trip per thread: a capped grid of 16 blocks per SM with 5 or 6 resident
+// ended in a mostly empty wave (64^4: 808 us with 5 blocks of 96 registers and
+// that grid, 729 with the blocks refilled as they end, 690 with 6 blocks per SM;
+// 8 per SM 696).
+__global__ void __launch_bounds__(128, 6)
 k_project_prep(float4 *__restrict__ dst, const float4 *__restrict__ vel,
                const float *__restrict__ phiOrg, const float *__restrict__ phiTarget,
                float *__restrict__ marker, Dims4 d, BoxDecoder bx, uint32_t nbox,
@@ -1232,9 +1233,9 @@ void launch_project_cells(float4 *dst, const float4 *vel, const float *phiOrg,
     const BoxDecoder bx = make_decoder(d.x - 4, d.y - 4, d.z - 4, 2, 2, 2, 2 + t0);
     const long long nbox = vol * nt;
     if (t0 > 0) k_zero_counters<<<1, 1, 0, s>>>(counters);
-    k_project_prep<<<grid_for(nbox, 128, 16), 128, 0, s>>>(dst, vel, phiOrg, phiTarget, marker,
-                                                           d, bx, (uint32_t)nbox, threshPhi,
-                                                           maxIter, (ProjState *)queue, counters);
+    k_project_prep<<<(unsigned)((nbox + 127) / 128), 128, 0, s>>>(
+        dst, vel, phiOrg, phiTarget, marker, d, bx, (uint32_t)nbox, threshPhi, maxIter,
+        (ProjState *)queue, counters);
     k_project_search<<<sm_count() * per_sm, 128, 0, s>>>(dst, phiOrg, marker, d, threshPhi,
                                                          maxIter, (const ProjState *)queue,
                                                          counters, counters + 1);
