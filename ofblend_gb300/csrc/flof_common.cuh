@@ -342,12 +342,12 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 // starts with pdl_wait).  Falls back to an ordinary launch if the attribute is
 // refused.
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*k)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
-                       Args... args) {
+inline void launch_pdl_smem(void (*k)(KArgs...), dim3 grid, unsigned block, size_t smem,
+                            cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -356,8 +356,13 @@ inline void launch_pdl(void (*k)(KArgs...), unsigned grid, unsigned block, cudaS
   cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, k, args...) != cudaSuccess) {
     cudaGetLastError();
-    k<<<grid, block, 0, s>>>(args...);
+    k<<<grid, block, smem, s>>>(args...);
   }
+}
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*k)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
+                       Args... args) {
+  launch_pdl_smem(k, dim3(grid), block, 0, s, args...);
 }
 
 // ---- reductions -----------------------------------------------------------

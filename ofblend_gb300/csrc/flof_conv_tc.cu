@@ -58,6 +58,7 @@ struct TcArgs {
   int M, N, K, Kpad;      // rows, columns, reduction length, WT row length
   int relu, kslice, ncols;
   int bias_row;           // MODE 2: the last row is all ones (the bias gradient)
+  NetGradEpi epi;         // MODE 1, unsplit only
 };
 
 // A tap of the reduction: its source voxel is the row's voxel plus `off`
@@ -303,8 +304,13 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
     fill_vtab(vtab[1], tid, kbeg, 1, nch, kend, rout, rin, p.stride, p.cin);
   }
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  // the tables above come from the arguments alone; from here on the operands
+  // are read.  The next grid is let in when every block of this one holds its
+  // tensor memory.
+  pdl_wait();
   fence_before_sync();
   __syncthreads();
+  pdl_launch_dependents();
   fence_after_sync();
   const uint32_t tacc = tbase;
   const uint32_t idesc = idesc_bf16_f32(TB_M, N);
@@ -471,6 +477,27 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
             v[j] = p.relu && y < 0.f ? 0.f : y;
           }
         }
+        if (!split && MODE == 1) {
+          const float4 *add = reinterpret_cast<const float4 *>(
+              p.epi.add ? p.epi.add + orow * p.epi.addp + c0 : nullptr);
+          const float4 *mask =
+              reinterpret_cast<const float4 *>(p.epi.mask ? p.epi.mask + orow * N + c0 : nullptr);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (add) {
+              const float4 w = __ldg(add + q);
+              v[4 * q] = w.x + v[4 * q], v[4 * q + 1] = w.y + v[4 * q + 1];
+              v[4 * q + 2] = w.z + v[4 * q + 2], v[4 * q + 3] = w.w + v[4 * q + 3];
+            }
+            if (mask) {
+              const float4 w = __ldg(mask + q);
+              v[4 * q] = w.x > 0.f ? v[4 * q] : 0.f;
+              v[4 * q + 1] = w.y > 0.f ? v[4 * q + 1] : 0.f;
+              v[4 * q + 2] = w.z > 0.f ? v[4 * q + 2] : 0.f;
+              v[4 * q + 3] = w.w > 0.f ? v[4 * q + 3] : 0.f;
+            }
+          }
+        }
         float4 *dst = reinterpret_cast<float4 *>(C + orow * N + c0);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -486,18 +513,85 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
   }
 }
 
-// out[m][n] = sum over the slices (in order) + bias[n], then ReLU
-__global__ void k_sum_slices_epi(const float *__restrict__ work, float *__restrict__ out,
-                                 long long n, int nz, int N, const float *__restrict__ bias,
-                                 int relu) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int z = 0; z < nz; ++z) s += work[(size_t)z * n + q];
-    if (bias) s += bias[q % N];
-    if (relu && s < 0.f) s = 0.f;
-    out[q] = s;
+// What a sum of slices becomes as it is stored: forward: bias and ReLU; input
+// gradient: NetGradEpi; weight gradient: added to what is there (acc).
+struct SumEpi {
+  const float *bias;
+  int relu, acc;
+  NetGradEpi grad;
+};
+
+// out[m][n] = sum over the slices + epilogue, four columns per thread.  GRP
+// threads (of different warps) share an entry's slices, thread g adding g, g +
+// GRP, ... in order, and thread 0 adds the GRP sums in order: with one thread
+// per entry the two-channel layer's weight gradient (228 slices of 2608
+// entries) was a chain of 228 loads, 6.4 us.  The sums are deterministic.
+template <int GRP>
+__global__ void __launch_bounds__(256)
+k_sum_slices(const float4 *__restrict__ work, float4 *out, uint32_t n4, int nz, FastDiv fN4,
+             SumEpi e) {
+  constexpr int NE = 256 / GRP;
+  __shared__ float4 sh[GRP > 1 ? 256 : 1];
+  const int lane = threadIdx.x % NE, g = threadIdx.x / NE;
+  const uint32_t q = blockIdx.x * NE + lane;
+  pdl_wait();
+  pdl_launch_dependents();
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (q < n4) {
+#pragma unroll 4
+    for (int z = g; z < nz; z += GRP) {
+      const float4 w = __ldg(work + (size_t)z * n4 + q);
+      s.x += w.x, s.y += w.y, s.z += w.z, s.w += w.w;
+    }
   }
+  if (GRP > 1) {
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    if (g > 0) return;
+    for (int k = 1; k < GRP; ++k) {
+      const float4 w = sh[k * NE + lane];
+      s.x += w.x, s.y += w.y, s.z += w.z, s.w += w.w;
+    }
+  }
+  if (q >= n4) return;
+  const uint32_t row = fN4.div(q), c = 4 * (q - row * fN4.d);
+  if (e.bias) {
+    const float *b = e.bias + c;
+    s.x += __ldg(b), s.y += __ldg(b + 1), s.z += __ldg(b + 2), s.w += __ldg(b + 3);
+  }
+  if (e.relu) {
+    s.x = s.x < 0.f ? 0.f : s.x, s.y = s.y < 0.f ? 0.f : s.y;
+    s.z = s.z < 0.f ? 0.f : s.z, s.w = s.w < 0.f ? 0.f : s.w;
+  }
+  if (e.grad.add) {
+    const float4 a = __ldg(
+        reinterpret_cast<const float4 *>(e.grad.add + (size_t)row * e.grad.addp + c));
+    s.x = a.x + s.x, s.y = a.y + s.y, s.z = a.z + s.z, s.w = a.w + s.w;
+  }
+  if (e.grad.mask) {
+    const float4 y = __ldg(reinterpret_cast<const float4 *>(e.grad.mask) + q);
+    s.x = y.x > 0.f ? s.x : 0.f, s.y = y.y > 0.f ? s.y : 0.f;
+    s.z = y.z > 0.f ? s.z : 0.f, s.w = y.w > 0.f ? s.w : 0.f;
+  }
+  if (e.acc) {
+    const float4 o = out[q];
+    s.x = o.x + s.x, s.y = o.y + s.y, s.z = o.z + s.z, s.w = o.w + s.w;
+  }
+  out[q] = s;
+}
+
+// n entries of rows of N; every pointer and row length is a multiple of 16
+// bytes (N is a multiple of 16, the network's tensors and layer offsets are)
+void sum_slices(const float *work, float *out, long long n, int nz, int N, const SumEpi &e,
+                cudaStream_t s) {
+  const uint32_t n4 = (uint32_t)(n / 4);
+  const FastDiv f((uint32_t)N / 4);
+  if (nz >= 16)
+    launch_pdl(k_sum_slices<8>, (n4 + 31) / 32, 256, s, (const float4 *)work, (float4 *)out, n4,
+               nz, f, e);
+  else
+    launch_pdl(k_sum_slices<1>, (n4 + 255) / 256, 256, s, (const float4 *)work, (float4 *)out, n4,
+               nz, f, e);
 }
 
 // BF16 copies of one layer's weights W[tap][ci][co]: WB in the same order,
@@ -517,61 +611,6 @@ __global__ void k_weights_tc(const float *__restrict__ wq, uint16_t *__restrict_
     const long long co = q / K, k = q - co * K;
     wt[(size_t)co * kpad + k] = bits(wq[(size_t)k * cout + co]);
   }
-}
-
-// Weight and bias gradient of a 1^4 convolution with CI inputs and CO
-// outputs: each thread accumulates its voxels' products, the block reduces
-// them in a fixed order into part[block][CI CO + CO].
-template <int CI, int CO>
-__global__ void __launch_bounds__(256) k_wgrad_1x1(const float *__restrict__ in,
-                                                   const float *__restrict__ dout, long long V,
-                                                   float *__restrict__ part) {
-  constexpr int NV = CI * CO + CO;
-  __shared__ float red[8][NV];
-  float acc[NV];
-#pragma unroll
-  for (int j = 0; j < NV; ++j) acc[j] = 0.f;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V;
-       v += (long long)gridDim.x * blockDim.x) {
-    float a[CI], d[CO];
-#pragma unroll
-    for (int c = 0; c < CI; ++c) a[c] = __ldg(in + v * CI + c);
-#pragma unroll
-    for (int c = 0; c < CO; ++c) d[c] = __ldg(dout + v * CO + c);
-#pragma unroll
-    for (int ci = 0; ci < CI; ++ci)
-#pragma unroll
-      for (int co = 0; co < CO; ++co) acc[ci * CO + co] += a[ci] * d[co];
-#pragma unroll
-    for (int co = 0; co < CO; ++co) acc[CI * CO + co] += d[co];
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    float x = acc[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[warp][j] = x;
-  }
-  __syncthreads();
-  for (int j = threadIdx.x; j < NV; j += blockDim.x) {
-    float x = 0.f;
-    for (int w = 0; w < 8; ++w) x += red[w][j];
-    part[(size_t)blockIdx.x * NV + j] = x;
-  }
-}
-
-// out[j] = sum over the blocks' partials: one warp per entry, lane l adds
-// blocks l, l + 32, ... in order, then a fixed butterfly (deterministic)
-__global__ void k_sum_parts(const float *__restrict__ part, int nblocks, int nv,
-                            float *__restrict__ out) {
-  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (j >= nv) return;
-  float x = 0.f;
-  for (int b = lane; b < nblocks; b += 32) x += part[(size_t)b * nv + j];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  if (lane == 0) out[j] = x;
 }
 
 struct TcPlan {
@@ -651,7 +690,7 @@ void launch_tc(const TcArgs &a0, int nz, cudaStream_t s, int gy = 1) {
   a.ncols = pow2_cols(a.N);
   tc_attr<MODE, VEC>();
   dim3 grid((a.M + TB_M - 1) / TB_M, gy, nz);
-  k_conv_tc<MODE, VEC><<<grid, TB_W, tc_smem<MODE>(a.N), s>>>(a);
+  launch_pdl_smem(k_conv_tc<MODE, VEC>, grid, TB_W, tc_smem<MODE>(a.N), s, a);
   // a refused launch (configuration) is reported here, not by a later sync
   fh::cuda_check(cudaGetLastError(), "k_conv_tc launch");
 }
@@ -676,49 +715,24 @@ TcPlan plan_fwd(long long M, long long K, int cin, int cout) {
 
 // ---- launchers --------------------------------------------------------------
 
-bool net_tc_fwd_ok(int cin, int cout, int ks) {
-  (void)cin;
-  return ks == 3 && cout % 16 == 0 && cout <= 128;
-}
-bool net_tc_bwd_data_ok(int cin, int cout, int ks) {
-  return ks == 3 && cin % 16 == 0 && cin <= 128 && cout % 8 == 0;
-}
-bool net_tc_bwd_weight_ok(int cin, int cout, int ks) {
-  (void)cin;
-  return ks == 3 && cout % 16 == 0 && cout <= 128;
-}
 int net_tc_kpad(int cin, int ks) {
   const int K = (ks == 3 ? 81 : 1) * cin;
   return (K + TB_K - 1) / TB_K * TB_K;
 }
 
-size_t net_tc_work(int rin, int rout, int cin, int cout, int ks) {
+// the first layer has no input gradient
+size_t net_tc_work(int rin, int rout, int cin, int cout, bool first) {
   size_t w = 0;
   const long long Vi = (long long)rin * rin * rin * rin, Vo = (long long)rout * rout * rout * rout;
-  if (net_tc_fwd_ok(cin, cout, ks)) {
-    const TcPlan pl = plan_fwd(Vo, net_tc_kpad(cin, ks), cin, cout);
-    if (pl.nz > 1) w = std::max(w, (size_t)pl.nz * (size_t)Vo * cout);
-  }
-  if (net_tc_bwd_data_ok(cin, cout, ks)) {
+  const TcPlan pf = plan_fwd(Vo, net_tc_kpad(cin, 3), cin, cout);
+  if (pf.nz > 1) w = std::max(w, (size_t)pf.nz * (size_t)Vo * cout);
+  if (!first) {
     const int nz = rin == rout ? tc_plan_for<1, 1>(Vi, 81LL * cout, cin).nz
                                : cls_slices(Vo, 16LL * cout);
     if (nz > 1) w = std::max(w, (size_t)nz * (size_t)Vi * cin);
   }
-  if (net_tc_bwd_weight_ok(cin, cout, ks)) {
-    const TcPlan pl = tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout);
-    w = std::max(w, (size_t)pl.nz * (81 * cin + 1) * cout);
-  }
-  return w;
-}
-
-bool net_wgrad_1x1_ok(int cin, int cout, int ks) { return ks == 1 && cin == 16 && cout == 4; }
-size_t net_wgrad_1x1_work() { return (size_t)2 * 152 * (16 * 4 + 4) * 4; }
-
-void net_wgrad_1x1(const float *in, const float *dout, float *dw, float *work, long long V,
-                   cudaStream_t s) {
-  const int nb = std::min(2 * sm_count(), 4 * 152);
-  k_wgrad_1x1<16, 4><<<nb, 256, 0, s>>>(in, dout, V, work);
-  k_sum_parts<<<(16 * 4 + 4 + 3) / 4, 128, 0, s>>>(work, nb, 16 * 4 + 4, dw);
+  const TcPlan pl = tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout);
+  return std::max(w, (size_t)pl.nz * (81 * cin + 1) * cout);
 }
 
 void net_weights_tc(const float *wq, uint16_t *wb, uint16_t *wt, int cin, int cout, int ks,
@@ -752,14 +766,15 @@ void net_tc_conv_fwd(const float *in, const uint16_t *wt, const float *b, float 
     launch_tc<0, 0>(a, pl.nz, s);
   if (pl.nz > 1) {
     const long long n = (long long)a.M * a.N;
-    k_sum_slices_epi<<<grid_for(n, 256), 256, 0, s>>>(work, out, n, pl.nz, a.N, b, relu);
+    sum_slices(work, out, n, pl.nz, a.N, SumEpi{b, relu, 0, {}}, s);
   }
 }
 
 void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, float *work,
-                          int rin, int rout, int cin, int cout, int stride, int *err,
-                          cudaStream_t s) {
+                          int rin, int rout, int cin, int cout, int stride, NetGradEpi epi,
+                          int *err, cudaStream_t s) {
   TcArgs a{};
+  a.epi = epi;
   a.A = dout;
   a.Bw = wb;
   a.err = err;
@@ -777,7 +792,7 @@ void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, flo
     launch_tc<1, 1>(a, nz, s, 16);
     if (nz > 1) {
       const long long n = (long long)rin * rin * rin * rin * cin;
-      k_sum_slices_epi<<<grid_for(n, 256), 256, 0, s>>>(work, din, n, nz, cin, nullptr, 0);
+      sum_slices(work, din, n, nz, cin, SumEpi{nullptr, 0, 0, epi}, s);
     }
     return;
   }
@@ -790,12 +805,13 @@ void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, flo
   launch_tc<1, 1>(a, pl.nz, s);
   if (pl.nz > 1) {
     const long long n = (long long)a.M * a.N;
-    k_sum_slices_epi<<<grid_for(n, 256), 256, 0, s>>>(work, din, n, pl.nz, a.N, nullptr, 0);
+    sum_slices(work, din, n, pl.nz, a.N, SumEpi{nullptr, 0, 0, epi}, s);
   }
 }
 
-void net_tc_conv_bwd_weight(const float *in, const float *dout, float *dw, float *work, int rin,
-                            int rout, int cin, int cout, int stride, int *err, cudaStream_t s) {
+void net_tc_conv_bwd_weight(const float *in, const float *dout, float *grad, float *work, int rin,
+                            int rout, int cin, int cout, int stride, int acc, int *err,
+                            cudaStream_t s) {
   TcArgs a{};
   a.A = in;
   a.B32 = dout;
@@ -811,7 +827,7 @@ void net_tc_conv_bwd_weight(const float *in, const float *dout, float *dw, float
   a.C = work;
   launch_tc<2, 0>(a, pl.nz, s);
   const long long n = (long long)a.M * a.N;
-  k_sum_slices_epi<<<grid_for(n, 256), 256, 0, s>>>(work, dw, n, pl.nz, a.N, nullptr, 0);
+  sum_slices(work, grad, n, pl.nz, a.N, SumEpi{nullptr, 0, acc, {}}, s);
 }
 
 }  // namespace flof

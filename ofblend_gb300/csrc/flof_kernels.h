@@ -450,59 +450,58 @@ void launch_rescale_slices(float *phi, Dims4 d, const float *w, cudaStream_t s);
 void launch_add_inner3(float *a, int X, int Y, int Z, float v, cudaStream_t s);
 
 // ---- learned warm start network (flof_net.cu) -----------------------------------
-// Channels-last tensors over cubic 4D grids; 3^4 (pad 1) or 1^4 convolutions.
-void net_conv_fwd(const float *in, const float *w, const float *b, float *out, int rin, int rout,
-                  int cin, int cout, int ks, int stride, int relu, cudaStream_t s);
-void net_conv_bwd_data(const float *dout, const float *w, float *din, int rin, int rout,
-                       int cin, int cout, int ks, int stride, cudaStream_t s);
-// dw = weight gradient; work holds net_conv_bwd_weight_work(...) floats
-size_t net_conv_bwd_weight_work(int rout, int cin, int cout, int ks);
-void net_conv_bwd_weight(const float *in, const float *dout, float *dw, float *work, int rin,
-                         int rout, int cin, int cout, int ks, int stride, cudaStream_t s);
-void net_relu_bwd(float *dy, const float *y, long long n, cudaStream_t s);
+// Channels-last tensors over cubic 4D grids.
+// The output layer: a 1^4 convolution of NET_HEAD_IN channels to the four
+// velocity components, weights w[ci][co] followed by the bias.
+constexpr int NET_HEAD_IN = 16, NET_HEAD_OUT = 4;
+void net_head_fwd(const float *in, const float *wb, float *out, long long V, cudaStream_t s);
+// Mean squared error of the output layer against `target`, its gradient with
+// respect to the layer's input masked by the input's ReLU (din) and to its
+// weights and bias (grad).  acc: grad and loss are added to, else written;
+// part holds net_head_work(V) doubles.
+size_t net_head_work(long long V);
+void net_head_grad(const float *in, const float *wb, const float *target, float *din, float *grad,
+                   double *loss, double *part, long long V, int acc, cudaStream_t s);
 void net_upcat(const float *lo, const float *skip, float *out, int R, int c1, int c2,
                cudaStream_t s);
-void net_upcat_bwd(const float *dout, float *dlo, float *dskip, int R, int c1, int c2,
+// gradient of net_upcat with respect to lo, masked by lo's ReLU
+void net_upcat_bwd(const float *dout, const float *lo, float *dlo, int R, int c1, int c2,
                    cudaStream_t s);
-void net_bias_grad(const float *d, float *db, long long V, int C, cudaStream_t s);
-void net_mse(const float *pred, const float *target, float *dpred, long long n, double *partial,
-             unsigned *counter, double *loss, cudaStream_t s);
 void net_adam(float *w, float *wq, const float *g, float *m, float *v, long long n, float lr,
               int step, float gscale, cudaStream_t s);
 void net_round_bf16(const float *w, float *wq, long long n, cudaStream_t s);
 void net_input(const float *i0, const float *i1, float *x, long long V, float scale,
                cudaStream_t s);
-void net_add_into(float *a, const float *b, long long n, cudaStream_t s);
 
-// Tensor-core (tcgen05) versions of the 3^4 convolutions (flof_conv_tc.cu).
-// The *_ok predicates name the shapes they take; the weights enter as BF16
-// copies made by net_weights_tc: WB[tap][ci][co] (input gradient) and
+// Tensor-core (tcgen05) 3^4 convolutions, padding 1, stride 1 or 2
+// (flof_conv_tc.cu).  Output channel counts are multiples of 16 up to 128
+// (input channel counts too, for the input gradient); the weights enter as
+// BF16 copies made by net_weights_tc: WB[tap][ci][co] (input gradient) and
 // WT[co][kpad] (forward, rows of net_tc_kpad entries, zero tail).  `work`
 // holds net_tc_work(...) floats; a block whose bounded wait runs out stores
 // FLOF_DEV_ERR_TC_TIMEOUT in *err.
-bool net_tc_fwd_ok(int cin, int cout, int ks);
-bool net_tc_bwd_data_ok(int cin, int cout, int ks);
-bool net_tc_bwd_weight_ok(int cin, int cout, int ks);
 int net_tc_kpad(int cin, int ks);
-size_t net_tc_work(int rin, int rout, int cin, int cout, int ks);
+size_t net_tc_work(int rin, int rout, int cin, int cout, bool first);
 void net_weights_tc(const float *wq, uint16_t *wb, uint16_t *wt, int cin, int cout, int ks,
                     cudaStream_t s);
 void net_tc_conv_fwd(const float *in, const uint16_t *wt, const float *b, float *out,
                      float *work, int rin, int rout, int cin, int cout, int stride, int relu,
                      int *err, cudaStream_t s);
+// What happens to an input gradient as it is stored: `add` (nullable; rows of
+// `addp` floats) is added first, then entries whose `mask` (nullable; the
+// input itself, behind a ReLU) is not positive become zero.
+struct NetGradEpi {
+  const float *add = nullptr;
+  int addp = 0;
+  const float *mask = nullptr;
+};
 void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, float *work,
-                          int rin, int rout, int cin, int cout, int stride, int *err,
-                          cudaStream_t s);
-// Weight and bias gradient of the 1^4 output layer (16 -> 4 channels) over
-// V voxels: dw receives the 64 weight entries then the 4 bias entries; work
-// holds net_wgrad_1x1_work() floats.
-bool net_wgrad_1x1_ok(int cin, int cout, int ks);
-size_t net_wgrad_1x1_work();
-void net_wgrad_1x1(const float *in, const float *dout, float *dw, float *work, long long V,
-                   cudaStream_t s);
-// dw receives 81 cin cout weight-gradient entries followed by the cout bias
-// gradients
-void net_tc_conv_bwd_weight(const float *in, const float *dout, float *dw, float *work, int rin,
-                            int rout, int cin, int cout, int stride, int *err, cudaStream_t s);
+                          int rin, int rout, int cin, int cout, int stride, NetGradEpi epi,
+                          int *err, cudaStream_t s);
+// grad: 81 cin cout weight-gradient entries followed by the cout bias
+// gradients, written, or added to (acc)
+void net_tc_conv_bwd_weight(const float *in, const float *dout, float *grad, float *work, int rin,
+                            int rout, int cin, int cout, int stride, int acc, int *err,
+                            cudaStream_t s);
 
 }  // namespace flof

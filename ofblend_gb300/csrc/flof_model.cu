@@ -44,7 +44,6 @@ struct flof_model {
   long long nparams = 0;
   long long woff[8], boff[8], wsize[8];
   float *w = nullptr, *wq = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
-  float *scratch = nullptr;  // one layer's weight gradient
   float *work = nullptr;     // split-reduction slices of a convolution
   // BF16 weight copies of the tensor-core convolutions: WB (the weights'
   // own order) at woff, WT (transposed, rows of kpad) at wtoff
@@ -52,11 +51,10 @@ struct flof_model {
   long long wtoff[8];
   int step = 0;
   // activations and their gradients
-  float *x = nullptr, *a[7] = {}, *c5 = nullptr, *c6 = nullptr, *out = nullptr;
-  float *da[7] = {}, *dc5 = nullptr, *dc6 = nullptr, *dout = nullptr, *tmp = nullptr;
+  float *x = nullptr, *a[7] = {}, *c5 = nullptr, *c6 = nullptr;
+  float *da[7] = {}, *dc5 = nullptr, *dc6 = nullptr;
   double *dloss = nullptr;  // device loss accumulator
-  double *part = nullptr;
-  unsigned *cnt = nullptr;
+  double *part = nullptr;   // partials of the output layer's sums
   double *hloss = nullptr;  // pinned
   std::vector<void *> allocs;
 
@@ -86,18 +84,15 @@ void refresh_tc_weights(flof_model *m) {
   }
 }
 
-void forward(flof_model *m, const float *i0, const float *i1, float *out) {
+// the activations up to the output layer's input (a[6])
+void forward(flof_model *m, const float *i0, const float *i1) {
   const int R = m->R;
   cudaStream_t s = S(m);
   net_input(i0, i1, m->x, m->V(1), INPUT_SCALE, s);
   auto conv = [&](int l, const float *in, float *o) {
     const LayerDef &L = LAYERS[l];
-    if (net_tc_fwd_ok(L.cin, L.cout, L.ks))
-      net_tc_conv_fwd(in, m->wt + m->wtoff[l], m->wq + m->boff[l], o, m->work, R / L.rin_div,
-                      R / L.rout_div, L.cin, L.cout, L.stride, L.relu, E(m), s);
-    else
-      net_conv_fwd(in, m->wq + m->woff[l], m->wq + m->boff[l], o, R / L.rin_div,
-                   R / L.rout_div, L.cin, L.cout, L.ks, L.stride, L.relu, s);
+    net_tc_conv_fwd(in, m->wt + m->wtoff[l], m->wq + m->boff[l], o, m->work, R / L.rin_div,
+                    R / L.rout_div, L.cin, L.cout, L.stride, L.relu, E(m), s);
   };
   conv(0, m->x, m->a[0]);
   conv(1, m->a[0], m->a[1]);
@@ -108,66 +103,56 @@ void forward(flof_model *m, const float *i0, const float *i1, float *out) {
   conv(5, m->c5, m->a[5]);
   net_upcat(m->a[5], m->a[0], m->c6, R, 32, 16, s);
   conv(6, m->c6, m->a[6]);
-  conv(7, m->a[6], out);
 }
 
-// gradient of layer l's weights and bias into the accumulators, and (when din
-// is given) of its input
-void layer_bwd(flof_model *m, int l, const float *in, const float *dy, float *din) {
+void predict(flof_model *m, const float *i0, const float *i1, float *out) {
+  forward(m, i0, i1);
+  net_head_fwd(m->a[6], m->wq + m->woff[7], out, m->V(1), S(m));
+}
+
+// Gradient of layer l's weights and bias (the bias follows the weights in
+// grad), and (when din is given) of its input, stored through `epi`.
+void layer_bwd(flof_model *m, int l, const float *in, const float *dy, int acc, float *din,
+               const NetGradEpi &epi) {
   const LayerDef &L = LAYERS[l];
-  const int R = m->R;
-  cudaStream_t s = S(m);
-  const int rin = R / L.rin_div, rout = R / L.rout_div;
-  if (net_wgrad_1x1_ok(L.cin, L.cout, L.ks)) {
-    net_wgrad_1x1(in, dy, m->scratch, m->work, (long long)rout * rout * rout * rout, s);
-    net_add_into(m->grad + m->woff[l], m->scratch, m->wsize[l] + L.cout, s);
-  } else if (net_tc_bwd_weight_ok(L.cin, L.cout, L.ks)) {
-    // weights and bias in one pass; the bias follows the weights in grad
-    net_tc_conv_bwd_weight(in, dy, m->scratch, m->work, rin, rout, L.cin, L.cout, L.stride,
-                           E(m), s);
-    net_add_into(m->grad + m->woff[l], m->scratch, m->wsize[l] + L.cout, s);
-  } else {
-    net_conv_bwd_weight(in, dy, m->scratch, m->work, rin, rout, L.cin, L.cout, L.ks, L.stride,
-                        s);
-    net_add_into(m->grad + m->woff[l], m->scratch, m->wsize[l], s);
-    net_bias_grad(dy, m->scratch, (long long)rout * rout * rout * rout, L.cout, s);
-    net_add_into(m->grad + m->boff[l], m->scratch, L.cout, s);
-  }
-  if (!din) return;
-  if (net_tc_bwd_data_ok(L.cin, L.cout, L.ks))
-    net_tc_conv_bwd_data(dy, m->wb + m->woff[l], din, m->work, rin, rout, L.cin, L.cout,
-                         L.stride, E(m), s);
-  else
-    net_conv_bwd_data(dy, m->wq + m->woff[l], din, rin, rout, L.cin, L.cout, L.ks, L.stride, s);
+  const int rin = m->R / L.rin_div, rout = m->R / L.rout_div;
+  net_tc_conv_bwd_weight(in, dy, m->grad + m->woff[l], m->work, rin, rout, L.cin, L.cout,
+                         L.stride, acc, E(m), S(m));
+  if (din)
+    net_tc_conv_bwd_data(dy, m->wb + m->woff[l], din, m->work, rin, rout, L.cin, L.cout, L.stride,
+                         epi, E(m), S(m));
 }
 
-// loss of one sample, gradients added to m->grad
-void backward(flof_model *m, const float *target) {
+// Loss of one sample and its gradients: written, or (acc) added to dloss and
+// grad.  The gradient of a concatenated tensor's skip half is read where the
+// layer below it stores its own gradient of that tensor, and each ReLU's
+// backward pass is the mask of the kernel that stores the gradient.
+void backward(flof_model *m, const float *target, int acc) {
   const int R = m->R;
   cudaStream_t s = S(m);
-  const long long n = m->V(1) * 4;
-  net_mse(m->out, target, m->dout, n, m->part, m->cnt, m->dloss, s);
-  layer_bwd(m, 7, m->a[6], m->dout, m->da[6]);
-  net_relu_bwd(m->da[6], m->a[6], m->V(1) * 16, s);
-  layer_bwd(m, 6, m->c6, m->da[6], m->dc6);
-  CK(cudaMemsetAsync(m->da[0], 0, m->V(1) * 16 * sizeof(float), s));
-  net_upcat_bwd(m->dc6, m->da[5], m->da[0], R, 32, 16, s);
-  net_relu_bwd(m->da[5], m->a[5], m->V(2) * 32, s);
-  layer_bwd(m, 5, m->c5, m->da[5], m->dc5);
-  CK(cudaMemsetAsync(m->da[2], 0, m->V(2) * 32 * sizeof(float), s));
-  net_upcat_bwd(m->dc5, m->da[4], m->da[2], R / 2, 64, 32, s);
-  net_relu_bwd(m->da[4], m->a[4], m->V(4) * 64, s);
-  layer_bwd(m, 4, m->a[3], m->da[4], m->da[3]);
-  net_relu_bwd(m->da[3], m->a[3], m->V(4) * 64, s);
-  layer_bwd(m, 3, m->a[2], m->da[3], m->tmp);
-  net_add_into(m->da[2], m->tmp, m->V(2) * 32, s);
-  net_relu_bwd(m->da[2], m->a[2], m->V(2) * 32, s);
-  layer_bwd(m, 2, m->a[1], m->da[2], m->da[1]);
-  net_relu_bwd(m->da[1], m->a[1], m->V(2) * 32, s);
-  layer_bwd(m, 1, m->a[0], m->da[1], m->tmp);
-  net_add_into(m->da[0], m->tmp, m->V(1) * 16, s);
-  net_relu_bwd(m->da[0], m->a[0], m->V(1) * 16, s);
-  layer_bwd(m, 0, m->x, m->da[0], nullptr);
+  auto masked = [](const float *y) {
+    NetGradEpi e;
+    e.mask = y;
+    return e;
+  };
+  auto skipped = [](const float *d, int pitch, const float *y) {
+    NetGradEpi e;
+    e.add = d;
+    e.addp = pitch;
+    e.mask = y;
+    return e;
+  };
+  net_head_grad(m->a[6], m->wq + m->woff[7], target, m->da[6], m->grad + m->woff[7], m->dloss,
+                m->part, m->V(1), acc, s);
+  layer_bwd(m, 6, m->c6, m->da[6], acc, m->dc6, {});
+  net_upcat_bwd(m->dc6, m->a[5], m->da[5], R, 32, 16, s);
+  layer_bwd(m, 5, m->c5, m->da[5], acc, m->dc5, {});
+  net_upcat_bwd(m->dc5, m->a[4], m->da[4], R / 2, 64, 32, s);
+  layer_bwd(m, 4, m->a[3], m->da[4], acc, m->da[3], masked(m->a[3]));
+  layer_bwd(m, 3, m->a[2], m->da[3], acc, m->da[2], skipped(m->dc5 + 64, 96, m->a[2]));
+  layer_bwd(m, 2, m->a[1], m->da[2], acc, m->da[1], masked(m->a[1]));
+  layer_bwd(m, 1, m->a[0], m->da[1], acc, m->da[0], skipped(m->dc6 + 32, 48, m->a[0]));
+  layer_bwd(m, 0, m->x, m->da[0], acc, nullptr, {});
 }
 
 void need_model_grid(flof_model *m, const flof_grid *g, int elem, const char *name) {
@@ -182,7 +167,7 @@ void need_model_grid(flof_model *m, const flof_grid *g, int elem, const char *na
 namespace fh {
 // The warm start's prediction for the coarsest level (used by the driver).
 void model_predict_raw(flof_model *m, const float *i0, const float *i1, float4 *vel) {
-  forward(m, i0, i1, (float *)vel);
+  predict(m, i0, i1, (float *)vel);
   CK(cudaGetLastError());
 }
 int model_res(const flof_model *m) { return m->R; }
@@ -206,7 +191,7 @@ FLOF_API int flof_model_create(flof_ctx *c, int res, flof_model **out) {
     m = new flof_model();
     m->ctx = c;
     m->R = res;
-    long long off = 0, maxw = 0;
+    long long off = 0;
     for (int l = 0; l < 8; ++l) {
       const LayerDef &L = LAYERS[l];
       const long long taps = L.ks == 3 ? 81 : 1;
@@ -215,7 +200,6 @@ FLOF_API int flof_model_create(flof_ctx *c, int res, flof_model **out) {
       off += m->wsize[l];
       m->boff[l] = off;
       off += L.cout;
-      maxw = m->wsize[l] > maxw ? m->wsize[l] : maxw;
     }
     m->nparams = off;
     m->w = m->alloc(off);
@@ -223,14 +207,13 @@ FLOF_API int flof_model_create(flof_ctx *c, int res, flof_model **out) {
     m->grad = m->alloc(off);
     m->m = m->alloc(off);
     m->v = m->alloc(off);
-    m->scratch = m->alloc(maxw + 128);  // a weight gradient and its bias gradient
     size_t maxwork = 0;
     long long wtsize = 0;
     for (int l = 0; l < 8; ++l) {
       const LayerDef &L = LAYERS[l];
-      const size_t wk = net_conv_bwd_weight_work(res / L.rout_div, L.cin, L.cout, L.ks);
-      const size_t wt = net_tc_work(res / L.rin_div, res / L.rout_div, L.cin, L.cout, L.ks);
-      maxwork = std::max(maxwork, std::max(std::max(wk, wt), net_wgrad_1x1_work()));
+      if (L.ks == 3)
+        maxwork = std::max(maxwork, net_tc_work(res / L.rin_div, res / L.rout_div, L.cin, L.cout,
+                                                l == 0));
       m->wtoff[l] = wtsize;
       wtsize += (long long)L.cout * net_tc_kpad(L.cin, L.ks);
     }
@@ -249,13 +232,8 @@ FLOF_API int flof_model_create(flof_ctx *c, int res, flof_model **out) {
     m->dc5 = m->alloc(V2 * 96);
     m->c6 = m->alloc(V1 * 48);
     m->dc6 = m->alloc(V1 * 48);
-    m->out = m->alloc(V1 * 4);
-    m->dout = m->alloc(V1 * 4);
-    m->tmp = m->alloc(V1 * 16);
     m->dloss = (double *)m->alloc(2);
-    m->part = (double *)m->alloc(2 * 4096);
-    m->cnt = (unsigned *)m->alloc(1);
-    CK(cudaMemsetAsync(m->cnt, 0, sizeof(unsigned), c->stream));
+    m->part = (double *)m->alloc(2 * net_head_work(V1));
     CK(cudaMallocHost(&m->hloss, sizeof(double)));
     CK(cudaMemsetAsync(m->m, 0, off * sizeof(float), c->stream));
     CK(cudaMemsetAsync(m->v, 0, off * sizeof(float), c->stream));
@@ -351,7 +329,7 @@ FLOF_API int flof_model_predict(flof_model *m, const flof_grid *i0, const flof_g
     need_model_grid(m, i1, FLOF_REAL, "i1");
     need_model_grid(m, vel, FLOF_VEC4, "vel");
     set_ctx_device(m->ctx);
-    forward(m, i0->f(), i1->f(), vel->f());
+    predict(m, i0->f(), i1->f(), vel->f());
     CK(cudaGetLastError());  // a refused launch of any network kernel
     CK(cudaStreamSynchronize(S(m)));
     check_device_errors(m->ctx);
@@ -369,10 +347,8 @@ FLOF_API int flof_model_loss_grad(flof_model *m, const flof_grid *i0, const flof
     need_model_grid(m, i1, FLOF_REAL, "i1");
     need_model_grid(m, target, FLOF_VEC4, "target");
     set_ctx_device(m->ctx);
-    CK(cudaMemsetAsync(m->grad, 0, m->nparams * sizeof(float), S(m)));
-    CK(cudaMemsetAsync(m->dloss, 0, sizeof(double), S(m)));
-    forward(m, i0->f(), i1->f(), m->out);
-    backward(m, target->f());
+    forward(m, i0->f(), i1->f());
+    backward(m, target->f(), 0);
     CK(cudaMemcpyAsync(m->hloss, m->dloss, sizeof(double), cudaMemcpyDeviceToHost, S(m)));
     if (grad_host)
       CK(cudaMemcpyAsync(grad_host, m->grad, m->nparams * sizeof(float), cudaMemcpyDeviceToHost,
@@ -399,11 +375,9 @@ FLOF_API int flof_model_train_step(flof_model *m, int n, const flof_grid *const 
     }
     need(lr > 0.f, "learning rate must be positive");
     set_ctx_device(m->ctx);
-    CK(cudaMemsetAsync(m->grad, 0, m->nparams * sizeof(float), S(m)));
-    CK(cudaMemsetAsync(m->dloss, 0, sizeof(double), S(m)));
     for (int q = 0; q < n; ++q) {
-      forward(m, i0s[q]->f(), i1s[q]->f(), m->out);
-      backward(m, targets[q]->f());
+      forward(m, i0s[q]->f(), i1s[q]->f());
+      backward(m, targets[q]->f(), q > 0);
     }
     m->step++;
     net_adam(m->w, m->wq, m->grad, m->m, m->v, m->nparams, lr, m->step, 1.f / n, S(m));
