@@ -167,6 +167,40 @@ __device__ __forceinline__ void gather2(float (&xw)[KG_T][8], const int2 *vt, in
     }
 }
 
+// What 16 columns from c0 of an output row become as they are stored:
+// forward: bias and ReLU; input gradient: NetGradEpi
+template <int MODE>
+__device__ __forceinline__ void epilogue16(float (&v)[16], const float *bias, int relu,
+                                           const NetGradEpi &epi, size_t row, int N, int c0) {
+  if (MODE == 0) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float y = v[j] + (bias ? __ldg(bias + c0 + j) : 0.f);
+      v[j] = relu && y < 0.f ? 0.f : y;
+    }
+    return;
+  }
+  const float4 *add =
+      reinterpret_cast<const float4 *>(epi.add ? epi.add + row * epi.addp + c0 : nullptr);
+  const float4 *mask =
+      reinterpret_cast<const float4 *>(epi.mask ? epi.mask + row * N + c0 : nullptr);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (add) {
+      const float4 w = __ldg(add + q);
+      v[4 * q] = w.x + v[4 * q], v[4 * q + 1] = w.y + v[4 * q + 1];
+      v[4 * q + 2] = w.z + v[4 * q + 2], v[4 * q + 3] = w.w + v[4 * q + 3];
+    }
+    if (mask) {
+      const float4 w = __ldg(mask + q);
+      v[4 * q] = w.x > 0.f ? v[4 * q] : 0.f;
+      v[4 * q + 1] = w.y > 0.f ? v[4 * q + 1] : 0.f;
+      v[4 * q + 2] = w.z > 0.f ? v[4 * q + 2] : 0.f;
+      v[4 * q + 3] = w.w > 0.f ? v[4 * q + 3] : 0.f;
+    }
+  }
+}
+
 template <int MODE, int VEC>
 __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
   extern __shared__ unsigned char smem_raw[];
@@ -470,34 +504,7 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
         for (int j = 0; j < 16; ++j) v[j] = 0.f;
       }
       if (r < p.M) {
-        if (!split && MODE == 0) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float y = v[j] + (p.bias ? __ldg(p.bias + c0 + j) : 0.f);
-            v[j] = p.relu && y < 0.f ? 0.f : y;
-          }
-        }
-        if (!split && MODE == 1) {
-          const float4 *add = reinterpret_cast<const float4 *>(
-              p.epi.add ? p.epi.add + orow * p.epi.addp + c0 : nullptr);
-          const float4 *mask =
-              reinterpret_cast<const float4 *>(p.epi.mask ? p.epi.mask + orow * N + c0 : nullptr);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (add) {
-              const float4 w = __ldg(add + q);
-              v[4 * q] = w.x + v[4 * q], v[4 * q + 1] = w.y + v[4 * q + 1];
-              v[4 * q + 2] = w.z + v[4 * q + 2], v[4 * q + 3] = w.w + v[4 * q + 3];
-            }
-            if (mask) {
-              const float4 w = __ldg(mask + q);
-              v[4 * q] = w.x > 0.f ? v[4 * q] : 0.f;
-              v[4 * q + 1] = w.y > 0.f ? v[4 * q + 1] : 0.f;
-              v[4 * q + 2] = w.z > 0.f ? v[4 * q + 2] : 0.f;
-              v[4 * q + 3] = w.w > 0.f ? v[4 * q + 3] : 0.f;
-            }
-          }
-        }
+        if (!split && MODE < 2) epilogue16<MODE>(v, p.bias, p.relu, p.epi, orow, N, c0);
         float4 *dst = reinterpret_cast<float4 *>(C + orow * N + c0);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -513,6 +520,229 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
   }
 }
 
+// ---- stride-1 input gradient from a halo tile ------------------------------------
+//
+// out[v][n] = sum over taps and channels of A[v + 1 - tap][c] W[tap][n][c], 128
+// output voxels per block: 8 along x times 16 rows.  Rows are counted through
+// the plane padded by one voxel on each side, rho = z (R + 2) + y, so that
+// the input row of tap (dy, dz) is row rho + dy + (R + 2) dz for every
+// output row; the two rows between planes give results that are not stored.
+// A chunk of the reduction is one t offset times 16 channels: the block loads
+// the 16 + 2 + 2 (R + 2) rows of 10 voxels that its 27 (x, y, z) taps read,
+// once, as BF16 parts hi and lo, in 16-byte units of 8 channels:
+//   [part][channel group][row][10 voxels][16 bytes]
+// Eight voxels along x of one channel group are then one core matrix of the
+// unswizzled K-major operand wherever they start, so each tap is the same
+// tile read from another start address: row groups 160 bytes apart, channel
+// groups (rows x 160) bytes apart.  The im2col form of this file loads and
+// converts every tap of every voxel anew: 81 values per input value instead
+// of 3 (R + 2 + 9) 10 / 64 (13 at R = 16).  At the 16^4 network's layers
+// (channels in the gradient -> columns): 16 -> 48 at 16^4 70 us (im2col 97),
+// 32 -> 96 at 8^4 17 (36), 32 -> 32 at 8^4 11 (14), 64 -> 64 at 4^4 8 (15).
+// Bound by the products' 128 x 16 operand reads and, at 4^4 and 8^4, by the
+// latency of a chunk.
+// The tensor core drops bits at each accumulation, so the products go to
+// several accumulators that the stores add up in FP32: the lo parts to one,
+// the hi parts of successive taps in turn to three (one where N > 64).  The
+// forward pass keeps the im2col form: a change in the last bits of its
+// activations moves some across zero, and with them the gradient.
+struct HaloArgs {
+  const float *A;          // output gradient, C channels
+  const uint16_t *Bw;      // WB[tap][n][C]
+  float *out;              // result rows x N, or slices of it
+  int *err;
+  int R, C, N, ncg;        // extent, channels, columns, groups of 16 channels
+  int nx, nr;              // tiles along x, and of rows per plane
+  int cslice;              // chunks per slice
+  int pitch, nacc;         // accumulators: columns apart, number
+  NetGradEpi epi;          // unsplit only
+};
+
+constexpr int HX = 10;     // voxels of a loaded row
+constexpr int HTAPS = 27;  // taps of a chunk
+
+__host__ __device__ constexpr int halo_rows(int R) { return 16 + 2 + 2 * (R + 2); }
+__host__ __device__ constexpr int halo_stage(int R, int N) {
+  return (halo_rows(R) * HX * 64 + HTAPS * 32 * N + 127) / 128 * 128;
+}
+__host__ __device__ constexpr int halo_table(int R) {
+  return (halo_rows(R) * HX * 4 + 127) / 128 * 128;
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void load_ch8(float (&x)[8], const float *__restrict__ src) {
+  const float4 a = __ldg(reinterpret_cast<const float4 *>(src));
+  const float4 b = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+  x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+  x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+}
+
+__global__ void __launch_bounds__(TB_W, 2) k_dgrad_halo(HaloArgs p) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t bars[2];
+  __shared__ uint32_t tbase;
+  unsigned char *smem = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int R = p.R, N = p.N, RP = R + 2;
+  const int nv = halo_rows(R) * HX;  // voxels of a loaded slab
+  int *voff = reinterpret_cast<int *>(smem);  // their offsets in a t plane, -1 outside
+  unsigned char *stages = smem + halo_table(R);
+  const int stage_bytes = halo_stage(R, N);
+
+  const int tile = blockIdx.x;
+  const int x0 = tile % p.nx * 8, rho0 = tile / p.nx % p.nr * 16, t = tile / (p.nx * p.nr);
+  const int cbeg = blockIdx.z * p.cslice, cend = min(3 * p.ncg, cbeg + p.cslice);
+
+  if (warp == 0) tmem_alloc(&tbase, (uint32_t)(p.pitch * p.nacc));
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+  }
+  for (int v = tid; v < nv; v += TB_W) {
+    const int row = v / HX, rho = rho0 + row;
+    const int x = x0 + (v - row * HX) - 1, z = rho / RP - 1, y = rho % RP - 1;
+    const bool in = x >= 0 && x < R && y >= 0 && y < R && z >= 0 && z < R;
+    voff[v] = in ? x + R * (y + R * z) : -1;
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  // everything above comes from the arguments alone; the next grid is let in
+  // when every block of this one holds its tensor memory
+  pdl_wait();
+  fence_before_sync();
+  __syncthreads();
+  pdl_launch_dependents();
+  fence_after_sync();
+  const uint32_t tacc = tbase;
+  const uint32_t idesc = idesc_bf16_f32(TB_M, N);
+  const bool producer = tid < TB_T;
+
+  int issued = 0;  // chunks whose MMAs were issued (block-uniform)
+  bool bad = false;
+  for (int c = cbeg; c < cend; ++c) {
+    const int dt = c / p.ncg, cg = c - dt * p.ncg, ti = t + dt - 1;
+    if (ti < 0 || ti >= R) continue;  // the whole chunk falls off the grid
+    const int s = issued & 1;
+    unsigned char *Ahi = stages + s * stage_bytes, *Alo = Ahi + nv * 32, *Bs = Alo + nv * 32;
+    if (producer && issued >= 2 && !mbar_wait_bounded(&bars[s], ((issued - 2) >> 1) & 1))
+      bad = true;
+    if (producer && !bad) {
+      // ---- weights: 27 taps x 2 channel groups x N rows of 16 bytes
+      for (int r = warp; r < HTAPS * 2; r += TB_T / 32) {
+        const int tap = (r >> 1) + HTAPS * dt, c0 = cg * 16 + (r & 1) * 8;
+        for (int n = lane; n < N; n += 32) {
+          unsigned char *dst = Bs + (r * N + n) * 16;
+          const uint16_t *src = p.Bw + ((size_t)(80 - tap) * N + n) * p.C + c0;
+          cp_async16(dst, src);
+        }
+      }
+      // ---- input slab: 2 channel groups x nv voxels, three at a time
+      const float *base = p.A + (size_t)ti * R * R * R * p.C;
+      constexpr int U = 3;
+      for (int e0 = tid; e0 < 2 * nv; e0 += U * TB_T) {
+        float x[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int e = e0 + u * TB_T;
+          const int kg = e >= nv, v = e - kg * nv;
+          const int off = e < 2 * nv ? voff[v] : -1;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[u][j] = 0.f;
+          if (off >= 0) load_ch8(x[u], base + (size_t)off * p.C + cg * 16 + kg * 8);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int e = e0 + u * TB_T;
+          if (e < 2 * nv) {
+            uint4 h, l;
+            split8(x[u], h, l);
+            *reinterpret_cast<uint4 *>(Ahi + e * 16) = h;
+            *reinterpret_cast<uint4 *>(Alo + e * 16) = l;
+          }
+        }
+      }
+      cp_async_wait();
+      fence_proxy_async_smem();
+    }
+    if (__syncthreads_or(bad)) break;
+    if (tid == TB_T) {
+      fence_after_sync();
+      const uint32_t a_hi = smem_addr(Ahi), a_lo = smem_addr(Alo), b0 = smem_addr(Bs);
+      const uint32_t lbo = (uint32_t)nv * 16;
+      const int nhi = p.nacc - 1;
+#pragma unroll 1
+      for (int tap = 0, a = 0; tap < HTAPS; ++tap, a = a + 1 < nhi ? a + 1 : 0) {
+        const int dz = tap / 9, dy = tap / 3 - dz * 3, dx = tap % 3;
+        const uint32_t off = (uint32_t)(dx + HX * (dy + RP * dz)) * 16;
+        const uint64_t db = smem_desc(b0 + tap * N * 32, (uint32_t)N * 16, 128);
+        mma_bf16(tacc + (a + 1) * p.pitch, smem_desc(a_hi + off, lbo, HX * 16), db, idesc,
+                 issued > 0 || tap >= nhi);
+        mma_bf16(tacc, smem_desc(a_lo + off, lbo, HX * 16), db, idesc, (issued | tap) != 0);
+      }
+      mma_commit(&bars[s]);
+    }
+    ++issued;
+  }
+
+  // wait for the last issued chunk (its commit covers every earlier MMA)
+  bool ok = !bad;
+  if (issued > 0) {
+    const int last = issued - 1;
+    if (!mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) ok = false;
+  }
+  if (!ok) atomicExch(p.err, FLOF_DEV_ERR_TC_TIMEOUT);
+  ok = __syncthreads_and(ok);
+  // a slice whose chunks all fall off the grid contributes zeros
+  const bool empty = ok && issued == 0;
+  ok = ok && issued > 0;
+  fence_after_sync();
+  if ((ok || empty) && producer) {
+    const int q4 = warp & 3;
+    const int r = 32 * q4 + lane;
+    const int x = x0 + (r & 7), rho = rho0 + (r >> 3), z = rho / RP, y = rho - z * RP;
+    const bool in = x < R && y < R && z < R;
+    const size_t vol = (size_t)R * R * R;
+    const bool split = gridDim.z > 1;
+    const size_t orow = (size_t)t * vol + (in ? x + R * (y + R * z) : 0);
+    float *out = p.out + (split ? (size_t)blockIdx.z * vol * R * N : 0);
+    for (int c0 = 16 * (warp >> 2); c0 < N; c0 += 32) {
+      float v[16];
+      if (ok) {
+        const uint32_t ta = tacc + ((uint32_t)(32 * q4) << 16) + (uint32_t)c0;
+        tmem_ld16(ta + p.pitch, v);
+        for (int k = 2; k <= p.nacc; ++k) {  // the others, the lo products last
+          float w[16];
+          tmem_ld16(ta + (k < p.nacc ? k : 0) * p.pitch, w);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += w[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+      }
+      if (in) {
+        if (!split) epilogue16<1>(v, nullptr, 0, p.epi, orow, N, c0);
+        float4 *dst = reinterpret_cast<float4 *>(out + orow * N + c0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      }
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tacc, (uint32_t)(p.pitch * p.nacc));
+  }
+}
+
 // What a sum of slices becomes as it is stored: forward: bias and ReLU; input
 // gradient: NetGradEpi; weight gradient: added to what is there (acc).
 struct SumEpi {
@@ -525,7 +755,8 @@ struct SumEpi {
 // threads (of different warps) share an entry's slices, thread g adding g, g +
 // GRP, ... in order, and thread 0 adds the GRP sums in order: with one thread
 // per entry the two-channel layer's weight gradient (228 slices of 2608
-// entries) was a chain of 228 loads, 6.4 us.  The sums are deterministic.
+// entries) was a chain of 228 loads, 6.4 us.  Forward sums, whose ReLU turns
+// a last bit into a gradient's presence, are taken in slice order throughout.
 template <int GRP>
 __global__ void __launch_bounds__(256)
 k_sum_slices(const float4 *__restrict__ work, float4 *out, uint32_t n4, int nz, FastDiv fN4,
@@ -586,7 +817,7 @@ void sum_slices(const float *work, float *out, long long n, int nz, int N, const
                 cudaStream_t s) {
   const uint32_t n4 = (uint32_t)(n / 4);
   const FastDiv f((uint32_t)N / 4);
-  if (nz >= 16)
+  if (nz >= 16 && !e.relu)
     launch_pdl(k_sum_slices<8>, (n4 + 31) / 32, 256, s, (const float4 *)work, (float4 *)out, n4,
                nz, f, e);
   else
@@ -707,6 +938,52 @@ int cls_slices(long long M, long long K) {
   return (int)((chunks + per - 1) / per);
 }
 
+// Halo tiles fit when two stages do (227 KB a block, a little of it static); nz slices of `cslice`
+// chunks each.
+struct HaloPlan {
+  int nz, cslice, tiles, smem;
+};
+bool halo_ok(int R, int C, int N) {
+  return C % 16 == 0 && halo_table(R) + 2 * halo_stage(R, N) + 128 <= 226 * 1024;
+}
+
+// A split into nz slices takes ceil(tiles nz / slots) waves of blocks, each
+// about 3 us of set-up and stores and 1.3 us per chunk, plus the pass that
+// sums the slices (2.5 us and 8 bytes per slice entry at 6 TB/s).
+HaloPlan halo_plan(int R, int C, int N) {
+  HaloPlan pl;
+  pl.smem = halo_table(R) + 2 * halo_stage(R, N) + 128;
+  pl.tiles = (R + 7) / 8 * ((R * (R + 2) + 15) / 16) * R;
+  const int nch = 3 * (C / 16);
+  const int resident = std::max(1, std::min(2, 228 * 1024 / (pl.smem + 1024)));
+  const long long slots = (long long)resident * sm_count();
+  const double sum_us = (double)R * R * R * R * N * 8 / 6e6;
+  double best = 1e300;
+  for (int nz = 1; nz <= nch; ++nz) {
+    const int per = (nch + nz - 1) / nz, z = (nch + per - 1) / per;
+    const long long waves = (pl.tiles * (long long)z + slots - 1) / slots;
+    const double us = waves * (3.0 + 1.3 * per) + (z > 1 ? 2.5 + z * sum_us : 0.0);
+    if (us < best) best = us, pl.nz = z, pl.cslice = per;
+  }
+  return pl;
+}
+
+void launch_halo(const HaloArgs &a0, const HaloPlan &pl, cudaStream_t s) {
+  HaloArgs a = a0;
+  a.pitch = pow2_cols(a.N);
+  a.nacc = a.N > 64 ? 2 : 4;  // at most 256 columns: two blocks per SM
+  a.ncg = a.C / 16;
+  a.nx = (a.R + 7) / 8;
+  a.nr = (a.R * (a.R + 2) + 15) / 16;
+  a.cslice = pl.cslice;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_dgrad_halo, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           226 * 1024);
+  fh::cuda_check(attr, "cudaFuncSetAttribute(k_dgrad_halo)");
+  launch_pdl_smem(k_dgrad_halo, dim3(pl.tiles, 1, pl.nz), TB_W, (size_t)pl.smem, s, a);
+  fh::cuda_check(cudaGetLastError(), "k_dgrad_halo launch");
+}
+
 TcPlan plan_fwd(long long M, long long K, int cin, int cout) {
   return cin % 8 == 0 ? tc_plan_for<0, 1>(M, K, cout) : tc_plan_for<0, 0>(M, K, cout);
 }
@@ -724,11 +1001,13 @@ int net_tc_kpad(int cin, int ks) {
 size_t net_tc_work(int rin, int rout, int cin, int cout, bool first) {
   size_t w = 0;
   const long long Vi = (long long)rin * rin * rin * rin, Vo = (long long)rout * rout * rout * rout;
-  const TcPlan pf = plan_fwd(Vo, net_tc_kpad(cin, 3), cin, cout);
-  if (pf.nz > 1) w = std::max(w, (size_t)pf.nz * (size_t)Vo * cout);
+  const bool same = rin == rout;
+  const int nf = plan_fwd(Vo, net_tc_kpad(cin, 3), cin, cout).nz;
+  if (nf > 1) w = std::max(w, (size_t)nf * (size_t)Vo * cout);
   if (!first) {
-    const int nz = rin == rout ? tc_plan_for<1, 1>(Vi, 81LL * cout, cin).nz
-                               : cls_slices(Vo, 16LL * cout);
+    const int nz = !same ? cls_slices(Vo, 16LL * cout)
+                   : halo_ok(rin, cout, cin) ? halo_plan(rin, cout, cin).nz
+                                       : tc_plan_for<1, 1>(Vi, 81LL * cout, cin).nz;
     if (nz > 1) w = std::max(w, (size_t)nz * (size_t)Vi * cin);
   }
   const TcPlan pl = tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout);
@@ -773,6 +1052,21 @@ void net_tc_conv_fwd(const float *in, const uint16_t *wt, const float *b, float 
 void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, float *work,
                           int rin, int rout, int cin, int cout, int stride, NetGradEpi epi,
                           int *err, cudaStream_t s) {
+  if (stride == 1 && halo_ok(rin, cout, cin)) {
+    const HaloPlan pl = halo_plan(rin, cout, cin);
+    HaloArgs a{};
+    a.A = dout;
+    a.Bw = wb;
+    a.err = err;
+    a.R = rin, a.C = cout, a.N = cin;
+    a.epi = epi;
+    a.out = pl.nz > 1 ? work : din;
+    launch_halo(a, pl, s);
+    if (pl.nz > 1)
+      sum_slices(work, din, (long long)rin * rin * rin * rin * cin, pl.nz, cin,
+                 SumEpi{nullptr, 0, 0, epi}, s);
+    return;
+  }
   TcArgs a{};
   a.epi = epi;
   a.A = dout;
