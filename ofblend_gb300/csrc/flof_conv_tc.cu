@@ -10,7 +10,11 @@
 //   weight gradient:          acc += A_hi B_hi + A_lo B_hi + A_hi B_lo (3 MMAs)
 // with FP32 accumulation in tensor memory.
 //
-// Per block: 256 threads gather a 128 x 64 reduction chunk of the operand
+// Stride-1 gradients read each operand value once per tile (k_dgrad_halo,
+// k_wgrad_halo below).  The forward pass and the stride-2 gradients (k_conv_tc)
+// are implicit GEMMs over an im2col gather.
+//
+// k_conv_tc, per block: 256 threads gather a 128 x 64 reduction chunk of the operand
 // (im2col on the fly: voxel rows x (tap, channel), or (tap, channel) rows x
 // voxels for the weight gradient) through registers into shared memory in
 // the 128-byte-swizzled K-major layout (flof_tcgen05.cuh), while the
@@ -743,6 +747,280 @@ __global__ void __launch_bounds__(TB_W, 2) k_dgrad_halo(HaloArgs p) {
   }
 }
 
+// ---- stride-1 weight gradient from halo tiles -----------------------------------
+//
+// grad[tap][ci][co] = sum over voxels u of in[u][ci] dout[u + 1 - tap][co].  A
+// block keeps nine taps (all x and y offsets, one z and one t offset) of cc <=
+// 64 input and 16 output channels in tensor memory and walks its share of the
+// 128-voxel tiles (8 along x times 16 rows of the padded plane, as above).
+// Both operands are stored in 16-byte units of 8 channels, voxel by voxel, one
+// part (hi, lo) and channel group after another: the unswizzled MN-major
+// layout, 8 voxels to a core matrix.  The 18 rows of 10 voxels of dout that the
+// taps read are stored three times, each 8 voxels wide and shifted for its x
+// offset, so that one MMA per y offset and 16 voxels multiplies (hi, lo) input
+// channels (rows 0 .. cc - 1 and cc .. 2 cc - 1) by (hi, lo) x three x offsets
+// x 16 output channels (96 columns), and a y offset is a start address one row
+// on.  lo x lo is left out when the sums are taken out; rows past 2 cc multiply
+// whatever follows in shared memory and are never read.  The tensor core drops
+// bits at each accumulation: after at most WG_DRAIN tiles the sums are added to
+// the block's slice in FP32 and begin anew (without, the network's gradient at
+// 20^4 was 1.5 times as far from 64 bits as the im2col form's; with FP32 sums in
+// registers the kernel spilled and took 80 us).  The bias gradient is summed
+// in FP32 by the threads that stage dout, in the middle taps' block.
+// Bound by the latency of a tile's loads (the 288 columns leave room for one
+// block per SM): 48 -> 16 channels at 16^4 78 us (im2col 192; with the tap's
+// shift on the input's side, one MMA of 32 columns per tap from a misaligned
+// start, 120), 96 -> 32 at 8^4 23 (43), 64 -> 64 at 4^4 9 (11), 32 -> 32 at 8^4
+// 14 (12).
+struct WgradArgs {
+  const float *in, *dout;
+  float *out;             // slices: 2 per blockIdx.z, of 81 cin + 1 rows of cout
+  int *err;
+  int R, cin, cout;
+  int cc, ncc, nco;       // input channels per block, blocks of them, of 16 output channels
+  int nx, nr, tiles, per;  // tiles along x, of rows, in all, per slice
+  int drain;              // tiles between drains
+  FastDiv frp;            // by R + 2
+};
+
+constexpr int WG_CO = 16;                  // output channels of a block
+constexpr int WG_ROWS = 18, WG_NV = WG_ROWS * HX;  // dout rows and voxels of a tile
+constexpr int WG_BG = WG_ROWS * 128;       // bytes of a stored dout channel group
+constexpr int WG_N = 6 * WG_CO;            // columns of an MMA
+constexpr int WG_DRAIN = 20;               // most tiles (8 accumulations each) between drains
+constexpr int WG_COLS = 512;               // tensor-memory columns: 3 WG_N, a power of two
+
+__host__ __device__ constexpr int wg_stage(int cc) {
+  return 2 * (cc / 8) * TB_M * 16 + 6 * (WG_CO / 8) * WG_BG;
+}
+// the MMA's 128 rows read 16 channel groups, whatever cc: room for the second
+// stage's
+__host__ __device__ constexpr int wg_smem(int cc) {
+  const int st = wg_stage(cc), reach = st + 16 * TB_M * 16;
+  return (2 * st > reach ? 2 * st : reach) + 128;
+}
+
+__global__ void __launch_bounds__(TB_W, 1) k_wgrad_halo(WgradArgs p) {
+  constexpr int CO = WG_CO, NV = WG_NV, GO = CO / 8, BG = WG_BG;
+  constexpr int UA = 4;                            // input units per thread (cc = 64)
+  constexpr int UB = (GO * NV + TB_T - 1) / TB_T;  // dout units per thread
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t bars[2];
+  __shared__ uint32_t tbase;
+  unsigned char *smem = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int R = p.R, RP = R + 2, ga = p.cc / 8;
+  const int stage_bytes = wg_stage(p.cc);
+  // tap block (z offset, t offset), input and output channels
+  int q = blockIdx.x;
+  const int n0 = q % p.nco * CO;
+  q /= p.nco;
+  const int c0 = q % p.ncc * p.cc, tg = q / p.ncc;
+  const int dz = tg % 3, dt = tg / 3;
+  // the middle taps' block sees every voxel of dout
+  const bool bias = dz == 1 && dt == 1 && c0 == 0;
+  const int tbeg = blockIdx.z * p.per, tend = min(p.tiles, tbeg + p.per);
+
+  if (warp == 0) tmem_alloc(&tbase, (uint32_t)WG_COLS);
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  pdl_wait();
+  fence_before_sync();
+  __syncthreads();
+  pdl_launch_dependents();
+  fence_after_sync();
+  const uint32_t tacc = tbase;
+  // both operands MN-major (bits 15 and 16)
+  const uint32_t idesc = idesc_bf16_f32(TB_M, WG_N) | (1u << 15) | (1u << 16);
+  const bool producer = tid < TB_T;
+
+  float a[UA][8], b[UB][8], bsum[UB][8];
+#pragma unroll
+  for (int u = 0; u < UB; ++u)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bsum[u][j] = 0.f;
+  // the loads of a tile: ga x 128 units of the input, GO x NV of dout
+  auto load = [&](int tile) {
+    const int x0 = tile % p.nx * 8, rho0 = tile / p.nx % p.nr * 16, t = tile / (p.nx * p.nr);
+#pragma unroll
+    for (int u = 0; u < UA; ++u) {
+      const int e = tid + u * TB_T, g = e >> 7, r = e & (TB_M - 1);
+      const int rho = rho0 + (r >> 3), z = (int)p.frp.div((uint32_t)rho);
+      const int x = x0 + (r & 7), y = rho - z * RP;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[u][j] = 0.f;
+      if (g < ga && x < R && y < R && z < R)
+        load_ch8(a[u], p.in + (size_t)(x + R * (y + R * (z + R * t))) * p.cin + c0 + g * 8);
+    }
+    const float *base = p.dout + (size_t)(t + 1 - dt) * R * R * R * p.cout + n0;
+#pragma unroll
+    for (int u = 0; u < UB; ++u) {
+      const int e = tid + u * TB_T, g = e / NV, v = e - g * NV, row = v / HX;
+      const int rho = rho0 + RP * (2 - dz) + row;
+      const int zz = (int)p.frp.div((uint32_t)rho);
+      const int x = x0 + (v - row * HX) - 1, y = rho - zz * RP - 1, z = zz - 1;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[u][j] = 0.f;
+      if (g < GO && x >= 0 && x < R && y >= 0 && y < R && z >= 0 && z < R)
+        load_ch8(b[u], base + (size_t)(x + R * (y + R * z)) * p.cout + g * 8);
+    }
+  };
+  // the sums in tensor memory, written (first) or added to the block's rows of
+  // its slice; a hi row adds its products with lo dout.  Warps 0-3 and 4-7 take
+  // alternate taps.
+  const size_t slice = (size_t)(81 * p.cin + 1) * p.cout;
+  float *out = p.out + 2 * (size_t)blockIdx.z * slice;
+  auto drain = [&](bool first, bool zero) {
+    const int r = 32 * (warp & 3) + lane, part = r >= p.cc, ci = r - part * p.cc;
+    fence_after_sync();
+#pragma unroll 1
+    for (int tap = warp >> 2; tap < 9; tap += 2) {
+      const uint32_t ta = tacc + ((uint32_t)(32 * (warp & 3)) << 16) +
+                          (uint32_t)(tap / 3 * WG_N + tap % 3 * CO);
+      float v[16], w[16];
+      if (!zero) {
+        tmem_ld16(ta, v);
+        tmem_ld16(ta + 3 * CO, w);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = zero ? 0.f : part ? v[j] : v[j] + w[j];
+      if (r < 2 * p.cc) {
+        float4 *dst = reinterpret_cast<float4 *>(
+            out + part * slice + (size_t)((tap + 9 * tg) * p.cin + c0 + ci) * p.cout + n0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          if (!first) {
+            const float4 q4 = dst[j];
+            o = make_float4(q4.x + o.x, q4.y + o.y, q4.z + o.z, q4.w + o.w);
+          }
+          dst[j] = o;
+        }
+      }
+    }
+    fence_before_sync();
+  };
+  // tiles whose dout tile falls off the grid in t contribute nothing
+  const int plane = p.nx * p.nr;
+  const int lo = max(tbeg, dt == 2 ? plane : 0);
+  const int hi = min(tend, dt == 0 ? p.tiles - plane : p.tiles);
+
+  int issued = 0;  // tiles whose MMAs were issued (block-uniform)
+  bool bad = false, fresh = true;  // fresh: the next MMAs begin new sums
+  if (producer && lo < hi) load(lo);
+  for (int tile = lo; tile < hi; ++tile) {
+    const int s = issued & 1;
+    unsigned char *As = smem + s * stage_bytes, *Bs = As + 2 * ga * TB_M * 16;
+    if (producer && issued >= 2 && !mbar_wait_bounded(&bars[s], ((issued - 2) >> 1) & 1))
+      bad = true;
+    if (tile != lo && (tile - lo) % p.drain == 0) {
+      const int last = issued - 1;
+      if (producer && !bad && !mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) bad = true;
+      if (producer && !bad) drain(issued == p.drain, false);
+      fresh = true;
+    }
+    if (producer && !bad) {
+#pragma unroll
+      for (int u = 0; u < UA; ++u) {
+        const int e = tid + u * TB_T;
+        if ((e >> 7) < ga) {
+          uint4 h, l;
+          split8(a[u], h, l);
+          *reinterpret_cast<uint4 *>(As + e * 16) = h;
+          *reinterpret_cast<uint4 *>(As + (ga * TB_M + e) * 16) = l;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        const int e = tid + u * TB_T, g = e / NV, v = e - g * NV, row = v / HX;
+        const int xx = v - row * HX;
+        if (g < GO) {
+          uint4 h, l;
+          split8(b[u], h, l);
+          // groups [part][x offset][channel group]; column x of the copy for
+          // offset dx holds dout at x + 1 - dx, element x + 2 - dx of the row
+#pragma unroll
+          for (int dx = 0; dx < 3; ++dx) {
+            const int x = xx - 2 + dx;
+            if (x >= 0 && x < 8) {
+              unsigned char *dst = Bs + (dx * GO + g) * BG + row * 128 + x * 16;
+              *reinterpret_cast<uint4 *>(dst) = h;
+              *reinterpret_cast<uint4 *>(dst + 3 * GO * BG) = l;
+            }
+          }
+          // each voxel of dout once: the middle y offset's rows, eight columns
+          if (bias && row >= 1 && row <= 16 && xx >= 1 && xx <= 8)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bsum[u][j] += b[u][j];
+        }
+      }
+      if (tile + 1 < hi) load(tile + 1);  // in flight across the barrier and the MMAs
+      fence_proxy_async_smem();
+    }
+    if (__syncthreads_or(bad)) break;
+    if (tid == TB_T) {
+      fence_after_sync();
+      const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
+#pragma unroll 1
+      for (int ks = 0; ks < TB_M / 16; ++ks) {  // two rows of 8 voxels
+        const uint64_t da = smem_desc(a0 + ks * 256, 128, TB_M * 16);
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy)
+          mma_bf16(tacc + dy * WG_N, da, smem_desc(b0 + ks * 256 + (2 - dy) * 128, 128, BG), idesc,
+                   !fresh || ks > 0);
+      }
+      mma_commit(&bars[s]);
+    }
+    fresh = false;
+    ++issued;
+  }
+
+  // wait for the last issued tile (its commit covers every earlier MMA)
+  bool ok = !bad;
+  if (issued > 0) {
+    const int last = issued - 1;
+    if (!mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) ok = false;
+  }
+  if (!ok) atomicExch(p.err, FLOF_DEV_ERR_TC_TIMEOUT);
+  ok = __syncthreads_and(ok);
+  // a slice without a tile: zeros
+  if (ok && producer) drain(issued <= p.drain, issued == 0);
+  if (bias) {
+    // the threads' sums [group][voxel][8], then four partial sums per channel
+    float *bs = reinterpret_cast<float *>(smem), *bp = bs + GO * NV * 8;
+    if (producer)
+#pragma unroll
+      for (int u = 0; u < UB; ++u) {
+        const int e = tid + u * TB_T;
+        if (e < GO * NV)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) bs[e * 8 + j] = bsum[u][j];
+      }
+    __syncthreads();
+    if (tid < 4 * CO) {
+      const int n = tid % CO, h = tid / CO;
+      float x = 0.f;
+      for (int v = h; v < NV; v += 4) x += bs[((n >> 3) * NV + v) * 8 + (n & 7)];
+      bp[tid] = x;
+    }
+    __syncthreads();
+    if (tid < 2 * CO) {
+      const int n = tid % CO;
+      const float x = (bp[n] + bp[CO + n]) + (bp[2 * CO + n] + bp[3 * CO + n]);
+      out[(tid / CO) * slice + (size_t)81 * p.cin * p.cout + n0 + n] = tid < CO ? x : 0.f;
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tacc, (uint32_t)WG_COLS);
+  }
+}
+
 // What a sum of slices becomes as it is stored: forward: bias and ReLU; input
 // gradient: NetGradEpi; weight gradient: added to what is there (acc).
 struct SumEpi {
@@ -984,6 +1262,43 @@ void launch_halo(const HaloArgs &a0, const HaloPlan &pl, cudaStream_t s) {
   fh::cuda_check(cudaGetLastError(), "k_dgrad_halo launch");
 }
 
+// Weight gradient from halo tiles: blocks of at most 64 input and 16 output
+// channels, tiles per slice.  A block takes about 4 us of set-up and stores and
+// 1.2 us per tile, the sum of the slices 8 bytes per entry of a slice pair at 4
+// TB/s; the count with the lowest estimate wins.
+bool wgrad_halo_ok(int cin, int cout, int stride) {
+  return stride == 1 && cin % 16 == 0 && cout % 16 == 0;
+}
+struct WgradPlan {
+  int nz, per, tiles, ncc, nco;
+  int blocks() const { return 9 * ncc * nco; }
+};
+WgradPlan wgrad_halo_plan(int R, int cin, int cout) {
+  WgradPlan pl;
+  pl.ncc = (cin + 63) / 64;
+  while (cin % (8 * pl.ncc) != 0) ++pl.ncc;
+  pl.nco = cout / 16;
+  pl.tiles = (R + 7) / 8 * ((R * (R + 2) + 15) / 16) * R;
+  const double sum_us = (81.0 * cin + 1) * cout * 8 / 4e6;
+  double best = 1e300;
+  const int most = std::min(pl.tiles, 64);
+  for (int nz = 1; nz <= most; ++nz) {
+    const int per = (pl.tiles + nz - 1) / nz, z = (pl.tiles + per - 1) / per;
+    const int waves = (pl.blocks() * z + sm_count() - 1) / sm_count();
+    const double us = waves * (4.0 + 1.2 * per) + z * sum_us;
+    if (us < best) best = us, pl.nz = z, pl.per = per;
+  }
+  return pl;
+}
+
+void launch_wgrad_halo(const WgradArgs &a, const WgradPlan &pl, cudaStream_t s) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_wgrad_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, wg_smem(64));
+  fh::cuda_check(attr, "cudaFuncSetAttribute(k_wgrad_halo)");
+  launch_pdl_smem(k_wgrad_halo, dim3(pl.blocks(), 1, pl.nz), TB_W, (size_t)wg_smem(a.cc), s, a);
+  fh::cuda_check(cudaGetLastError(), "k_wgrad_halo launch");
+}
+
 TcPlan plan_fwd(long long M, long long K, int cin, int cout) {
   return cin % 8 == 0 ? tc_plan_for<0, 1>(M, K, cout) : tc_plan_for<0, 0>(M, K, cout);
 }
@@ -1010,8 +1325,10 @@ size_t net_tc_work(int rin, int rout, int cin, int cout, bool first) {
                                        : tc_plan_for<1, 1>(Vi, 81LL * cout, cin).nz;
     if (nz > 1) w = std::max(w, (size_t)nz * (size_t)Vi * cin);
   }
-  const TcPlan pl = tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout);
-  return std::max(w, (size_t)pl.nz * (81 * cin + 1) * cout);
+  const int nw = wgrad_halo_ok(cin, cout, same ? 1 : 2)
+                     ? 2 * wgrad_halo_plan(rin, cin, cout).nz
+                     : tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout).nz;
+  return std::max(w, (size_t)nw * (81 * cin + 1) * cout);
 }
 
 void net_weights_tc(const float *wq, uint16_t *wb, uint16_t *wt, int cin, int cout, int ks,
@@ -1106,6 +1423,26 @@ void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, flo
 void net_tc_conv_bwd_weight(const float *in, const float *dout, float *grad, float *work, int rin,
                             int rout, int cin, int cout, int stride, int acc, int *err,
                             cudaStream_t s) {
+  if (wgrad_halo_ok(cin, cout, stride)) {
+    const WgradPlan pl = wgrad_halo_plan(rin, cin, cout);
+    WgradArgs a{};
+    a.in = in;
+    a.dout = dout;
+    a.out = work;
+    a.err = err;
+    a.R = rin, a.cin = cin, a.cout = cout;
+    a.ncc = pl.ncc, a.cc = cin / pl.ncc, a.nco = pl.nco;
+    a.nx = (rin + 7) / 8;
+    a.nr = (rin * (rin + 2) + 15) / 16;
+    a.tiles = pl.tiles, a.per = pl.per;
+    const int drains = (pl.per + WG_DRAIN - 1) / WG_DRAIN;
+    a.drain = (pl.per + drains - 1) / drains;
+    a.frp = FastDiv((uint32_t)rin + 2);
+    launch_wgrad_halo(a, pl, s);
+    sum_slices(work, grad, (81LL * cin + 1) * cout, 2 * pl.nz, cout, SumEpi{nullptr, 0, acc, {}},
+               s);
+    return;
+  }
   TcArgs a{};
   a.A = in;
   a.B32 = dout;
