@@ -690,15 +690,16 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
     A = dst;
     float4 *B = tmp.v();
     CK(cudaMemsetAsync(dst, 0, vec_bytes(d), c->stream));
+    // The sweeps only rewrite unmarked interior cells; both buffers carry the
+    // projected values everywhere else (the reference's tmp copy).
+    if (doCvExtrapol > 0) CK(cudaMemsetAsync(B, 0, vec_bytes(d), c->stream));
     CK(cudaMemsetAsync(marker.p, 0, real_bytes(d), c->stream));
     CK(cudaMemsetAsync(pcount.p, 0, 2 * sizeof(unsigned int), c->stream));
     KLP(c, KC_PROJECT, d.x, d.cells() * 44,
-        launch_project_cells(dst, vel, phiOrg, phiTarget, marker.f(), d, threshPhi, maxIter,
-                             pqueue.p, (unsigned int *)pcount.p, c->stream));
+        launch_project_cells(dst, doCvExtrapol > 0 ? B : nullptr, vel, phiOrg, phiTarget,
+                             marker.f(), d, threshPhi, maxIter, pqueue.p,
+                             (unsigned int *)pcount.p, c->stream));
     if (doCvExtrapol > 0) {
-      // The sweeps only rewrite unmarked interior cells; both buffers carry
-      // the projected values everywhere else (the reference's tmp copy).
-      CK(cudaMemcpyAsync(B, A, vec_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
       if (c->slab_tma) {  // the plain-load sweeps read the marker
         KLP(c, KC_EXPOL_MASK, d.x, d.cells() * 4,
             launch_expol_mask(marker.f(), (uint16_t *)mask.p, d, c->stream));
@@ -729,20 +730,22 @@ void corr_vels_of(flof_ctx *c, Dims4 d, float4 *dst, float4 *vel, const float *p
       }
       std::swap(A, B);
     }
+    // setBound zeroes c <= resetBnd and c >= n - 1 - resetBnd: only the cells
+    // inside change vel, and only the last round's correction is handed out
     const int resetBnd = trunc_f(resetBndWidth * (float)d.x) + 1;
-    if (postVelBlur > 1e-6f)  // setBound zeroes c <= resetBnd and c >= n - 1 - resetBnd
-      gauss_blur(c, (float *)A, d, 4, (float)(0.5 * postVelBlur), blurType,
-                 resetBndWidth > 0.f ? inner_box(d, (long long)resetBnd + 1) : whole_box(d));
-    if (resetBndWidth > 0.f)
+    const CellBox box =
+        resetBndWidth > 0.f ? inner_box(d, (long long)resetBnd + 1) : whole_box(d);
+    if (postVelBlur > 1e-6f)
+      gauss_blur(c, (float *)A, d, 4, (float)(0.5 * postVelBlur), blurType, box);
+    KLP(c, KC_ELEMWISE, d.x, box.cells() * 48, launch_sub_box(vel, A, d, box, c->stream));
+    postVelBlur = (float)((double)postVelBlur * 0.5);
+    if (singleStep > 0) singleStep--;
+    const bool last = !(postVelBlur >= blurThreshold || singleStep);
+    if (last && resetBndWidth > 0.f)
       KLP(c, KC_BORDER, d.x, 0,
           launch_set_bound((float *)A, d, 4, make_float4(0.f, 0.f, 0.f, 0.f), resetBnd,
                              c->stream));
-    KLP(c, KC_ELEMWISE, d.x, d.cells() * 48,
-        launch_add_scaled((float *)vel, (const float *)A, d.cells(), 4,
-                            make_float4(-1.f, -1.f, -1.f, -1.f), c->stream));
-    postVelBlur = (float)((double)postVelBlur * 0.5);
-    if (singleStep > 0) singleStep--;
-    if (A != dst) {
+    if (last && A != dst) {
       // keep the round's correction in dst (the reference swaps pointers)
       CK(cudaMemcpyAsync(dst, A, vec_bytes(d), cudaMemcpyDeviceToDevice, c->stream));
       A = dst;

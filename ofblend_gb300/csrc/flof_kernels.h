@@ -347,6 +347,8 @@ inline CellBox grow_box(CellBox b, Dims4 d, int g, unsigned axes = 15u) {
     }
   return b;
 }
+// a -= b over the box's cells
+void launch_sub_box(float4 *a, const float4 *b, Dims4 d, const CellBox &box, cudaStream_t s);
 // One pass of knGaussianBlur over bnd=1 cells; when zero_border, the border
 // ring of dst is written with zeros.  wtab holds exp weights by squared
 // distance (host-computed, as the reference's float(exp(double))).
@@ -416,8 +418,9 @@ bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, co
 // knProjectCells in two kernels: the normals and the cells that finish
 // without a search, then the searches of the others, taken from `queue`
 // (project_queue_bytes(d) bytes: the whole box or a t slab of it at a time)
-// by whichever lane is free.  `counters` is two unsigned ints, zero on entry.
-void launch_project_cells(float4 *dst, const float4 *vel, const float *phiOrg,
+// by whichever lane is free.  `counters` is two unsigned ints, zero on entry;
+// dst, dst2 (nullable; receives what dst does) and marker are zero on entry.
+void launch_project_cells(float4 *dst, float4 *dst2, const float4 *vel, const float *phiOrg,
                           const float *phiTarget, float *marker, Dims4 d,
                           float threshPhi, int maxIter, void *queue, unsigned int *counters,
                           cudaStream_t s);

@@ -141,6 +141,26 @@ void launch_add_scaled(float *a, const float *b, long long ncell, int nc, float4
   binary_op<2>(a, b, ncell * nc, f, nc == 4, s);
 }
 
+__global__ void __launch_bounds__(NT)
+k_sub_box(float4 *__restrict__ a, const float4 *__restrict__ b, Dims4 d, BoxDecoder bx,
+          uint32_t n) {
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    int i, j, k, l;
+    bx.decode(q, i, j, k, l);
+    const idx_t id = d.index(i, j, k, l);
+    const float4 x = a[id], y = __ldg(b + id);
+    a[id] = make_float4(x.x - y.x, x.y - y.y, x.z - y.z, x.w - y.w);
+  }
+}
+void launch_sub_box(float4 *a, const float4 *b, Dims4 d, const CellBox &box, cudaStream_t s) {
+  const long long n = box.cells();
+  if (n == 0) return;
+  const BoxDecoder bx = make_decoder(box.hi[0] - box.lo[0], box.hi[1] - box.lo[1],
+                                     box.hi[2] - box.lo[2], box.lo[0], box.lo[1], box.lo[2],
+                                     box.lo[3]);
+  k_sub_box<<<grid_for(n, NT), NT, 0, s>>>(a, b, d, bx, (uint32_t)n);
+}
+
 // ---------------------------------------------------------------------------
 // Borders (grid4d.cpp:355-407)
 // ---------------------------------------------------------------------------

@@ -980,14 +980,16 @@ struct ProjState {
   uint32_t id, pad;
 };
 
-// The outcome of a cell's projection (optflow4d.cpp:725-732).
-__device__ __forceinline__ void project_write(float4 *__restrict__ dst, float *__restrict__ marker,
-                                              idx_t id, float4 nrm, float dd, float threshPhi) {
-  if (fabsf(dd) > threshPhi) {
-    dst[id] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
-  }
-  dst[id] = make_float4(nrm.x * dd, nrm.y * dd, nrm.z * dd, nrm.w * dd);
+// The outcome of a cell's projection (optflow4d.cpp:725-732): dst, dst2 (the
+// extrapolation's second buffer, nullable) and marker stay zero where the
+// distance found is above the threshold.
+__device__ __forceinline__ void project_write(float4 *__restrict__ dst, float4 *__restrict__ dst2,
+                                              float *__restrict__ marker, idx_t id, float4 nrm,
+                                              float dd, float threshPhi) {
+  if (fabsf(dd) > threshPhi) return;
+  const float4 v = make_float4(nrm.x * dd, nrm.y * dd, nrm.z * dd, nrm.w * dd);
+  dst[id] = v;
+  if (dst2) dst2[id] = v;
   marker[id] = 1.f;
 }
 
@@ -1000,7 +1002,8 @@ __device__ __forceinline__ void project_write(float4 *__restrict__ dst, float *_
 // that grid, 729 with the blocks refilled as they end, 690 with 6 blocks per SM;
 // 8 per SM 696).
 __global__ void __launch_bounds__(128, 6)
-k_project_prep(float4 *__restrict__ dst, const float4 *__restrict__ vel,
+k_project_prep(float4 *__restrict__ dst, float4 *__restrict__ dst2,
+               const float4 *__restrict__ vel,
                const float *__restrict__ phiOrg, const float *__restrict__ phiTarget,
                float *__restrict__ marker, Dims4 d, BoxDecoder bx, uint32_t nbox,
                float threshPhi, int maxIter, ProjState *__restrict__ queue,
@@ -1078,9 +1081,9 @@ k_project_prep(float4 *__restrict__ dst, const float4 *__restrict__ vel,
           for (int s = 0; s < maxIter; ++s) dd -= step;
         }
       }
-      project_write(dst, marker, id, nrm, dd, threshPhi);
+      project_write(dst, dst2, marker, id, nrm, dd, threshPhi);
     } else if (maxIter <= 0) {
-      project_write(dst, marker, id, nrm, dd, threshPhi);
+      project_write(dst, dst2, marker, id, nrm, dd, threshPhi);
     } else {
       search = true;
       S.p = make_float4(p0, p1, p2, p3);
@@ -1110,7 +1113,8 @@ k_project_prep(float4 *__restrict__ dst, const float4 *__restrict__ vel,
 // which lane runs a cell.
 constexpr int PROJ_CHUNK = 64;
 __global__ void __launch_bounds__(128)
-k_project_search(float4 *__restrict__ dst, const float *__restrict__ phiOrg,
+k_project_search(float4 *__restrict__ dst, float4 *__restrict__ dst2,
+                 const float *__restrict__ phiOrg,
                  float *__restrict__ marker, Dims4 d, float threshPhi, int maxIter,
                  const ProjState *__restrict__ queue, const unsigned int *__restrict__ qcount,
                  unsigned int *__restrict__ qhead) {
@@ -1187,7 +1191,7 @@ k_project_search(float4 *__restrict__ dst, const float *__restrict__ phiOrg,
     }
     if (++s >= maxIter) done = true;
     if (done) {
-      project_write(dst, marker, S.id, S.nrm, S.dd, threshPhi);
+      project_write(dst, dst2, marker, S.id, S.nrm, S.dd, threshPhi);
       active = false;
     }
     }
@@ -1214,7 +1218,7 @@ long long project_queue_cells(Dims4 d) {
 
 size_t project_queue_bytes(Dims4 d) { return sizeof(ProjState) * (size_t)project_queue_cells(d); }
 
-void launch_project_cells(float4 *dst, const float4 *vel, const float *phiOrg,
+void launch_project_cells(float4 *dst, float4 *dst2, const float4 *vel, const float *phiOrg,
                           const float *phiTarget, float *marker, Dims4 d,
                           float threshPhi, int maxIter, void *queue, unsigned int *counters,
                           cudaStream_t s) {
@@ -1234,9 +1238,9 @@ void launch_project_cells(float4 *dst, const float4 *vel, const float *phiOrg,
     const long long nbox = vol * nt;
     if (t0 > 0) k_zero_counters<<<1, 1, 0, s>>>(counters);
     k_project_prep<<<(unsigned)((nbox + 127) / 128), 128, 0, s>>>(
-        dst, vel, phiOrg, phiTarget, marker, d, bx, (uint32_t)nbox, threshPhi, maxIter,
+        dst, dst2, vel, phiOrg, phiTarget, marker, d, bx, (uint32_t)nbox, threshPhi, maxIter,
         (ProjState *)queue, counters);
-    k_project_search<<<sm_count() * per_sm, 128, 0, s>>>(dst, phiOrg, marker, d, threshPhi,
+    k_project_search<<<sm_count() * per_sm, 128, 0, s>>>(dst, dst2, phiOrg, marker, d, threshPhi,
                                                          maxIter, (const ProjState *)queue,
                                                          counters, counters + 1);
   }
