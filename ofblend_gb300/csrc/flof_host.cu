@@ -276,6 +276,9 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
   if (it != owner->tunes.end()) return it->second;
   const size_t vb = vec_bytes(d);
   DBuf p(c, vb), g(c, vb), q(c, vb), x(c, vb), r(c, vb), stb(c, sizeof(CGState));
+  DBuf p2(c, vb);
+  CGRing ring;
+  for (int m = 0; m < CG_RING; ++m) ring.p[m] = m % 2 ? p2.v() : p.v();
   CK(cudaMemsetAsync(p.p, 0, vb, c->stream));
   CK(cudaMemsetAsync(g.p, 0, vb, c->stream));
   CK(cudaMemsetAsync(x.p, 0, vb, c->stream));
@@ -306,7 +309,7 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
     CGTune cand = best;
     cand.mv_tt = tt;
     const float ms = time_it([&] {
-      launch_cg_matvec(p.v(), g.v(), q.v(), d, k, st, c->dpart, c->stream, cand);
+      launch_cg_matvec(p.v(), g.v(), q.v(), d, k, st, c->dpart, 0, c->stream, cand);
     });
     if (ms < bt) {
       bt = ms;
@@ -319,9 +322,9 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
     CGTune cand = best;
     cand.per_sm = ps;
     const float ms = time_it([&] {
-      launch_cg_update(r.v(), q.v(), g.v(), d, k, st, c->dpart, c->fpart, 1 << 30, c->stream,
-                       cand);
-      launch_cg_direction(x.v(), p.v(), r.v(), g.v(), d, k, st, c->stream, cand);
+      for (int slot = 0; slot < CG_RING; ++slot)
+        launch_cg_step(x.v(), r.v(), q.v(), ring, slot, g.v(), nullptr, d, k, st, c->dpart,
+                       c->fpart, 1 << 30, c->stream, cand);
     });
     if (ms < bt) {
       bt = ms;
@@ -340,30 +343,13 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
 // waiting; every kernel returns at once when the state says done.  After each
 // chunk the host reads the state (into c->st_h) and sizes the next chunk from
 // the observed reduction rate.
-void pcg_update(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 *r,
-                const float4 *q, const float4 *g, const float *i1, int maxIter) {
-  launch_cg_update(r, q, g, d, k, c->st, c->dpart, c->fpart, maxIter, c->stream, tu, i1);
-}
-void pcg_update(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 *r,
-                const float4 *q, const BF4 *g, const float *, int maxIter) {
-  launch_cg_update(r, q, g, d, k, c->st, c->dpart, c->fpart, maxIter, c->stream, tu);
-}
-void pcg_direction(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 *x,
-                   float4 *p, const float4 *r, const float4 *g, const float *i1) {
-  launch_cg_direction(x, p, r, g, d, k, c->st, c->stream, tu, i1);
-}
-void pcg_direction(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 *x,
-                   float4 *p, const float4 *r, const BF4 *g, const float *) {
-  launch_cg_direction(x, p, r, g, d, k, c->st, c->stream, tu);
-}
-
-// i1: the FP32 solve's target level set; the update and direction kernels
-// rebuild the preconditioner's gradient from it (null: they read g).
+// i1: the FP32 solve's target level set; the step kernel rebuilds the
+// preconditioner's gradient from it (null: it reads g).
 template <class GT>
 void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 *x, float4 *r,
               float4 *p, float4 *q, const GT *g, int maxIter, const float *i1 = nullptr) {
   const double gb = sizeof(GT) == 8 ? 8.0 : 16.0;  // bytes of g per cell
-  const double gpc = i1 ? 4.0 : gb;                 // bytes of g or i1 per cell in update/direction
+  const double gpc = i1 ? 4.0 : gb;                // bytes of g or i1 per cell in the step
   if (resident_cells_ok(d) && maxIter > 0) {
     // one cooperative launch; its blocks wait on one another, so its share of
     // the SMs is held until it has ended
@@ -386,16 +372,25 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
       return;
     }
   }
+  CGRing ring;
+  ring.p[0] = p;
+  DBuf more[CG_RING];
+  for (int m = 1; m < CG_RING; ++m) {
+    more[m] = DBuf(c, vec_bytes(d));
+    ring.p[m] = more[m].v();
+    CK(cudaMemsetAsync(ring.p[m], 0, vec_bytes(d), c->stream));  // the border rows
+  }
   int it = 0;
   int chunk = 4;
   for (;;) {
     const int n = (maxIter - it) < chunk ? (maxIter - it) : chunk;
     for (int s = 0; s < n; ++s) {
+      const int slot = (it + s) % CG_RING;
       KLP(c, KC_MATVEC, d.x, nint(d) * (32 + gb),
-          launch_cg_matvec(p, g, q, d, k, c->st, c->dpart, c->stream, tu));
-      KLP(c, KC_UPDATE, d.x, nint(d) * (48 + gpc),
-          pcg_update(c, d, k, tu, r, q, g, i1, maxIter));
-      KLP(c, KC_DIRECTION, d.x, nint(d) * (80 + gpc), pcg_direction(c, d, k, tu, x, p, r, g, i1));
+          launch_cg_matvec(ring.p[slot], g, q, d, k, c->st, c->dpart, slot, c->stream, tu));
+      KLP(c, KC_STEP, d.x, nint(d) * (80 + gpc + (slot == CG_RING - 1 ? 16 * (CG_RING + 1) : 0)),
+          launch_cg_step(x, r, q, ring, slot, g, i1, d, k, c->st, c->dpart, c->fpart, maxIter,
+                         c->stream, tu));
     }
     it += n;
     CK(cudaMemcpyAsync(c->st_h, c->st, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream));
@@ -413,6 +408,10 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
       chunk = chunk * 2 > 64 ? 64 : chunk * 2;
     }
   }
+  const int left = c->st_h->iters % CG_RING;  // directions not yet added to x
+  if (left > 0)
+    KLP(c, KC_STEP, d.x, nint(d) * (32 + 16 * left),
+        launch_cg_flush(x, ring, left, d, c->st, c->stream));
 }
 
 // The PCG with the reference's arithmetic (FLOF_OPT_STRICT): the same
@@ -484,7 +483,7 @@ int mg_pcg(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, const OFAr
   for (;;) {
     const int n = (cap - it) < chunk ? (cap - it) : chunk;
     for (int s = 0; s < n; ++s) {
-      KLP(c, KC_MATVEC, d.x, nb * 48, launch_cg_matvec(p, g, q, d, k, c->st, c->dpart, c->stream, tu));
+      KLP(c, KC_MATVEC, d.x, nb * 48, launch_matvec(p, g, q, d, k, c->st, c->dpart, c->stream, tu));
       KLP(c, KC_UPDATE, d.x, nb * (i1 ? 116 : 128),
           launch_mgcg_update_pre(x, r, p, q, g, i1, x0.v(), d, k, mp, c->st, c->fpart, cap,
                                  c->stream));

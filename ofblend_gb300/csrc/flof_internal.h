@@ -99,13 +99,13 @@ struct Pool {
 enum KClass {
   KC_OTHER = 0, KC_ASSEMBLE, KC_MATVEC, KC_UPDATE, KC_DIRECTION, KC_COPYBACK, KC_BLUR,
   KC_PROJECT, KC_EXPOL, KC_ADVECT, KC_RESAMPLE, KC_LSDIFF, KC_REDUCE, KC_ELEMWISE, KC_BORDER,
-  KC_LOOKUP, KC_DEFORM, KC_BLEND, KC_EXPOL_MASK, KC_MG, KC_RESIDENT, KC_COUNT
+  KC_LOOKUP, KC_DEFORM, KC_BLEND, KC_EXPOL_MASK, KC_MG, KC_RESIDENT, KC_STEP, KC_COUNT
 };
 inline const char *kc_names[KC_COUNT] = {
     "other", "of_assemble_init", "cg_matvec", "cg_update", "cg_direction", "of_copy_back",
     "gauss_blur", "project_cells", "expol_sweep", "advect", "resample", "ls_diff", "reduce",
     "elementwise", "border", "lookup_slice", "deform_twoway", "blend_slices", "expol_mask",
-    "mg_vcycle", "cg_resident"};
+    "mg_vcycle", "cg_resident", "cg_step"};
 
 struct ProfRec {
   int cls;

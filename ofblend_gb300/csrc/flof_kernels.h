@@ -130,6 +130,12 @@ void launch_lookup_slice_twoway(float *dst, int dx, int dy, int dz,
                                 float4 defoFactor, int bordSkip, cudaStream_t s);
 
 // ---- optical flow system and PCG ---------------------------------------------------
+// Search directions that a plain solve keeps before it adds them to x.
+constexpr int CG_RING = 4;
+struct CGRing {
+  float4 *p[CG_RING];
+};
+
 struct CGState {
   double sigma;     // z . r of the current iterate
   double alpha;     // sigma / (p . A p)
@@ -137,13 +143,14 @@ struct CGState {
   double acc;       // accuracy * max(r0)
   double resIni;    // max(r0)
   double pAp;
+  double aOld, sgOld, qzOld, pqOld;  // the last step's alpha, z.r, q.z and p.q
   float alphaf;     // (float)alpha and (float)beta, the values the kernels use
   float betaf;
+  float al[CG_RING];  // alpha of the directions in the ring
   float resMax;     // max(r) after the last update
   float retResidual;  // resMax / resIni
   int done;         // 0 running; see CG_* below
   int iters;
-  int xpend;        // 1: x += alpha p of the last update is still to be applied
   unsigned int counter[4];
   unsigned int gbar;  // arrivals at the resident solve's grid barriers
 };
@@ -175,33 +182,29 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
                              float4 *p, float4 *x, Dims4 d, OFConsts c,
                              float accuracy, CGState *st, double *dpart,
                              float *fpart, cudaStream_t s);
-void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d,
-                      OFConsts c, CGState *st, double *dpart, cudaStream_t s,
-                      const CGTune &tu = CGTune());
-// The update (r -= alpha q, z.r, max r) takes the iteration number from
-// st->iters and leaves x += alpha p to the direction kernel, which reads p
-// anyway (st->xpend); the direction kernel applies it even after the update
-// has ended the solve.  The x values are those of the textbook order bit for
-// bit.
+// q = A p, p.q and alpha.
+void launch_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
+                   double *dpart, cudaStream_t s, const CGTune &tu = CGTune());
+// One iteration of the plain PCG is launch_cg_matvec and launch_cg_step with
+// slot = iteration % CG_RING.  The matvec reads ring.p[slot] and forms alpha and
+// beta; the step updates r, writes the next direction to the ring's next
+// buffer, and in the last slot adds the ring's directions to x.  launch_cg_flush
+// adds what is left when the solve ends in another slot.
 // With i1 (the level's target level set, from which the assembly built g)
-// the two kernels rebuild g from it instead of reading g.
-void launch_cg_update(float4 *r, const float4 *q, const float4 *g, Dims4 d, OFConsts c,
-                      CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
-                      const CGTune &tu = CGTune(), const float *i1 = nullptr);
-void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const float4 *g, Dims4 d,
-                         OFConsts c, CGState *st, cudaStream_t s,
-                         const CGTune &tu = CGTune(), const float *i1 = nullptr);
-// The same three kernels with the image gradient stored in BF16 (mixed
-// precision: the matrix g g^T + diag I is built from the rounded gradient).
-void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d,
-                      OFConsts c, CGState *st, double *dpart, cudaStream_t s,
-                      const CGTune &tu = CGTune());
-void launch_cg_update(float4 *r, const float4 *q, const BF4 *g, Dims4 d, OFConsts c,
-                      CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
-                      const CGTune &tu = CGTune());
-void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const BF4 *g, Dims4 d,
-                         OFConsts c, CGState *st, cudaStream_t s,
-                         const CGTune &tu = CGTune());
+// the step rebuilds g from it instead of reading g.  g in BF16: mixed
+// precision (the matrix g g^T + diag I is built from the rounded gradient).
+void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
+                      CGState *st, double *dpart, int slot, cudaStream_t s, const CGTune &tu);
+void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
+                      double *dpart, int slot, cudaStream_t s, const CGTune &tu);
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+                    const float4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st,
+                    double *dpart, float *fpart, int maxIter, cudaStream_t s, const CGTune &tu);
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+                    const BF4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st, double *dpart,
+                    float *fpart, int maxIter, cudaStream_t s, const CGTune &tu);
+void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState *st,
+                     cudaStream_t s);
 // ---- resident PCG (flof_resident.cu) -------------------------------------------
 // The whole iteration of a level whose cells fit the SMs as one cooperative
 // launch, from the state that the assembly or launch_cg_init_r left; it ends

@@ -166,7 +166,6 @@ k_cg_init_r(const float4 *__restrict__ r, const GT *__restrict__ g, float4 *__re
       st->resIni = residual;
       st->resMax = m;
       st->iters = 0;
-      st->xpend = 0;
       st->gbar = 0;
       st->counter[0] = 0;
       if (residual < (double)1e-6f) {

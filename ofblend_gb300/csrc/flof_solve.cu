@@ -129,7 +129,6 @@ k_of_assemble_init(const float *__restrict__ i0w, const float *__restrict__ i1,
       st->resIni = residual;
       st->resMax = m;
       st->iters = 0;
-      st->xpend = 0;
       st->gbar = 0;
       st->counter[0] = 0;
       if (residual < (double)1e-6f) {
@@ -178,7 +177,46 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
 // the z-neighbour loads hit L2.  The grid is persistent (a fixed number of
 // blocks per SM); p.Ap is accumulated per thread in float-float and summed
 // in double by the last block to finish, in a fixed order.
+//
+// DOTS (the plain PCG): the kernel also forms q.M^-1 q, from which its last
+// block predicts the next z.r, and so beta, before r is updated (cg_scalars).
+// The step kernel then has alpha and beta and updates r and p in one pass.
+// The extra sum costs 6 us of 148 at 64^4.  The loads need the eight blocks per
+// SM that 64 registers allow: at 105 registers it takes 186 us; with correctly
+// rounded reciprocals, 195-200.
 constexpr int MV_NT = 128;
+
+// alpha, and beta before the step that it belongs to.  With r' = r - a q,
+//   z'.r' = z.r - 2 a q.z + a^2 q.M^-1 q,
+// where q.z is not summed but follows from p.q: z = p - b p_old (b and p_old
+// the last step's), so q.z = p.q - b q.p_old.  q.p_old is zero but for
+// rounding; that rounding must not be left out, as each step would double it.
+// It is known from the last step's sums (A symmetric, q_old = (r_old - r) / a_old,
+// and the sigma that the step summed afresh from the updated r):
+//   q.p_old = p.q_old = z.q_old + b p_old.q_old,
+//   z.q_old = (z.r_old - z.r) / a_old,  z.r_old = z_old.r = z_old.r_old - a_old q_old.z_old.
+// So no error passes from one beta to the next but the rounding of the vectors.
+// alpha itself uses the fresh sigma.
+__device__ __forceinline__ void cg_scalars(CGState *st, double pq, double qmq, int slot) {
+  const double sg = st->sigma;
+  st->pAp = pq;
+  st->alpha = sg / pq;
+  st->alphaf = (float)st->alpha;
+  st->al[slot] = st->alphaf;
+  const double a = (double)st->alphaf;  // the value the step uses
+  double qz = pq;
+  if (st->iters > 0) {
+    const double ao = st->aOld, bo = (double)st->betaf;
+    const double zro = st->sgOld - ao * st->qzOld;
+    qz -= bo * ((zro - sg) / ao + bo * st->pqOld);
+  }
+  st->beta = fma(a * a, qmq, fma(-2.0 * a, qz, sg)) / sg;
+  st->betaf = (float)st->beta;
+  st->aOld = a;
+  st->sgOld = sg;
+  st->qzOld = qz;
+  st->pqOld = pq;
+}
 
 struct MVShape {
   FastDiv fx;        // interior x extent
@@ -213,21 +251,25 @@ __device__ __forceinline__ void mv_load(MVLoads &a, const float4 *__restrict__ p
   a.zp = __ldg(p + id + sZ);
 }
 
+__device__ __forceinline__ float rcp_1ulp(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // OFFD: the neighbour terms are present (applyMat skips them for a zero
 // off-diagonal, optflow4d.cpp:215).  MV_TT: t planes per work item.
-template <bool OFFD, int MV_TT, class GT>
-__global__ void __launch_bounds__(MV_NT)
+template <bool OFFD, int MV_TT, bool DOTS, class GT>
+__global__ void __launch_bounds__(MV_NT, 8)
 k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
             float4 *__restrict__ q, Dims4 d, MVShape sh, OFConsts c, CGState *st,
-            double *dpart) {
+            double *dpart, int slot) {
   pdl_wait();
   pdl_launch_dependents();
-  // the previous direction kernel has applied any pending x update
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->xpend = 0;
   if (st->done) return;
   __shared__ double shd[MV_NT / 32];
   __shared__ FF shff[MV_NT / 32];
-  FF dot = {0.f, 0.f};
+  FF dot = {0.f, 0.f}, dotm = {0.f, 0.f};
   const idx_t sY = d.x, sZ = d.sz(), sT = d.st();
   const float o = c.offd;
   for (int item = blockIdx.x; item < sh.items; item += gridDim.x) {
@@ -277,21 +319,42 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
       ff_add(dot, pc.y * qq.y);
       ff_add(dot, pc.z * qq.z);
       ff_add(dot, pc.w * qq.w);
+      if (DOTS) {
+        // for beta only, whose own rounding to float is larger than the last
+        // bit of these reciprocals
+        const float ux = rcp_1ulp(cur.gg.x * cur.gg.x + c.diag) * qq.x;
+        const float uy = rcp_1ulp(cur.gg.y * cur.gg.y + c.diag) * qq.y;
+        const float uz = rcp_1ulp(cur.gg.z * cur.gg.z + c.diag) * qq.z;
+        const float uw = rcp_1ulp(cur.gg.w * cur.gg.w + c.diag) * qq.w;
+        ff_add(dotm, (ux * qq.x + uy * qq.y) + (uz * qq.z + uw * qq.w));
+      }
       pm = pc;
       pc = cur.pp;
       cur = nxt;
     }
   }
   const double bd = block_sum_ff<MV_NT>(dot, shff);
-  if (threadIdx.x == 0) dpart[blockIdx.x] = bd;
+  const double bm = DOTS ? block_sum_ff<MV_NT>(dotm, shff) : 0.0;
+  if (threadIdx.x == 0) {
+    dpart[blockIdx.x] = bd;
+    if (DOTS) dpart[gridDim.x + blockIdx.x] = bm;
+  }
   if (last_block_arrives(&st->counter[1])) {
-    double s = 0.0;
-    for (int q2 = threadIdx.x; q2 < (int)gridDim.x; q2 += blockDim.x) s += __ldcg(dpart + q2);
+    double s = 0.0, sm = 0.0;
+    for (int q2 = threadIdx.x; q2 < (int)gridDim.x; q2 += blockDim.x) {
+      s += __ldcg(dpart + q2);
+      if (DOTS) sm += __ldcg(dpart + gridDim.x + q2);
+    }
     s = block_sum<MV_NT>(s, shd);
+    if (DOTS) sm = block_sum<MV_NT>(sm, shd);
     if (threadIdx.x == 0) {
-      st->pAp = s;
-      st->alpha = st->sigma / s;
-      st->alphaf = (float)st->alpha;
+      if (DOTS) {
+        cg_scalars(st, s, sm, slot);
+      } else {
+        st->pAp = s;
+        st->alpha = st->sigma / s;
+        st->alphaf = (float)st->alpha;
+      }
       st->counter[1] = 0;
     }
   }
@@ -299,9 +362,9 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
 
 namespace {
 
-template <bool OFFD, int TT, class GT>
+template <bool OFFD, int TT, bool DOTS, class GT>
 void matvec_variant(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c,
-                    CGState *st, double *dpart, cudaStream_t s) {
+                    CGState *st, double *dpart, cudaStream_t s, int slot) {
   MVShape sh;
   const int ex = d.x > 2 ? d.x - 2 : 1, ey = d.y > 2 ? d.y - 2 : 1;
   const int ez = d.z > 2 ? d.z - 2 : 1;
@@ -316,49 +379,52 @@ void matvec_variant(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c
   // resident blocks per SM of this instantiation (computed once, thread-safe)
   static const int per_sm = [] {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_cg_matvec<OFFD, TT, GT>, MV_NT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_cg_matvec<OFFD, TT, DOTS, GT>, MV_NT, 0);
     return n < 1 ? 1 : n;
   }();
   int blocks = sm_count() * per_sm;
   if (blocks > sh.items) blocks = sh.items > 0 ? sh.items : 1;
-  launch_pdl(k_cg_matvec<OFFD, TT, GT>, blocks, MV_NT, s, p, g, q, d, sh, c, st, dpart);
+  launch_pdl(k_cg_matvec<OFFD, TT, DOTS, GT>, blocks, MV_NT, s, p, g, q, d, sh, c, st, dpart,
+             slot);
 }
 
-template <bool OFFD, class GT>
+template <bool OFFD, bool DOTS, class GT>
 void matvec_tt(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
-               double *dpart, cudaStream_t s, int tt) {
+               double *dpart, cudaStream_t s, int tt, int slot) {
   if (tt <= 4)
-    matvec_variant<OFFD, 4>(p, g, q, d, c, st, dpart, s);
+    matvec_variant<OFFD, 4, DOTS>(p, g, q, d, c, st, dpart, s, slot);
   else if (tt >= 16)
-    matvec_variant<OFFD, 16>(p, g, q, d, c, st, dpart, s);
+    matvec_variant<OFFD, 16, DOTS>(p, g, q, d, c, st, dpart, s, slot);
   else
-    matvec_variant<OFFD, 8>(p, g, q, d, c, st, dpart, s);
+    matvec_variant<OFFD, 8, DOTS>(p, g, q, d, c, st, dpart, s, slot);
 }
 
-template <class GT>
+template <bool DOTS, class GT>
 void matvec_any(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
-                double *dpart, cudaStream_t s, const CGTune &tu) {
+                double *dpart, cudaStream_t s, const CGTune &tu, int slot) {
   if (c.offd != 0.f)
-    matvec_tt<true>(p, g, q, d, c, st, dpart, s, tu.mv_tt);
+    matvec_tt<true, DOTS>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
   else
-    matvec_tt<false>(p, g, q, d, c, st, dpart, s, tu.mv_tt);
+    matvec_tt<false, DOTS>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
 }
 
 }  // namespace
 
-void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d,
-                      OFConsts c, CGState *st, double *dpart, cudaStream_t s,
-                      const CGTune &tu) {
-  matvec_any(p, g, q, d, c, st, dpart, s, tu);
+void launch_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
+                   double *dpart, cudaStream_t s, const CGTune &tu) {
+  matvec_any<false>(p, g, q, d, c, st, dpart, s, tu, 0);
 }
-void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d,
-                      OFConsts c, CGState *st, double *dpart, cudaStream_t s,
-                      const CGTune &tu) {
-  matvec_any(p, g, q, d, c, st, dpart, s, tu);
+void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
+                      CGState *st, double *dpart, int slot, cudaStream_t s, const CGTune &tu) {
+  matvec_any<true>(p, g, q, d, c, st, dpart, s, tu, slot);
+}
+void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
+                      double *dpart, int slot, cudaStream_t s, const CGTune &tu) {
+  matvec_any<true>(p, g, q, d, c, st, dpart, s, tu, slot);
 }
 
-// Where the update and direction kernels take the image gradient g for the
-// Jacobi preconditioner from: the stored g (FP32 or BF16), or g rebuilt from
+// Where the step kernel takes the image gradient g for the Jacobi
+// preconditioner from: the stored g (FP32 or BF16), or g rebuilt from
 // the target level set i1 with the assembly's own operations (central
 // differences times 1/(2 mDx), the same values bit for bit).  i1 is 4 bytes
 // per cell against 16 for g; its neighbour loads hit L1 and L2.
@@ -368,36 +434,87 @@ struct GradStored {
   __device__ __forceinline__ float4 operator()(idx_t id) const { return ld_g(g, id); }
 };
 
-// r -= alpha q; z = M^-1 r; sigma' = z.r; max(r).  x += alpha p is left to
-// the direction kernel (st->xpend).
-template <class GS>
+// r -= alpha q; z = M^-1 r; the next p = z + beta p; sigma' = z.r; max(r); and
+// in every CG_RING-th step x += the last CG_RING alpha p, added in order.
+//
+// Bound by HBM: q, r and p read, r and p written, i1 for g (84 bytes a cell),
+// and x.  Adding to x in every step reads and writes it each time (32 bytes);
+// the directions are kept in CG_RING buffers instead, so that a step in
+// CG_RING reads the earlier ones again and x once: (32 + 16 (CG_RING - 1)) /
+// CG_RING bytes a step, 20 for four buffers.  The ring's alpha p are added to
+// one another before they are added to x, so x is rounded once in four steps
+// (64^4 deformation against 64 bits: 7.5e-7 relative, 7.9e-7 when every step
+// adds to x).
+// An iteration (matvec and step) moves 152 bytes a cell; three kernels (matvec,
+// r, then x and p) moved 184.  Step at 64^4: 247 us (6.2 TB/s) with four
+// buffers, 259 with two, 270 with one; r and then x and p took 130 + 190 us.
+// Iteration: 64^4 463 -> 395 us, 48^4 166 -> 140, 40 x 42 x 38 x 48 107 -> 93.
+// pin and pout may be one buffer (CG_RING = 1); a cell is read before it is
+// written, by the same thread.
+__device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
+  x.x = __fmaf_rn(a, p.x, x.x);
+  x.y = __fmaf_rn(a, p.y, x.y);
+  x.z = __fmaf_rn(a, p.z, x.z);
+  x.w = __fmaf_rn(a, p.w, x.w);
+}
+
+template <bool XP, class GS>
 __global__ void __launch_bounds__(NT)
-k_cg_update(float4 *__restrict__ r, const float4 *__restrict__ q, GS gs, Dims4 d, BoxDecoder bx,
-            uint32_t nint, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter) {
+k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restrict__ q,
+          CGRing ring, const float4 *pin, float4 *pout, GS gs, Dims4 d, BoxDecoder bx,
+          uint32_t nint, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter) {
   pdl_wait();
   pdl_launch_dependents();
   if (st->done) return;
   __shared__ double shd[NT / 32];
   __shared__ FF shff[NT / 32];
   __shared__ float shf[NT / 32];
-  const float a = st->alphaf;
+  const float a = st->alphaf, b = st->betaf;
+  float al[CG_RING];
+#pragma unroll
+  for (int m = 0; m < CG_RING; ++m) al[m] = st->al[m];
   FF dot = {0.f, 0.f};
   float mx = -FLT_MAX;
-  auto cell = [&](idx_t id, float4 qq, float4 gv, float4 rr) {
-    rr.x = __fmaf_rn(-a, qq.x, rr.x);
-    rr.y = __fmaf_rn(-a, qq.y, rr.y);
-    rr.z = __fmaf_rn(-a, qq.z, rr.z);
-    rr.w = __fmaf_rn(-a, qq.w, rr.w);
+  struct In {
+    float4 q, g, r, p, x, po[CG_RING];
+  };
+  auto load = [&](idx_t id) {
+    In v;
+    v.q = __ldg(q + id);
+    v.r = r[id];
+    v.p = pin[id];
+    if (XP) {
+      v.x = x[id];
+#pragma unroll
+      for (int m = 0; m + 1 < CG_RING; ++m) v.po[m] = ring.p[m][id];
+    }
+    v.g = gs(id);
+    return v;
+  };
+  auto cell = [&](idx_t id, const In &v) {
+    float4 rr = v.r, pp = v.p;
+    axpy4(rr, -a, v.q);
     r[id] = rr;
-    const float4 pre = precond_of(gv, c.diag);
-    ff_add(dot, (rr.x * pre.x) * rr.x);
-    ff_add(dot, (rr.y * pre.y) * rr.y);
-    ff_add(dot, (rr.z * pre.z) * rr.z);
-    ff_add(dot, (rr.w * pre.w) * rr.w);
+    const float4 pre = precond_of(v.g, c.diag);
+    const float4 z = make_float4(rr.x * pre.x, rr.y * pre.y, rr.z * pre.z, rr.w * pre.w);
+    if (XP) {
+      float4 t = make_float4(a * pp.x, a * pp.y, a * pp.z, a * pp.w);
+#pragma unroll
+      for (int m = CG_RING - 2; m >= 0; --m) axpy4(t, al[m], v.po[m]);
+      x[id] = make_float4(v.x.x + t.x, v.x.y + t.y, v.x.z + t.z, v.x.w + t.w);
+    }
+    pp.x = __fmaf_rn(b, pp.x, z.x);
+    pp.y = __fmaf_rn(b, pp.y, z.y);
+    pp.z = __fmaf_rn(b, pp.z, z.z);
+    pp.w = __fmaf_rn(b, pp.w, z.w);
+    pout[id] = pp;
+    ff_add(dot, z.x * rr.x);
+    ff_add(dot, z.y * rr.y);
+    ff_add(dot, z.z * rr.z);
+    ff_add(dot, z.w * rr.w);
     mx = fmaxf(mx, fmaxf(fmaxf(rr.x, rr.y), fmaxf(rr.z, rr.w)));
   };
-  // two cells per trip with all loads issued first (the thread's cell order,
-  // and so the sum order, is that of the plain grid-stride loop)
+  // two cells per trip with all loads issued first
   const uint32_t stride = gridDim.x * blockDim.x;
   uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   for (; n + stride < nint; n += 2 * stride) {
@@ -406,17 +523,15 @@ k_cg_update(float4 *__restrict__ r, const float4 *__restrict__ q, GS gs, Dims4 d
     const idx_t i0 = d.index(i, j, k, l);
     bx.decode(n + stride, i, j, k, l);
     const idx_t i1 = d.index(i, j, k, l);
-    const float4 q0 = __ldg(q + i0), q1 = __ldg(q + i1);
-    const float4 g0 = gs(i0), g1 = gs(i1);
-    const float4 r0 = r[i0], r1 = r[i1];
-    cell(i0, q0, g0, r0);
-    cell(i1, q1, g1, r1);
+    const In v0 = load(i0), v1 = load(i1);
+    cell(i0, v0);
+    cell(i1, v1);
   }
   if (n < nint) {
     int i, j, k, l;
     bx.decode(n, i, j, k, l);
     const idx_t i0 = d.index(i, j, k, l);
-    cell(i0, __ldg(q + i0), gs(i0), r[i0]);
+    cell(i0, load(i0));
   }
   const double bd = block_sum_ff<NT>(dot, shff);
   const float bm = block_max<NT>(mx, shf);
@@ -439,17 +554,35 @@ k_cg_update(float4 *__restrict__ r, const float4 *__restrict__ q, GS gs, Dims4 d
       st->resMax = m;
       st->retResidual = (float)(residual / st->resIni);
       st->iters = iter + 1;
-      st->xpend = 1;
       st->counter[2] = 0;
       if (residual <= st->acc) {
         st->done = CG_CONVERGED;
       } else {
-        st->beta = s / st->sigma;
-        st->betaf = (float)st->beta;
         st->sigma = s;
         if (iter + 1 >= maxIter) st->done = CG_MAXITER;
       }
     }
+  }
+}
+
+// x += the first `count` alpha p of the ring, the ones that no step has added.
+__global__ void __launch_bounds__(NT)
+k_cg_flush(float4 *__restrict__ x, CGRing ring, int count, Dims4 d, BoxDecoder bx, uint32_t nint,
+           const CGState *st) {
+  pdl_wait();
+  pdl_launch_dependents();
+  float al[CG_RING];
+#pragma unroll
+  for (int m = 0; m < CG_RING; ++m) al[m] = st->al[m];
+  for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < nint; n += gridDim.x * blockDim.x) {
+    int i, j, k, l;
+    bx.decode(n, i, j, k, l);
+    const idx_t id = d.index(i, j, k, l);
+    float4 xx = x[id], t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int m = CG_RING - 2; m >= 0; --m)
+      if (m < count) axpy4(t, al[m], __ldg(ring.p[m] + id));
+    x[id] = make_float4(xx.x + t.x, xx.y + t.y, xx.z + t.z, xx.w + t.w);
   }
 }
 
@@ -466,127 +599,44 @@ int resident_per_sm(K kernel, int want) {
   return want < n ? want : n;
 }
 
-template <class GS>
-void update_launch(float4 *r, const float4 *q, GS gs, Dims4 d, OFConsts c, CGState *st,
-                   double *dpart, float *fpart, int maxIter, cudaStream_t s, const CGTune &tu) {
-  static const int occ = resident_per_sm(k_cg_update<GS>, 1 << 30);
+template <bool XP, class GS>
+void step_launch(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs,
+                 Dims4 d, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter,
+                 cudaStream_t s, const CGTune &tu) {
+  static const int occ = resident_per_sm(k_cg_step<XP, GS>, 1 << 30);
   const long long n = interior_count(d);
-  launch_pdl(k_cg_update<GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
-             NT, s, r, q, gs, d, interior_decoder(d), (uint32_t)n, c, st, dpart, fpart, maxIter);
+  launch_pdl(k_cg_step<XP, GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
+             NT, s, x, r, q, ring, (const float4 *)ring.p[slot], ring.p[XP ? 0 : slot + 1], gs, d,
+             interior_decoder(d), (uint32_t)n, c, st, dpart, fpart, maxIter);
 }
-void launch_cg_update(float4 *r, const float4 *q, const float4 *g, Dims4 d, OFConsts c,
-                      CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
-                      const CGTune &tu, const float *i1) {
-  if (i1)
-    update_launch(r, q, GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, d, c, st, dpart, fpart,
-                  maxIter, s, tu);
+template <class GS>
+void step_any(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs, Dims4 d,
+              OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
+              const CGTune &tu) {
+  if (slot == CG_RING - 1)
+    step_launch<true>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
   else
-    update_launch(r, q, GradStored<float4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_launch<false>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
 }
-void launch_cg_update(float4 *r, const float4 *q, const BF4 *g, Dims4 d, OFConsts c,
-                      CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
-                      const CGTune &tu) {
-  update_launch(r, q, GradStored<BF4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+                    const float4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st,
+                    double *dpart, float *fpart, int maxIter, cudaStream_t s, const CGTune &tu) {
+  if (i1)
+    step_any(x, r, q, ring, slot, GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, d, c, st, dpart,
+             fpart, maxIter, s, tu);
+  else
+    step_any(x, r, q, ring, slot, GradStored<float4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
 }
-
-// x += alpha p (the last update's, when pending); then, while the solve
-// runs, p = z + beta p.
-template <bool XP, bool PN, class GS>
-__device__ __forceinline__ void direction_cells(float4 *__restrict__ x, float4 *__restrict__ p,
-                                                const float4 *__restrict__ r, const GS &gs,
-                                                const Dims4 &d, const BoxDecoder &bx,
-                                                uint32_t nint, const OFConsts &c, float a,
-                                                float b) {
-  struct In {
-    float4 p, x, r, g;
-  };
-  auto load = [&](idx_t id) {
-    In v;
-    v.p = p[id];
-    if (XP) v.x = x[id];
-    if (PN) {
-      v.r = __ldg(r + id);
-      v.g = gs(id);
-    }
-    return v;
-  };
-  auto cell = [&](idx_t id, const In &v) {
-    float4 pp = v.p;
-    if (XP) {
-      float4 xx = v.x;
-      xx.x = __fmaf_rn(a, pp.x, xx.x);
-      xx.y = __fmaf_rn(a, pp.y, xx.y);
-      xx.z = __fmaf_rn(a, pp.z, xx.z);
-      xx.w = __fmaf_rn(a, pp.w, xx.w);
-      x[id] = xx;
-    }
-    if (PN) {
-      const float4 rr = v.r;
-      const float4 pre = precond_of(v.g, c.diag);
-      pp.x = __fmaf_rn(b, pp.x, rr.x * pre.x);
-      pp.y = __fmaf_rn(b, pp.y, rr.y * pre.y);
-      pp.z = __fmaf_rn(b, pp.z, rr.z * pre.z);
-      pp.w = __fmaf_rn(b, pp.w, rr.w * pre.w);
-      p[id] = pp;
-    }
-  };
-  // two cells per trip with all loads issued first
-  const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; n + stride < nint; n += 2 * stride) {
-    int i, j, k, l;
-    bx.decode(n, i, j, k, l);
-    const idx_t i0 = d.index(i, j, k, l);
-    bx.decode(n + stride, i, j, k, l);
-    const idx_t i1 = d.index(i, j, k, l);
-    const In v0 = load(i0), v1 = load(i1);
-    cell(i0, v0);
-    cell(i1, v1);
-  }
-  if (n < nint) {
-    int i, j, k, l;
-    bx.decode(n, i, j, k, l);
-    const idx_t i0 = d.index(i, j, k, l);
-    cell(i0, load(i0));
-  }
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+                    const BF4 *g, const float *, Dims4 d, OFConsts c, CGState *st, double *dpart,
+                    float *fpart, int maxIter, cudaStream_t s, const CGTune &tu) {
+  step_any(x, r, q, ring, slot, GradStored<BF4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
 }
-
-template <class GS>
-__global__ void __launch_bounds__(NT)
-k_cg_direction(float4 *__restrict__ x, float4 *__restrict__ p, const float4 *__restrict__ r,
-               GS gs, Dims4 d, BoxDecoder bx, uint32_t nint, OFConsts c, CGState *st) {
-  pdl_wait();
-  pdl_launch_dependents();
-  // st is read-only here: the update wrote it, the next matvec clears xpend
-  const bool xp = st->xpend != 0, run = st->done == 0;
-  const float a = st->alphaf, b = st->betaf;
-  if (xp && run)
-    direction_cells<true, true>(x, p, r, gs, d, bx, nint, c, a, b);
-  else if (xp)
-    direction_cells<true, false>(x, p, r, gs, d, bx, nint, c, a, b);
-  else if (run)
-    direction_cells<false, true>(x, p, r, gs, d, bx, nint, c, a, b);
-}
-
-template <class GS>
-void direction_launch(float4 *x, float4 *p, const float4 *r, GS gs, Dims4 d, OFConsts c,
-                      CGState *st, cudaStream_t s, const CGTune &tu) {
-  static const int occ = resident_per_sm(k_cg_direction<GS>, 1 << 30);
+void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState *st,
+                     cudaStream_t s) {
   const long long n = interior_count(d);
-  launch_pdl(k_cg_direction<GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
-             NT, s, x, p, r, gs, d, interior_decoder(d), (uint32_t)n, c, st);
-}
-void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const float4 *g, Dims4 d,
-                         OFConsts c, CGState *st, cudaStream_t s, const CGTune &tu,
-                         const float *i1) {
-  if (i1)
-    direction_launch(x, p, r, GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, d, c, st, s, tu);
-  else
-    direction_launch(x, p, r, GradStored<float4>{g}, d, c, st, s, tu);
-}
-void launch_cg_direction(float4 *x, float4 *p, const float4 *r, const BF4 *g, Dims4 d,
-                         OFConsts c, CGState *st, cudaStream_t s, const CGTune &tu) {
-  direction_launch(x, p, r, GradStored<BF4>{g}, d, c, st, s, tu);
+  launch_pdl(k_cg_flush, grid_for(n > 0 ? n : 1, NT), NT, s, x, ring, count, d,
+             interior_decoder(d), (uint32_t)n, (const CGState *)st);
 }
 
 // vel = x / mDx (optflow4d.cpp:520-529); a NaN residual resets the result to
