@@ -185,6 +185,9 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
 // q = A p, p.q and alpha.
 void launch_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                    double *dpart, cudaStream_t s, const CGTune &tu = CGTune());
+// The same with the reference's operations in its order.
+void launch_strict_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
+                          CGState *st, double *dpart, cudaStream_t s);
 // One iteration of the plain PCG is launch_cg_matvec and launch_cg_step with
 // slot = iteration % CG_RING.  The matvec reads ring.p[slot] and forms alpha and
 // beta; the step updates r, writes the next direction to the ring's next

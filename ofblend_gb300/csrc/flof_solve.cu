@@ -171,20 +171,29 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
 // A thread owns one interior (x,y) column cell at one z and walks MV_TT
 // consecutive t planes, keeping p at t-1, t and t+1 in registers, so the -t
 // and +t terms cost no extra load, and loading the next plane's operands
-// while it computes the current one.  A work item is (run of MV_NT cells of
-// the interior (x,y) plane, z, t chunk) with the (x,y) run fastest, so the
+// while it computes the current one.  A work item is (run of MV_RUN cells of
+// the interior (x,y) plane, MV_ZB planes z, t chunk) with the (x,y) run fastest, so the
 // blocks resident at one time cover neighbouring z at the same t chunk and
 // the z-neighbour loads hit L2.  The grid is persistent (a fixed number of
 // blocks per SM); p.Ap is accumulated per thread in float-float and summed
 // in double by the last block to finish, in a fixed order.
 //
-// DOTS (the plain PCG): the kernel also forms q.M^-1 q, from which its last
+// MV_DOTS (the plain PCG): the kernel also forms q.M^-1 q, from which its last
 // block predicts the next z.r, and so beta, before r is updated (cg_scalars).
 // The step kernel then has alpha and beta and updates r and p in one pass.
-// The extra sum costs 6 us of 148 at 64^4.  The loads need the eight blocks per
+// The extra sum costs 6 us of 148 at 64^4.  The loads need the 1024 threads per
 // SM that 64 registers allow: at 105 registers it takes 186 us; with correctly
-// rounded reciprocals, 195-200.
-constexpr int MV_NT = 128;
+// rounded reciprocals, 195-200.  Two z planes a block share their z neighbours
+// in L1 (148 -> 146 us at 64^4, 59 -> 57 at 48^4; four planes 150 and 61, rows of
+// 256 cells 152 and 59), the fused rows take 146 -> 142 and 57 -> 56 and halve
+// the rounding (the 64^4 deformation against 64 bits 7.5e-7 -> 4.8e-7).
+constexpr int MV_RUN = 128;
+constexpr int MV_ZB = 2;
+constexpr int MV_NT = MV_RUN * MV_ZB;
+// What a matvec computes: the reference's operations in its order and p.q
+// (strict mode, whose rows are applyMat's bit for bit), the same rows with
+// fused operations, or those and q.M^-1 q.
+enum { MV_REFERENCE = 0, MV_FUSED = 1, MV_DOTS = 2 };
 
 // alpha, and beta before the step that it belongs to.  With r' = r - a q,
 //   z'.r' = z.r - 2 a q.z + a^2 q.M^-1 q,
@@ -221,9 +230,9 @@ __device__ __forceinline__ void cg_scalars(CGState *st, double pq, double qmq, i
 struct MVShape {
   FastDiv fx;        // interior x extent
   int nxy;           // interior (x,y) cells
-  int runs;          // ceil(nxy / MV_NT)
-  FastDiv fruns, fz;  // runs, interior z extent
-  int items;         // runs * (Z-2) * tchunks
+  int runs;          // ceil(nxy / MV_RUN)
+  FastDiv fruns, fz;  // runs, groups of MV_ZB interior z planes
+  int items;         // runs * z groups * tchunks
 };
 
 __device__ __forceinline__ void mv_acc(float4 &v, float o, const float4 a) {
@@ -259,8 +268,8 @@ __device__ __forceinline__ float rcp_1ulp(float v) {
 
 // OFFD: the neighbour terms are present (applyMat skips them for a zero
 // off-diagonal, optflow4d.cpp:215).  MV_TT: t planes per work item.
-template <bool OFFD, int MV_TT, bool DOTS, class GT>
-__global__ void __launch_bounds__(MV_NT, 8)
+template <bool OFFD, int MV_TT, int MODE, class GT>
+__global__ void __launch_bounds__(MV_NT, 1024 / MV_NT)
 k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
             float4 *__restrict__ q, Dims4 d, MVShape sh, OFConsts c, CGState *st,
             double *dpart, int slot) {
@@ -276,9 +285,9 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
     const uint32_t r1 = sh.fruns.div((uint32_t)item);
     const int run = item - (int)r1 * sh.runs;
     const uint32_t tc = sh.fz.div(r1);
-    const int k = 1 + (int)(r1 - tc * sh.fz.d);
-    const int n = run * MV_NT + threadIdx.x;
-    if (n >= sh.nxy) continue;
+    const int k = 1 + (int)(r1 - tc * sh.fz.d) * MV_ZB + (int)threadIdx.x / MV_RUN;
+    const int n = run * MV_RUN + (int)threadIdx.x % MV_RUN;
+    if (n >= sh.nxy || k >= d.z - 1) continue;
     const uint32_t jj = sh.fx.div((uint32_t)n);
     const int i = 1 + (n - (int)(jj * sh.fx.d)), j = 1 + (int)jj;
     const int l0 = 1 + (int)tc * MV_TT;
@@ -290,36 +299,58 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
     for (int l = l0; l < l1; ++l, id += sT) {
       // the last plane reloads its own operands instead of reading past l1
       mv_load(nxt, p, g, l + 1 < l1 ? id + sT : id, sY, sZ, sT);
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (OFFD) {
-        mv_acc(v, o, pm);
-        mv_acc(v, o, cur.zm);
-        mv_acc(v, o, cur.ym);
-        mv_acc(v, o, cur.xm);
-        mv_acc(v, o, cur.xp);
-        mv_acc(v, o, cur.yp);
-        mv_acc(v, o, cur.zp);
-        mv_acc(v, o, cur.pp);
-      }
-      const float gv[4] = {cur.gg.x, cur.gg.y, cur.gg.z, cur.gg.w};
-      const float pv[4] = {pc.x, pc.y, pc.z, pc.w};
-      float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int dd = 0; dd < 4; ++dd) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          float b = gv[dd] * gv[m];
-          if (dd == m) b = b + c.diag;
-          vv[dd] += b * pv[m];
+      float4 qq;
+      if (MODE == MV_REFERENCE) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (OFFD) {
+          mv_acc(v, o, pm);
+          mv_acc(v, o, cur.zm);
+          mv_acc(v, o, cur.ym);
+          mv_acc(v, o, cur.xm);
+          mv_acc(v, o, cur.xp);
+          mv_acc(v, o, cur.yp);
+          mv_acc(v, o, cur.zp);
+          mv_acc(v, o, cur.pp);
         }
+        const float gv[4] = {cur.gg.x, cur.gg.y, cur.gg.z, cur.gg.w};
+        const float pv[4] = {pc.x, pc.y, pc.z, pc.w};
+        float vv[4] = {v.x, v.y, v.z, v.w};
+  #pragma unroll
+        for (int dd = 0; dd < 4; ++dd) {
+  #pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            float b = gv[dd] * gv[m];
+            if (dd == m) b = b + c.diag;
+            vv[dd] += b * pv[m];
+          }
+        }
+        qq = make_float4(vv[0], vv[1], vv[2], vv[3]);
+      } else {
+        // row c of g g^T + diag I and the neighbours' sum: 45 operations a cell
+        // in place of 116
+        const float gp = __fmaf_rn(
+            cur.gg.w, pc.w, __fmaf_rn(cur.gg.z, pc.z, __fmaf_rn(cur.gg.y, pc.y, cur.gg.x * pc.x)));
+        auto row = [&](float gc, float p0, float a0, float a1, float a2, float a3, float a4,
+                       float a5, float a6, float a7) {
+          float t = c.diag * p0;
+          if (OFFD) t = __fmaf_rn(o, ((a0 + a1) + (a2 + a3)) + ((a4 + a5) + (a6 + a7)), t);
+          return __fmaf_rn(gp, gc, t);
+        };
+        qq.x = row(cur.gg.x, pc.x, pm.x, cur.zm.x, cur.ym.x, cur.xm.x, cur.xp.x, cur.yp.x,
+                   cur.zp.x, cur.pp.x);
+        qq.y = row(cur.gg.y, pc.y, pm.y, cur.zm.y, cur.ym.y, cur.xm.y, cur.xp.y, cur.yp.y,
+                   cur.zp.y, cur.pp.y);
+        qq.z = row(cur.gg.z, pc.z, pm.z, cur.zm.z, cur.ym.z, cur.xm.z, cur.xp.z, cur.yp.z,
+                   cur.zp.z, cur.pp.z);
+        qq.w = row(cur.gg.w, pc.w, pm.w, cur.zm.w, cur.ym.w, cur.xm.w, cur.xp.w, cur.yp.w,
+                   cur.zp.w, cur.pp.w);
       }
-      const float4 qq = make_float4(vv[0], vv[1], vv[2], vv[3]);
       q[id] = qq;
       ff_add(dot, pc.x * qq.x);
       ff_add(dot, pc.y * qq.y);
       ff_add(dot, pc.z * qq.z);
       ff_add(dot, pc.w * qq.w);
-      if (DOTS) {
+      if (MODE == MV_DOTS) {
         // for beta only, whose own rounding to float is larger than the last
         // bit of these reciprocals
         const float ux = rcp_1ulp(cur.gg.x * cur.gg.x + c.diag) * qq.x;
@@ -334,21 +365,21 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
     }
   }
   const double bd = block_sum_ff<MV_NT>(dot, shff);
-  const double bm = DOTS ? block_sum_ff<MV_NT>(dotm, shff) : 0.0;
+  const double bm = MODE == MV_DOTS ? block_sum_ff<MV_NT>(dotm, shff) : 0.0;
   if (threadIdx.x == 0) {
     dpart[blockIdx.x] = bd;
-    if (DOTS) dpart[gridDim.x + blockIdx.x] = bm;
+    if (MODE == MV_DOTS) dpart[gridDim.x + blockIdx.x] = bm;
   }
   if (last_block_arrives(&st->counter[1])) {
     double s = 0.0, sm = 0.0;
     for (int q2 = threadIdx.x; q2 < (int)gridDim.x; q2 += blockDim.x) {
       s += __ldcg(dpart + q2);
-      if (DOTS) sm += __ldcg(dpart + gridDim.x + q2);
+      if (MODE == MV_DOTS) sm += __ldcg(dpart + gridDim.x + q2);
     }
     s = block_sum<MV_NT>(s, shd);
-    if (DOTS) sm = block_sum<MV_NT>(sm, shd);
+    if (MODE == MV_DOTS) sm = block_sum<MV_NT>(sm, shd);
     if (threadIdx.x == 0) {
-      if (DOTS) {
+      if (MODE == MV_DOTS) {
         cg_scalars(st, s, sm, slot);
       } else {
         st->pAp = s;
@@ -362,7 +393,7 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
 
 namespace {
 
-template <bool OFFD, int TT, bool DOTS, class GT>
+template <bool OFFD, int TT, int MODE, class GT>
 void matvec_variant(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c,
                     CGState *st, double *dpart, cudaStream_t s, int slot) {
   MVShape sh;
@@ -372,55 +403,60 @@ void matvec_variant(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c
   const bool empty = d.x < 3 || d.y < 3 || d.z < 3 || d.t < 3;
   sh.fx = FastDiv((uint32_t)ex);
   sh.nxy = empty ? 0 : ex * ey;
-  sh.runs = (ex * ey + MV_NT - 1) / MV_NT;
+  const int zb = (ez + MV_ZB - 1) / MV_ZB;
+  sh.runs = (ex * ey + MV_RUN - 1) / MV_RUN;
   sh.fruns = FastDiv((uint32_t)sh.runs);
-  sh.fz = FastDiv((uint32_t)ez);
-  sh.items = empty ? 0 : sh.runs * ez * tchunks;
+  sh.fz = FastDiv((uint32_t)zb);
+  sh.items = empty ? 0 : sh.runs * zb * tchunks;
   // resident blocks per SM of this instantiation (computed once, thread-safe)
   static const int per_sm = [] {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_cg_matvec<OFFD, TT, DOTS, GT>, MV_NT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_cg_matvec<OFFD, TT, MODE, GT>, MV_NT, 0);
     return n < 1 ? 1 : n;
   }();
   int blocks = sm_count() * per_sm;
   if (blocks > sh.items) blocks = sh.items > 0 ? sh.items : 1;
-  launch_pdl(k_cg_matvec<OFFD, TT, DOTS, GT>, blocks, MV_NT, s, p, g, q, d, sh, c, st, dpart,
+  launch_pdl(k_cg_matvec<OFFD, TT, MODE, GT>, blocks, MV_NT, s, p, g, q, d, sh, c, st, dpart,
              slot);
 }
 
-template <bool OFFD, bool DOTS, class GT>
+template <bool OFFD, int MODE, class GT>
 void matvec_tt(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                double *dpart, cudaStream_t s, int tt, int slot) {
   if (tt <= 4)
-    matvec_variant<OFFD, 4, DOTS>(p, g, q, d, c, st, dpart, s, slot);
+    matvec_variant<OFFD, 4, MODE>(p, g, q, d, c, st, dpart, s, slot);
   else if (tt >= 16)
-    matvec_variant<OFFD, 16, DOTS>(p, g, q, d, c, st, dpart, s, slot);
+    matvec_variant<OFFD, 16, MODE>(p, g, q, d, c, st, dpart, s, slot);
   else
-    matvec_variant<OFFD, 8, DOTS>(p, g, q, d, c, st, dpart, s, slot);
+    matvec_variant<OFFD, 8, MODE>(p, g, q, d, c, st, dpart, s, slot);
 }
 
-template <bool DOTS, class GT>
+template <int MODE, class GT>
 void matvec_any(const float4 *p, const GT *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                 double *dpart, cudaStream_t s, const CGTune &tu, int slot) {
   if (c.offd != 0.f)
-    matvec_tt<true, DOTS>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
+    matvec_tt<true, MODE>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
   else
-    matvec_tt<false, DOTS>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
+    matvec_tt<false, MODE>(p, g, q, d, c, st, dpart, s, tu.mv_tt, slot);
 }
 
 }  // namespace
 
 void launch_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                    double *dpart, cudaStream_t s, const CGTune &tu) {
-  matvec_any<false>(p, g, q, d, c, st, dpart, s, tu, 0);
+  matvec_any<MV_FUSED>(p, g, q, d, c, st, dpart, s, tu, 0);
+}
+void launch_strict_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
+                          CGState *st, double *dpart, cudaStream_t s) {
+  matvec_any<MV_REFERENCE>(p, g, q, d, c, st, dpart, s, CGTune(), 0);
 }
 void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
                       CGState *st, double *dpart, int slot, cudaStream_t s, const CGTune &tu) {
-  matvec_any<true>(p, g, q, d, c, st, dpart, s, tu, slot);
+  matvec_any<MV_DOTS>(p, g, q, d, c, st, dpart, s, tu, slot);
 }
 void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                       double *dpart, int slot, cudaStream_t s, const CGTune &tu) {
-  matvec_any<true>(p, g, q, d, c, st, dpart, s, tu, slot);
+  matvec_any<MV_DOTS>(p, g, q, d, c, st, dpart, s, tu, slot);
 }
 
 // Where the step kernel takes the image gradient g for the Jacobi
@@ -443,8 +479,8 @@ struct GradStored {
 // CG_RING reads the earlier ones again and x once: (32 + 16 (CG_RING - 1)) /
 // CG_RING bytes a step, 20 for four buffers.  The ring's alpha p are added to
 // one another before they are added to x, so x is rounded once in four steps
-// (64^4 deformation against 64 bits: 7.5e-7 relative, 7.9e-7 when every step
-// adds to x).
+// (with the reference's row operations the 64^4 deformation against 64 bits
+// is 7.5e-7 off, 7.9e-7 when every step adds to x).
 // An iteration (matvec and step) moves 152 bytes a cell; three kernels (matvec,
 // r, then x and p) moved 184.  Step at 64^4: 247 us (6.2 TB/s) with four
 // buffers, 259 with two, 270 with one; r and then x and p took 130 + 190 us.

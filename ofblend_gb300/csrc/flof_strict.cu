@@ -271,9 +271,9 @@ void launch_strict_iteration(float4 *x, float4 *r, float4 *p, float4 *q, const f
                              cudaStream_t s) {
   const long long nint = interior_cells(d);
   const BoxDecoder bx = interior_box(d);
-  // q = A p: the fast matvec's rows are the reference's applyMat bit for bit;
+  // q = A p: this matvec's rows are the reference's applyMat bit for bit;
   // its parallel p.q and alpha are replaced by the serial ones below
-  launch_matvec(p, g, q, d, c, st, dpart, s);
+  launch_strict_matvec(p, g, q, d, c, st, dpart, s);
   k_serial_sum<<<1, SER_NT, 0, s>>>(DotTerm{(const float *)p, (const float *)q, d, bx}, 4 * nint,
                                     FinAlpha{st});
   const int nb = grid_for(nint > 0 ? nint : 1, ST_NT, 4);
