@@ -485,6 +485,10 @@ struct GradStored {
 // r, then x and p) moved 184.  Step at 64^4: 247 us (6.2 TB/s) with four
 // buffers, 259 with two, 270 with one; r and then x and p took 130 + 190 us.
 // Iteration: 64^4 463 -> 395 us, 48^4 166 -> 140, 40 x 42 x 38 x 48 107 -> 93.
+// The step walks from the last cell to the first: it begins where the matvec
+// ended and ends where the next one begins, on q, p and r that L2 still holds
+// (64^4 389 -> 386 us an iteration, 48^4 138 -> 135, 40 x 42 x 38 x 48 92 -> 89).
+// Keeping x, g or q out of L2 (ld.cs) was slower: 10-20% of the kernel.
 // pin and pout may be one buffer (CG_RING = 1); a cell is read before it is
 // written, by the same thread.
 __device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
@@ -550,14 +554,14 @@ k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restri
     ff_add(dot, z.w * rr.w);
     mx = fmaxf(mx, fmaxf(fmaxf(rr.x, rr.y), fmaxf(rr.z, rr.w)));
   };
-  // two cells per trip with all loads issued first
+  // two cells per trip with all loads issued first, from the last cell down
   const uint32_t stride = gridDim.x * blockDim.x;
   uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   for (; n + stride < nint; n += 2 * stride) {
     int i, j, k, l;
-    bx.decode(n, i, j, k, l);
+    bx.decode(nint - 1 - n, i, j, k, l);
     const idx_t i0 = d.index(i, j, k, l);
-    bx.decode(n + stride, i, j, k, l);
+    bx.decode(nint - 1 - n - stride, i, j, k, l);
     const idx_t i1 = d.index(i, j, k, l);
     const In v0 = load(i0), v1 = load(i1);
     cell(i0, v0);
@@ -565,7 +569,7 @@ k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restri
   }
   if (n < nint) {
     int i, j, k, l;
-    bx.decode(n, i, j, k, l);
+    bx.decode(nint - 1 - n, i, j, k, l);
     const idx_t i0 = d.index(i, j, k, l);
     cell(i0, load(i0));
   }
