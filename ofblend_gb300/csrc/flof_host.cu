@@ -278,6 +278,7 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
   DBuf p(c, vb), g(c, vb), q(c, vb), x(c, vb), r(c, vb), stb(c, sizeof(CGState));
   DBuf p2(c, vb);
   CGRing ring;
+  ring.n = CG_RING;
   for (int m = 0; m < CG_RING; ++m) ring.p[m] = m % 2 ? p2.v() : p.v();
   CK(cudaMemsetAsync(p.p, 0, vb, c->stream));
   CK(cudaMemsetAsync(g.p, 0, vb, c->stream));
@@ -343,6 +344,25 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
 // waiting; every kernel returns at once when the state says done.  After each
 // chunk the host reads the state (into c->st_h) and sizes the next chunk from
 // the observed reduction rate.
+// The ring of search directions: p and CG_RING - 1 more grids, or p alone where
+// those do not fit, so that a level that fits with one p still runs.
+void make_ring(flof_ctx *c, Dims4 d, float4 *p, CGRing &ring, DBuf *more) {
+  ring.p[0] = p;
+  ring.n = CG_RING;
+  try {
+    for (int m = 1; m < CG_RING; ++m) more[m] = DBuf(c, vec_bytes(d));
+  } catch (const FlofError &e) {
+    if (e.code != FLOF_E_OOM) throw;
+    for (int m = 1; m < CG_RING; ++m) more[m].release();
+    ring.n = 1;
+  }
+  for (int m = 1; m < CG_RING; ++m) {
+    ring.p[m] = ring.n > 1 ? more[m].v() : p;
+    if (ring.n > 1)  // the border rows
+      CK(cudaMemsetAsync(ring.p[m], 0, vec_bytes(d), c->stream));
+  }
+}
+
 // i1: the FP32 solve's target level set; the step kernel rebuilds the
 // preconditioner's gradient from it (null: it reads g).
 template <class GT>
@@ -373,22 +393,17 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
     }
   }
   CGRing ring;
-  ring.p[0] = p;
   DBuf more[CG_RING];
-  for (int m = 1; m < CG_RING; ++m) {
-    more[m] = DBuf(c, vec_bytes(d));
-    ring.p[m] = more[m].v();
-    CK(cudaMemsetAsync(ring.p[m], 0, vec_bytes(d), c->stream));  // the border rows
-  }
+  make_ring(c, d, p, ring, more);
   int it = 0;
   int chunk = 4;
   for (;;) {
     const int n = (maxIter - it) < chunk ? (maxIter - it) : chunk;
     for (int s = 0; s < n; ++s) {
-      const int slot = (it + s) % CG_RING;
+      const int slot = (it + s) % ring.n;
       KLP(c, KC_MATVEC, d.x, nint(d) * (32 + gb),
           launch_cg_matvec(ring.p[slot], g, q, d, k, c->st, c->dpart, slot, c->stream, tu));
-      KLP(c, KC_STEP, d.x, nint(d) * (80 + gpc + (slot == CG_RING - 1 ? 16 * (CG_RING + 1) : 0)),
+      KLP(c, KC_STEP, d.x, nint(d) * (80 + gpc + (slot == ring.n - 1 ? 16 * (ring.n + 1) : 0)),
           launch_cg_step(x, r, q, ring, slot, g, i1, d, k, c->st, c->dpart, c->fpart, maxIter,
                          c->stream, tu));
     }
@@ -408,7 +423,7 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
       chunk = chunk * 2 > 64 ? 64 : chunk * 2;
     }
   }
-  const int left = c->st_h->iters % CG_RING;  // directions not yet added to x
+  const int left = c->st_h->iters % ring.n;  // directions not yet added to x
   if (left > 0)
     KLP(c, KC_STEP, d.x, nint(d) * (32 + 16 * left),
         launch_cg_flush(x, ring, left, d, c->st, c->stream));

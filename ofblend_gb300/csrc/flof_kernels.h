@@ -134,6 +134,7 @@ void launch_lookup_slice_twoway(float *dst, int dx, int dy, int dz,
 constexpr int CG_RING = 4;
 struct CGRing {
   float4 *p[CG_RING];
+  int n;  // CG_RING, or 1: p[0] only
 };
 
 struct CGState {
@@ -169,7 +170,7 @@ struct OFConsts {
 
 // Launch shapes of the PCG kernels, chosen per grid size by the autotuner
 // (defaults otherwise): t planes per matvec work item (4, 8 or 16) and
-// resident blocks per SM of the update / direction kernels.
+// resident blocks per SM of the step kernel.
 struct CGTune {
   int mv_tt = 8;
   int per_sm = 8;
@@ -189,7 +190,7 @@ void launch_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConst
 void launch_strict_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFConsts c,
                           CGState *st, double *dpart, cudaStream_t s);
 // One iteration of the plain PCG is launch_cg_matvec and launch_cg_step with
-// slot = iteration % CG_RING.  The matvec reads ring.p[slot] and forms alpha and
+// slot = iteration % ring.n.  The matvec reads ring.p[slot] and forms alpha and
 // beta; the step updates r, writes the next direction to the ring's next
 // buffer, and in the last slot adds the ring's directions to x.  launch_cg_flush
 // adds what is left when the solve ends in another slot.

@@ -489,8 +489,9 @@ struct GradStored {
 // ended and ends where the next one begins, on q, p and r that L2 still holds
 // (64^4 389 -> 386 us an iteration, 48^4 138 -> 135, 40 x 42 x 38 x 48 92 -> 89).
 // Keeping x, g or q out of L2 (ld.cs) was slower: 10-20% of the kernel.
-// pin and pout may be one buffer (CG_RING = 1); a cell is read before it is
-// written, by the same thread.
+// NX: the directions that this step adds to x.  Where memory for a ring is
+// short there is one buffer, pin = pout, and every step adds its own (NX = 1);
+// a cell is read before it is written, by the same thread.
 __device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
   x.x = __fmaf_rn(a, p.x, x.x);
   x.y = __fmaf_rn(a, p.y, x.y);
@@ -498,7 +499,7 @@ __device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
   x.w = __fmaf_rn(a, p.w, x.w);
 }
 
-template <bool XP, class GS>
+template <int NX, class GS>
 __global__ void __launch_bounds__(NT)
 k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restrict__ q,
           CGRing ring, const float4 *pin, float4 *pout, GS gs, Dims4 d, BoxDecoder bx,
@@ -510,23 +511,23 @@ k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restri
   __shared__ FF shff[NT / 32];
   __shared__ float shf[NT / 32];
   const float a = st->alphaf, b = st->betaf;
-  float al[CG_RING];
+  float al[NX > 1 ? NX : 1];
 #pragma unroll
-  for (int m = 0; m < CG_RING; ++m) al[m] = st->al[m];
+  for (int m = 0; m + 1 < NX; ++m) al[m] = st->al[m];
   FF dot = {0.f, 0.f};
   float mx = -FLT_MAX;
   struct In {
-    float4 q, g, r, p, x, po[CG_RING];
+    float4 q, g, r, p, x, po[NX > 1 ? NX - 1 : 1];
   };
   auto load = [&](idx_t id) {
     In v;
     v.q = __ldg(q + id);
     v.r = r[id];
     v.p = pin[id];
-    if (XP) {
+    if (NX > 0) {
       v.x = x[id];
 #pragma unroll
-      for (int m = 0; m + 1 < CG_RING; ++m) v.po[m] = ring.p[m][id];
+      for (int m = 0; m + 1 < NX; ++m) v.po[m] = ring.p[m][id];
     }
     v.g = gs(id);
     return v;
@@ -537,10 +538,10 @@ k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restri
     r[id] = rr;
     const float4 pre = precond_of(v.g, c.diag);
     const float4 z = make_float4(rr.x * pre.x, rr.y * pre.y, rr.z * pre.z, rr.w * pre.w);
-    if (XP) {
+    if (NX > 0) {
       float4 t = make_float4(a * pp.x, a * pp.y, a * pp.z, a * pp.w);
 #pragma unroll
-      for (int m = CG_RING - 2; m >= 0; --m) axpy4(t, al[m], v.po[m]);
+      for (int m = NX - 2; m >= 0; --m) axpy4(t, al[m], v.po[m]);
       x[id] = make_float4(v.x.x + t.x, v.x.y + t.y, v.x.z + t.z, v.x.w + t.w);
     }
     pp.x = __fmaf_rn(b, pp.x, z.x);
@@ -639,24 +640,26 @@ int resident_per_sm(K kernel, int want) {
   return want < n ? want : n;
 }
 
-template <bool XP, class GS>
+template <int NX, class GS>
 void step_launch(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs,
                  Dims4 d, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter,
                  cudaStream_t s, const CGTune &tu) {
-  static const int occ = resident_per_sm(k_cg_step<XP, GS>, 1 << 30);
+  static const int occ = resident_per_sm(k_cg_step<NX, GS>, 1 << 30);
   const long long n = interior_count(d);
-  launch_pdl(k_cg_step<XP, GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
-             NT, s, x, r, q, ring, (const float4 *)ring.p[slot], ring.p[XP ? 0 : slot + 1], gs, d,
+  launch_pdl(k_cg_step<NX, GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
+             NT, s, x, r, q, ring, (const float4 *)ring.p[slot], ring.p[NX > 0 ? 0 : slot + 1], gs, d,
              interior_decoder(d), (uint32_t)n, c, st, dpart, fpart, maxIter);
 }
 template <class GS>
 void step_any(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs, Dims4 d,
               OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
               const CGTune &tu) {
-  if (slot == CG_RING - 1)
-    step_launch<true>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+  if (ring.n == 1)
+    step_launch<1>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+  else if (slot == CG_RING - 1)
+    step_launch<CG_RING>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
   else
-    step_launch<false>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_launch<0>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
 }
 void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
                     const float4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st,

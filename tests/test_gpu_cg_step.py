@@ -61,3 +61,38 @@ def test_steps_match_64_bits(dims, smooth):
         # q, r, p and x are each rounded at some 20 places an iteration, and an
         # iteration carries the errors of those before it: 3 x 20 x n roundings
         assert np.linalg.norm(got - want) <= 60 * n * 2.0 ** -24 * np.linalg.norm(want)
+
+
+def test_one_direction_buffer_when_memory_is_short():
+    """Where the ring's extra buffers do not fit, the solve keeps one direction
+    and adds it to x in every step."""
+    import torch
+
+    import ofblend_gb300 as F
+
+    dims = (43, 45, 41, 42)
+    X, Y, Z, T = dims
+    grid = X * Y * Z * T * 16
+    rng = np.random.default_rng(7)
+    i0 = (rng.standard_normal((T, Z, Y, X)) * 0.01).astype(np.float32)
+    i1 = np.roll(i0, 1, axis=3) + np.float32(0.001)
+    want = cg64(i0, i1, 0.001, 0.0001, 5)
+    torch.cuda.empty_cache()
+    launches = []
+    for short in (False, True):
+        ctx = F.Context(0)
+        g0, g1 = (F.Grid4Real(dims=dims, ctx=ctx).from_numpy(v) for v in (i0, i1))
+        v = F.Grid4Vec4(dims=dims, ctx=ctx)
+        v.clear()
+        ctx.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        # g, r, p, q and x fit, and one or two of the three extra buffers
+        fill = torch.empty(max(0, free - 7 * grid) if short else 1, dtype=torch.uint8, device="cuda")
+        n0 = ctx.kernel_launches()
+        F.opticalFlow4d(v, g0, g1, wSmooth=0.001, wEnergy=0.0001, cgAccuracy=1e-12, cgMaxIter=5)
+        launches.append(ctx.kernel_launches() - n0)
+        del fill
+        torch.cuda.empty_cache()
+        got = v.to_numpy().astype(np.float64)
+        assert np.linalg.norm(got - want) <= 60 * 5 * 2.0 ** -24 * np.linalg.norm(want)
+    assert launches[1] == launches[0] - 1  # five steps leave one direction in the ring to add, none here
