@@ -276,10 +276,9 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
   if (it != owner->tunes.end()) return it->second;
   const size_t vb = vec_bytes(d);
   DBuf p(c, vb), g(c, vb), q(c, vb), x(c, vb), r(c, vb), stb(c, sizeof(CGState));
-  DBuf p2(c, vb);
   CGRing ring;
   ring.n = CG_RING;
-  for (int m = 0; m < CG_RING; ++m) ring.p[m] = m % 2 ? p2.v() : p.v();
+  for (int m = 0; m < CG_RING; ++m) ring.p[m] = p.v();  // one grid stands for all four
   CK(cudaMemsetAsync(p.p, 0, vb, c->stream));
   CK(cudaMemsetAsync(g.p, 0, vb, c->stream));
   CK(cudaMemsetAsync(x.p, 0, vb, c->stream));
