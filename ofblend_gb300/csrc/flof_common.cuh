@@ -97,6 +97,7 @@ struct AxisW {
   float w0, w1;
 };
 
+// n is at least 2: the corner at b + 1 is read whatever its weight.
 // A position below 0 is clamped before the index is taken, which gives b = 0
 // and the weights (1, 0) without three selects; NaN stays NaN (max.NaN).
 __device__ __forceinline__ AxisW axis_index(float p, int n) {

@@ -794,8 +794,11 @@ float multiscale(flof_ctx *c, Dims4 d, float4 *vel, const float *i0, const float
 
   DBuf i0warped(c, real_bytes(d));
 
-  if (d.x > p.minGridSize) {
-    Dims4 sd{d.x / 2, d.y / 2, d.z / 2, d.t / 2};
+  if (d.x > p.minGridSize && d.x > 1) {
+    // a short axis stays at one cell (the reference's halving would leave a
+    // grid without cells)
+    auto half = [](int n) { return n > 1 ? n / 2 : 1; };
+    Dims4 sd{half(d.x), half(d.y), half(d.z), half(d.t)};
     DBuf velSm(c, vec_bytes(sd)), i0Sm(c, real_bytes(sd)), i1Sm(c, real_bytes(sd));
     interpol_grid(c, i0Sm.f(), sd, i0, d, 1);
     interpol_grid(c, i1Sm.f(), sd, i1, d, 1);

@@ -202,8 +202,9 @@ __global__ void k_set_bound_neumann(float *a, Dims4 d, BoxDecoder bx, int nc, in
     if (l >= d.t - 1 - w) { sl = d.t - 1 - w - 1; set = true; }
     if (!set) continue;
     // Source cells lie strictly inside the written ring, so the in-place
-    // update does not depend on the visiting order.
-    const idx_t src = d.index(si, sj, sk, sl);
+    // update does not depend on the visiting order.  An axis of one cell (a
+    // coarse level of a short grid) has none: its cell stays.
+    const idx_t src = d.index(max(si, 0), max(sj, 0), max(sk, 0), max(sl, 0));
     if (nc == 4) ((float4 *)a)[q] = ((const float4 *)a)[src];
     else a[q] = a[src];
   }
@@ -511,10 +512,51 @@ k_resample_one(float *__restrict__ target, Dims4 td, BoxDecoder bx, uint32_t n,
     target[q] = mul != 1.f ? v * mul : v;
   }
 }
+// A source with an axis of one cell, as the coarse levels of a short grid have
+// (24^3 x 3 halves to 12^3 x 1).  Such an axis has no second corner: every
+// position takes its cell with weight 1, and the stride 0 keeps the corner
+// of weight 0 inside the grid (the kernels above would read a plane before it).
+struct ThinAxis {
+  AxisW w;
+  idx_t step;
+};
+__device__ __forceinline__ ThinAxis thin_axis(float p, int n, idx_t stride) {
+  if (n < 2) return ThinAxis{AxisW{0, 1.f, 0.f}, 0};
+  return ThinAxis{axis_index(p, n), stride};
+}
+__global__ void __launch_bounds__(NT)
+k_resample_thin(float *__restrict__ target, Dims4 td, BoxDecoder bx, uint32_t n,
+                const float *__restrict__ source, Dims4 sd, int nc, float4 fac, float4 off,
+                float mul) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  int i, j, k, l;
+  bx.decode(q, i, j, k, l);
+  const ThinAxis x = thin_axis((float)i * fac.x + off.x, sd.x, nc);
+  const ThinAxis y = thin_axis((float)j * fac.y + off.y, sd.y, (idx_t)sd.x * nc);
+  const ThinAxis z = thin_axis((float)k * fac.z + off.z, sd.z, sd.sz() * nc);
+  const ThinAxis t = thin_axis((float)l * fac.w + off.w, sd.t, sd.st() * nc);
+  const float *base = source + sd.index(x.w.b, y.w.b, z.w.b, t.w.b) * nc;
+  for (int c = 0; c < nc; ++c) {
+    float plane[2];
+    for (int m = 0; m < 2; ++m) {
+      const float *p = base + c + m * t.step, *py = p + y.step, *pz = p + z.step, *pyz = py + z.step;
+      plane[m] = plane_sum(__ldg(p), __ldg(py), __ldg(p + x.step), __ldg(py + x.step), __ldg(pz),
+                           __ldg(pyz), __ldg(pz + x.step), __ldg(pyz + x.step), x.w, y.w, z.w);
+    }
+    const float v = plane[0] * t.w.w0 + plane[1] * t.w.w1;
+    target[(size_t)q * nc + c] = mul != 1.f ? v * mul : v;
+  }
+}
 void launch_resample(float *target, Dims4 td, const float *source, Dims4 sd,
                      int nc, float4 fac, float4 off, cudaStream_t s, float mul) {
   if (td.cells() <= 0) return;
   BoxDecoder bx = make_decoder(td.x, td.y, td.z, 0, 0, 0, 0);
+  if (sd.x < 2 || sd.y < 2 || sd.z < 2 || sd.t < 2) {
+    const uint32_t n = (uint32_t)td.cells();
+    k_resample_thin<<<grid_all(n), NT, 0, s>>>(target, td, bx, n, source, sd, nc, fac, off, mul);
+    return;
+  }
   const int tt = planes_per_thread(td.cells(), RS_TT);
   // a thread with one plane has nothing to keep, and targets two source planes
   // apart (restriction by two) share none
