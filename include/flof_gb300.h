@@ -175,8 +175,15 @@ FLOF_API const char *flof_kernel_class_name(int cls);
  * FLOF_OPT_SLAB_TMA: 1 (default) the Vec4 Gaussian blur and the extrapolation
  *   sweeps of corrVelsOf4d use the TMA slab kernels; 0 their plain-load
  *   counterparts, which take the same sums in the same order (equal results;
- *   for checking one against the other). */
-enum { FLOF_OPT_CFL_SYNC = 2, FLOF_OPT_AUTOTUNE = 3, FLOF_OPT_STRICT = 4, FLOF_OPT_SLAB_TMA = 5 };
+ *   for checking one against the other).
+ * FLOF_OPT_RESIDENT_POLLS: the PCG of a small level is one launch whose blocks
+ *   wait for one another; when other work on the device keeps one of them from
+ *   starting for this many looks (about half a microsecond each; default
+ *   2^22, some two seconds), the level goes to the chained kernels, which
+ *   wait for nothing but their own stream.  0: it goes there at once.  The two
+ *   agree to rounding. */
+enum { FLOF_OPT_CFL_SYNC = 2, FLOF_OPT_AUTOTUNE = 3, FLOF_OPT_STRICT = 4, FLOF_OPT_SLAB_TMA = 5,
+       FLOF_OPT_RESIDENT_POLLS = 6 };
 FLOF_API int flof_ctx_set_option(flof_ctx *ctx, int option, int value);
 /* Parameters of the multigrid V-cycle of FLOF_SOLVER_MG (no reference
  * counterpart): damping of the block-Jacobi sweeps on the system's own grid

@@ -30,6 +30,7 @@ flof_ctx *worker(flof_ctx *c, size_t q) {
     w->autotune = c->autotune;
     w->strict = c->strict;
     w->slab_tma = c->slab_tma;
+    w->resident_polls = c->resident_polls;
     w->mg = c->mg;
     w->tune_owner = c;
     c->workers.push_back(w);

@@ -375,10 +375,11 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
     ResidentShare share;
     bool done = false;
     KLP(c, KC_RESIDENT, d.x, nint(d) * 64,
-        done = launch_cg_resident(x, r, p, q, g, d, k, c->st, c->dpart, maxIter, c->dev_err,
-                                  next_post(c), c->beside, share, c->stream));
-    if (done) {
-      wait_post(c, &c->hres->cg_seq);
+        done = launch_cg_resident(x, r, p, q, g, d, k, c->st, c->dpart, maxIter,
+                                  c->resident_polls, c->dev_err, next_post(c), c->beside, share,
+                                  c->stream));
+    if (done) wait_post(c, &c->hres->cg_seq);
+    if (done && c->hres->done != CG_LEFT) {
       c->st_h->done = c->hres->done;
       c->st_h->iters = c->hres->iters;
       c->st_h->resMax = c->hres->resMax;
@@ -1135,6 +1136,10 @@ FLOF_API int flof_ctx_set_option(flof_ctx *c, int option, int value) {
       need(value == 0 || value == 1, "FLOF_OPT_SLAB_TMA takes 0 or 1");
       c->slab_tma = value;
       for (flof_ctx *w : c->workers) w->slab_tma = value;
+    } else if (option == FLOF_OPT_RESIDENT_POLLS) {
+      need(value >= 0, "FLOF_OPT_RESIDENT_POLLS must not be negative");
+      c->resident_polls = value;
+      for (flof_ctx *w : c->workers) w->resident_polls = value;
     } else if (option == FLOF_OPT_AUTOTUNE) {
       need(value == 0 || value == 1, "FLOF_OPT_AUTOTUNE takes 0 or 1");
       c->autotune = value;

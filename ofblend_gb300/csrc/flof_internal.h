@@ -163,6 +163,9 @@ struct flof_ctx {
   // FLOF_OPT_SLAB_TMA: 1 the TMA slab kernels for the Vec4 blur and the
   // extrapolation sweeps, 0 their plain-load counterparts
   int slab_tma = 1;
+  // FLOF_OPT_RESIDENT_POLLS: how long the resident PCG's blocks wait for all of
+  // them to start (looks of about half a microsecond)
+  int resident_polls = 1 << 22;
   // parameters of the multigrid preconditioner (FLOF_SOLVER_MG) and the
   // number of its solves the plain PCG had to finish
   flof::MGParams mg;

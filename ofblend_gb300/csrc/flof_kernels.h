@@ -154,9 +154,11 @@ struct CGState {
   int iters;
   unsigned int counter[4];
   unsigned int gbar;  // arrivals at the resident solve's grid barriers
+  int gate;           // its gate: 0 until all blocks have come or one has shut it
 };
+// CG_LEFT: the resident solve's blocks did not all start; the state is as it was
 enum { CG_RUNNING = 0, CG_CONVERGED = 1, CG_FAILED_SIGMA = 2, CG_EARLY = 3,
-       CG_MAXITER = 4 };
+       CG_MAXITER = 4, CG_LEFT = 5 };
 
 struct OFConsts {
   float dxf;        // 1 / (2 mDx)
@@ -212,14 +214,16 @@ void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState 
 // ---- resident PCG (flof_resident.cu) -------------------------------------------
 // The whole iteration of a level whose cells fit the SMs as one cooperative
 // launch, from the state that the assembly or launch_cg_init_r left; it ends
-// with st->done set and the outcome posted to the host.  r is read only at the start and q is scratch.  False
-// (nothing launched) for a larger level, maxIter <= 0, or when the device
-// refuses the launch: the caller then chains the kernels above.  Its blocks
-// wait on one another, so those of all launches in flight are counted and the
-// call waits for room; `share` gives its part back when it goes out of scope,
-// after the stream has been waited for.  shared: other solves run beside this
-// one (the same result, on a quarter of the SMs where the level is small).
-// part holds at least 7 doubles per SM.
+// with st->done set and the outcome posted to the host.  r is read only at the
+// start and q is scratch.  False (nothing launched) for a larger level, maxIter
+// <= 0, or when the device refuses the launch: the caller then chains the
+// kernels above.  So it does when CG_LEFT is posted: a block had not started
+// after `polls` looks (about half a microsecond each), and x, r, p and *st are
+// as they were.  Its blocks wait on one another, so those of all launches in
+// flight are counted and the call waits for room; `share` gives its part back
+// when it goes out of scope, after the outcome has been waited for.  shared:
+// other solves run beside this one (the same result, on a quarter of the SMs
+// where the level is small).  part holds at least 7 doubles per SM.
 constexpr size_t RESIDENT_SMEM = 220 * 1024;  // shared memory for its cells, per SM
 bool resident_cells_ok(Dims4 d);
 struct ResidentShare {
@@ -232,10 +236,10 @@ struct ResidentShare {
   void give();
 };
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
-                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        OFConsts c, CGState *st, double *part, int maxIter, int polls, int *err,
                         HostPost post, bool shared, ResidentShare &share, cudaStream_t s);
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
-                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        OFConsts c, CGState *st, double *part, int maxIter, int polls, int *err,
                         HostPost post, bool shared, ResidentShare &share, cudaStream_t s);
 // ---- strict arithmetic (flof_strict.cu, FLOF_OPT_STRICT) ----------------------
 // The reference's PCG arithmetic operation for operation: double alpha and

@@ -167,6 +167,7 @@ k_cg_init_r(const float4 *__restrict__ r, const GT *__restrict__ g, float4 *__re
       st->resMax = m;
       st->iters = 0;
       st->gbar = 0;
+      st->gate = 0;
       st->counter[0] = 0;
       if (residual < (double)1e-6f) {
         st->retResidual = 0.f;

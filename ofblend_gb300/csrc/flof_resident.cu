@@ -27,10 +27,14 @@
 //   24^3 x 16    149k        22.6 / 9.2 us
 //
 // The blocks wait on one another, so the launch is cooperative and the blocks
-// of all launches in flight are counted (resident_share): they never exceed
-// the SMs, so all of them can be resident whatever else runs, as ordinary
-// kernels end by themselves.  Every wait is bounded; a block that gives up
-// records FLOF_DEV_ERR_GRID_TIMEOUT and returns, and the others after it.
+// of all launches in flight are counted (ResidentShare): they never exceed
+// the SMs.  Other work on the device can still keep a block from starting for
+// as long as it runs (a caller's long kernel on another stream).  So the first
+// meeting of the blocks is a gate (grid_gate): either all of them are there
+// within its wait and go on, or they leave the level as they found it, for the
+// chained kernels.  Past the gate every block is resident; the barriers' waits
+// are bounded all the same, and a block that gives up there records
+// FLOF_DEV_ERR_GRID_TIMEOUT and returns, and the others after it.
 //
 // The sums are formed per work group of `per` cells and then over the groups
 // in order, and a block holds M groups, so the result does not depend on M:
@@ -80,6 +84,43 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *counter, unsigned int
   return *ok_sh != 0;
 }
 
+// The first meeting: true when every block has come.  The last one to come
+// opens the gate; a block whose wait ends first shuts it.  Whichever happens
+// first holds for all blocks, those that start later among them.  The block
+// that shuts it tells the host.  limit: polls to wait; 0 shuts it at once.
+enum { GATE_UNDECIDED = 0, GATE_OPEN = 1, GATE_SHUT = 2 };
+__device__ __forceinline__ bool grid_gate(CGState *st, int limit, const HostPost &post,
+                                          int *ok_sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    bool shut = limit <= 0 && atomicCAS(&st->gate, GATE_UNDECIDED, GATE_SHUT) == GATE_UNDECIDED;
+    __threadfence();
+    if (atomicAdd(&st->gbar, 1u) + 1u == gridDim.x) {
+      __threadfence();
+      atomicCAS(&st->gate, GATE_UNDECIDED, GATE_OPEN);
+    }
+    int g = GATE_UNDECIDED;
+    for (int n = 0; n < limit && g == GATE_UNDECIDED; ++n)
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(g) : "l"(&st->gate) : "memory");
+    if (g == GATE_UNDECIDED) {
+      g = atomicCAS(&st->gate, GATE_UNDECIDED, GATE_SHUT);
+      if (g == GATE_UNDECIDED) {
+        g = GATE_SHUT;
+        shut = true;
+      }
+      __threadfence();
+    }
+    if (shut) {
+      post.hr->done = CG_LEFT;
+      __threadfence_system();
+      *(volatile unsigned int *)&post.hr->cg_seq = post.seq;
+    }
+    *ok_sh = g == GATE_OPEN;
+  }
+  __syncthreads();
+  return *ok_sh != 0;
+}
+
 // (float)(a / b) without the FP64 division (a chain of some twenty dependent
 // FP64 operations on a part with few FP64 lanes): the float quotient plus one
 // correction from its exact remainder.
@@ -113,7 +154,8 @@ template <int NTH, int M, int K, bool QREG, bool GS, class GT>
 __global__ void __launch_bounds__(NTH, 1)
 k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
               const GT *__restrict__ g, Dims4 d, BoxDecoder bx, uint32_t nint, uint32_t per,
-              int GV, OFConsts c, CGState *st, double *part, int maxIter, int *err, HostPost post) {
+              int GV, OFConsts c, CGState *st, double *part, int maxIter, int polls, int *err,
+              HostPost post) {
   extern __shared__ float4 res_sm[];
   __shared__ FF shff[3][NTH / 32];
   __shared__ float shm[NTH / 32];
@@ -221,7 +263,9 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
       }
     }
     target += gridDim.x;
-    if (!grid_barrier(&st->gbar, target, &ok)) {
+    if (it == 0) {  // nothing but q and part has been written
+      if (!grid_gate(st, polls, post, &ok)) return;
+    } else if (!grid_barrier(&st->gbar, target, &ok)) {
       if (threadIdx.x == 0) *(volatile int *)err = FLOF_DEV_ERR_GRID_TIMEOUT;
       return;
     }
@@ -344,7 +388,7 @@ struct ResidentArgs {
   OFConsts c;
   CGState *st;
   double *part;
-  int maxIter;
+  int maxIter, polls;
   int *err;
   HostPost post;
   cudaStream_t s;
@@ -402,7 +446,7 @@ bool launch_one(ResidentArgs a, const GT *g, ResidentShare &share) {
   int groups = (int)((a.n + a.per - 1) / a.per);
   const int grid = (groups + M - 1) / M;
   void *args[] = {&a.x, &r0,  &a.p, &a.q,  &g,    &a.d,       &bx,    &a.n,   &a.per,
-                  &groups, &a.c, &a.st, &a.part, &a.maxIter, &a.err, &a.post};
+                  &groups, &a.c, &a.st, &a.part, &a.maxIter, &a.polls, &a.err, &a.post};
   share.take(grid);
   if (cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(NTH), args, smem, a.s) !=
       cudaSuccess) {
@@ -454,15 +498,15 @@ void ResidentShare::give() {
 }
 
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *g, Dims4 d,
-                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        OFConsts c, CGState *st, double *part, int maxIter, int polls, int *err,
                         HostPost post, bool shared, ResidentShare &share, cudaStream_t s) {
-  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, err, post, s}, g,
+  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, polls, err, post, s}, g,
                     shared, share);
 }
 bool launch_cg_resident(float4 *x, float4 *r, float4 *p, float4 *q, const BF4 *g, Dims4 d,
-                        OFConsts c, CGState *st, double *part, int maxIter, int *err,
+                        OFConsts c, CGState *st, double *part, int maxIter, int polls, int *err,
                         HostPost post, bool shared, ResidentShare &share, cudaStream_t s) {
-  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, err, post, s}, g,
+  return launch_any(ResidentArgs{x, r, p, q, d, 0, 0, c, st, part, maxIter, polls, err, post, s}, g,
                     shared, share);
 }
 

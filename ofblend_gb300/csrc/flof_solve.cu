@@ -130,6 +130,7 @@ k_of_assemble_init(const float *__restrict__ i0w, const float *__restrict__ i1,
       st->resMax = m;
       st->iters = 0;
       st->gbar = 0;
+      st->gate = 0;
       st->counter[0] = 0;
       if (residual < (double)1e-6f) {
         st->retResidual = 0.f;
