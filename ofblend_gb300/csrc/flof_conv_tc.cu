@@ -1161,13 +1161,11 @@ int tc_smem(int N) {
   return 2 * (2 * A_TILE + (MODE == 2 ? 2 : 1) * N * TB_K * 2) + 1024;
 }
 
-// once per kernel: room for the largest stage pair (N = 128, two B tiles)
+// room for the largest stage pair (N = 128, two B tiles)
 template <int MODE, int VEC>
 void tc_attr() {
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_conv_tc<MODE, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           tc_smem<2>(128));
-  fh::cuda_check(attr, "cudaFuncSetAttribute(k_conv_tc)");
+  fh::cuda_check(allow_smem<k_conv_tc<MODE, VEC>>(tc_smem<2>(128)),
+                 "cudaFuncSetAttribute(k_conv_tc)");
 }
 
 // resident blocks per SM for N columns (N a multiple of 16 up to 128),
@@ -1254,10 +1252,7 @@ void launch_halo(const HaloArgs &a0, const HaloPlan &pl, cudaStream_t s) {
   a.nx = (a.R + 7) / 8;
   a.nr = (a.R * (a.R + 2) + 15) / 16;
   a.cslice = pl.cslice;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_dgrad_halo, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           226 * 1024);
-  fh::cuda_check(attr, "cudaFuncSetAttribute(k_dgrad_halo)");
+  fh::cuda_check(allow_smem<k_dgrad_halo>(226 * 1024), "cudaFuncSetAttribute(k_dgrad_halo)");
   launch_pdl_smem(k_dgrad_halo, dim3(pl.tiles, 1, pl.nz), TB_W, (size_t)pl.smem, s, a);
   fh::cuda_check(cudaGetLastError(), "k_dgrad_halo launch");
 }
@@ -1292,9 +1287,7 @@ WgradPlan wgrad_halo_plan(int R, int cin, int cout) {
 }
 
 void launch_wgrad_halo(const WgradArgs &a, const WgradPlan &pl, cudaStream_t s) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_wgrad_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, wg_smem(64));
-  fh::cuda_check(attr, "cudaFuncSetAttribute(k_wgrad_halo)");
+  fh::cuda_check(allow_smem<k_wgrad_halo>(wg_smem(64)), "cudaFuncSetAttribute(k_wgrad_halo)");
   launch_pdl_smem(k_wgrad_halo, dim3(pl.blocks(), 1, pl.nz), TB_W, (size_t)wg_smem(a.cc), s, a);
   fh::cuda_check(cudaGetLastError(), "k_wgrad_halo launch");
 }

@@ -9,14 +9,30 @@
 #include <vector>
 
 #include "flof_common.cuh"
+#include "flof_device.h"
 
 namespace flof {
 
 // Sets the thread-local message returned by flof_last_error().
 void set_last_error(const char *msg);
 
-// Number of SMs of the current device (cached), used to size grids.
+// Number of SMs of the current device (asked for once: the devices are alike),
+// used to size grids.
 int sm_count();
+int current_device();
+// Lets the kernel K use `bytes` of dynamic shared memory, asked for once per
+// device (the attribute belongs to the device that is current).
+template <auto K>
+inline cudaError_t allow_smem(size_t bytes) {
+  static PerDevice<cudaError_t> asked;
+  return asked.get(current_device(), [&] {
+    const cudaError_t e =
+        cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+  });
+}
+
 // Blocks for a grid-stride launch over n items with `nt` threads per block.
 int grid_for(long long n, int nt, int per_sm = 8);
 
@@ -220,13 +236,14 @@ void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState 
 // kernels above.  So it does when CG_LEFT is posted: a block had not started
 // after `polls` looks (about half a microsecond each), and x, r, p and *st are
 // as they were.  Its blocks wait on one another, so those of all launches in
-// flight are counted and the call waits for room; `share` gives its part back
+// flight on the device are counted and the call waits for room; `share` gives its part back
 // when it goes out of scope, after the outcome has been waited for.  shared:
 // other solves run beside this one (the same result, on a quarter of the SMs
 // where the level is small).  part holds at least 7 doubles per SM.
 constexpr size_t RESIDENT_SMEM = 220 * 1024;  // shared memory for its cells, per SM
 bool resident_cells_ok(Dims4 d);
 struct ResidentShare {
+  SmShares *shares = nullptr;  // the current device's
   int blocks = 0;
   ResidentShare() {}
   ResidentShare(const ResidentShare &) = delete;

@@ -22,6 +22,12 @@ int sm_count() {
   return n;
 }
 
+int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+
 int grid_for(long long n, int nt, int per_sm) {
   long long b = (n + nt - 1) / nt;
   long long cap = (long long)sm_count() * per_sm;

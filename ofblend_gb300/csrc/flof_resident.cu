@@ -40,9 +40,6 @@
 // in order, and a block holds M groups, so the result does not depend on M:
 // one solve alone spreads its groups over the SMs (M = 1), the solves of a
 // batch take a quarter of the SMs each (M = 4) and run side by side.
-#include <condition_variable>
-#include <mutex>
-
 #include "flof_kernels.h"
 
 namespace flof {
@@ -394,41 +391,14 @@ struct ResidentArgs {
   cudaStream_t s;
 };
 
-// The blocks of all launches in flight, at most one per SM in sum; waits in
-// the order of arrival.
-struct SmShares {
-  std::mutex mu;
-  std::condition_variable cv;
-  int used = 0;
-  unsigned long long next = 0, serving = 0;
-  void acquire(int n) {
-    std::unique_lock<std::mutex> lk(mu);
-    const unsigned long long mine = next++;
-    cv.wait(lk, [&] { return serving == mine && used + n <= sm_count(); });
-    ++serving;
-    used += n;
-    cv.notify_all();
-  }
-  void release(int n) {
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      used -= n;
-    }
-    cv.notify_all();
-  }
-};
-SmShares &sm_shares() {
-  static SmShares s;
-  return s;
-}
-
 template <int NTH, int M, int K, bool QREG, bool GS, class GT>
 bool launch_one(ResidentArgs a, const GT *g, ResidentShare &share) {
   auto k = k_cg_resident<NTH, M, K, QREG, GS, GT>;
   constexpr size_t per_cell = GS ? 32 : 16;
-  // the shared memory that the kernel may use, asked for once (thread-safe
-  // static init); 0 when the device refuses it
-  static const size_t smem_max = [&]() -> size_t {
+  // the shared memory that the kernel may use, asked for once per device; 0
+  // when the device refuses it
+  static PerDevice<size_t> asked;
+  const size_t smem_max = asked.get(current_device(), [&]() -> size_t {
     int n = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RESIDENT_SMEM) !=
             cudaSuccess ||
@@ -438,7 +408,7 @@ bool launch_one(ResidentArgs a, const GT *g, ResidentShare &share) {
       return 0;
     }
     return RESIDENT_SMEM;
-  }();
+  });
   const size_t smem = per_cell * a.per * M;
   if (smem > smem_max) return false;
   BoxDecoder bx = make_decoder(a.d.x - 2, a.d.y - 2, a.d.z - 2, 1, 1, 1, 1);
@@ -489,11 +459,12 @@ bool resident_cells_ok(Dims4 d) {
 }
 
 void ResidentShare::take(int n) {
-  sm_shares().acquire(n);
+  shares = &sm_shares(current_device());
+  shares->acquire(n, sm_count());
   blocks = n;
 }
 void ResidentShare::give() {
-  if (blocks) sm_shares().release(blocks);
+  if (blocks) shares->release(blocks);
   blocks = 0;
 }
 

@@ -701,15 +701,9 @@ bool launch_blur_shape(const float4 *src, float4 *dst, Dims4 d, const float *wsu
   const int tiles_x = (box.hi[0] - box.lo[0] + LW - 1) / LW, h = b.nw * UNIT + 2 * S;
   CUtensorMap map;
   if (!encode_slab_map(&map, src, d, W, h)) return false;
-  static const bool attr = [] {
-    if (cudaFuncSetAttribute(k_blur_tma<S, LW, RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             BW_NS * blur_stride(W, BW_MAXW * UNIT + 2 * S)) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return true;
-  }();
-  if (!attr) return false;
+  if (allow_smem<k_blur_tma<S, LW, RY>>(BW_NS * blur_stride(W, BW_MAXW * UNIT + 2 * S)) !=
+      cudaSuccess)
+    return false;
   const dim3 grid(tiles_x * b.ny, box.hi[2] - box.lo[2], box.hi[3] - box.lo[3]);
   k_blur_tma<S, LW, RY><<<grid, 32 * b.nw, BW_NS * blur_stride(W, h), st>>>(
       map, dst, d, tiles_x, wsum, wt, 0x8000000080000000ull, zero_border, box, err);
@@ -833,15 +827,7 @@ bool launch_expol_tw(const float4 *in, float4 *out, const uint16_t *mask, const 
   if (grid.y > 65535 || grid.z > 65535) return false;
   CUtensorMap map;
   if (!encode_slab_map(&map, in, d, ETW_W, ETW_H, ETW_SPC)) return false;
-  static const bool attr = [] {
-    if (cudaFuncSetAttribute(k_expol_tw, cudaFuncAttributeMaxDynamicSharedMemorySize, ETW_SMEM) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return true;
-  }();
-  if (!attr) return false;
+  if (allow_smem<k_expol_tw>(ETW_SMEM) != cudaSuccess) return false;
   k_expol_tw<<<grid, 32 * ETW_NW, ETW_SMEM, st>>>(map, out, d, (d.x + TX - 1) / TX, mask, dist,
                                                   sweep, err);
   return true;
@@ -853,15 +839,7 @@ bool launch_expol_sep_tw(const float4 *in, float4 *out, const uint16_t *mask, co
   if (grid.y > 65535 || grid.z > 65535) return false;
   CUtensorMap map;
   if (!encode_slab_map(&map, in, d, ETW_W, ETW_H, ESW_SPC)) return false;
-  static const bool attr = [] {
-    if (cudaFuncSetAttribute(k_expol_sep_tw, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             ESW_SMEM) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return true;
-  }();
-  if (!attr) return false;
+  if (allow_smem<k_expol_sep_tw>(ESW_SMEM) != cudaSuccess) return false;
   k_expol_sep_tw<<<grid, 32 * ESW_NW, ESW_SMEM, st>>>(map, out, d, (d.x + TX - 1) / TX, mask,
                                                       dist, sweep, err);
   return true;
