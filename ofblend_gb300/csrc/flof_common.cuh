@@ -366,6 +366,19 @@ inline void launch_pdl(void (*k)(KArgs...), unsigned grid, unsigned block, cudaS
   launch_pdl_smem(k, dim3(grid), block, 0, s, args...);
 }
 
+// 1 / v for the sums that give beta: the hardware's approximation (off by up to
+// a bit, the same way in every cell of equal v) and one Newton step
+// r + r (1 - v r), which squares its error and leaves the rounding of the
+// result.  Where 1 - v r is no small number (v is 0, infinite or subnormal) the
+// approximation stands.  At 64^4 the matvec takes 143.8 us with it, 142.3 with
+// the approximation alone and 176 with __frcp_rn.
+__device__ __forceinline__ float rcp_newton(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  const float e = __fmaf_rn(-v, r, 1.0f);
+  return fabsf(e) < 0.5f ? __fmaf_rn(r, e, r) : r;
+}
+
 // ---- reductions -----------------------------------------------------------
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -172,6 +172,8 @@ struct CGState {
   unsigned int gbar;  // arrivals at the resident solve's grid barriers
   int gate;           // its gate: 0 until all blocks have come or one has shut it
 };
+// The predicted beta at and below which it is rounding only (flof_solve.cu).
+constexpr double CG_BETA_FLOOR = 1.0 / (1 << 26);
 // CG_LEFT: the resident solve's blocks did not all start; the state is as it was
 enum { CG_RUNNING = 0, CG_CONVERGED = 1, CG_FAILED_SIGMA = 2, CG_EARLY = 3,
        CG_MAXITER = 4, CG_LEFT = 5 };

@@ -217,14 +217,21 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
       qq.y = row(gg.y, pc.y, tm.y, zm.y, ym.y, xm.y, xp.y, yp.y, zp.y, tp.y);
       qq.z = row(gg.z, pc.z, tm.z, zm.z, ym.z, xm.z, xp.z, yp.z, zp.z, tp.z);
       qq.w = row(gg.w, pc.w, tm.w, zm.w, ym.w, xm.w, xp.w, yp.w, zp.w, tp.w);
-      const float4 pre = res_precond(gg, c.diag);
+      const float4 pre = make_float4(rcp_newton(gg.x * gg.x + c.diag), rcp_newton(gg.y * gg.y + c.diag),
+                                     rcp_newton(gg.z * gg.z + c.diag), rcp_newton(gg.w * gg.w + c.diag));
       ff_add(d0, pc.x * qq.x);
       ff_add(d0, pc.y * qq.y);
       ff_add(d0, pc.z * qq.z);
       ff_add(d0, pc.w * qq.w);
       const float ux = pre.x * qq.x, uy = pre.y * qq.y, uz = pre.z * qq.z, uw = pre.w * qq.w;
-      ff_add(d1, (ux * r.x + uy * r.y) + (uz * r.z + uw * r.w));
-      ff_add(d2, (ux * qq.x + uy * qq.y) + (uz * qq.z + uw * qq.w));
+      ff_add(d1, ux * r.x);
+      ff_add(d1, uy * r.y);
+      ff_add(d1, uz * r.z);
+      ff_add(d1, uw * r.w);
+      ff_add(d2, ux * qq.x);
+      ff_add(d2, uy * qq.y);
+      ff_add(d2, uz * qq.z);
+      ff_add(d2, uw * qq.w);
       return qq;
     };
 #pragma unroll
@@ -295,7 +302,8 @@ k_cg_resident(float4 *x, const float4 *__restrict__ r0, float4 *p, float4 *qg,
         const float af = quotient(sg, fin[0]);
         const double a = (double)af;
         ab[0] = af;
-        ab[1] = quotient(fma(a * a, fin[2], fma(-2.0 * a, fin[1], sg)), sg);
+        const double zr = fma(a * a, fin[2], fma(-2.0 * a, fin[1], sg));
+        ab[1] = zr < CG_BETA_FLOOR * sg ? 0.f : quotient(zr, sg);
       }
     }
     __syncthreads();

@@ -183,11 +183,13 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
 // block predicts the next z.r, and so beta, before r is updated (cg_scalars).
 // The step kernel then has alpha and beta and updates r and p in one pass.
 // The extra sum costs 6 us of 148 at 64^4.  The loads need the 1024 threads per
-// SM that 64 registers allow: at 105 registers it takes 186 us; with correctly
-// rounded reciprocals, 195-200.  Two z planes a block share their z neighbours
+// SM that 64 registers allow: at 105 registers it takes 186 us.  Two z planes a block share their z neighbours
 // in L1 (148 -> 146 us at 64^4, 59 -> 57 at 48^4; four planes 150 and 61, rows of
 // 256 cells 152 and 59), the fused rows take 146 -> 142 and 57 -> 56 and halve
-// the rounding (the 64^4 deformation against 64 bits 7.5e-7 -> 4.8e-7).
+// the rounding (the 64^4 deformation against 64 bits 7.5e-7 -> 4.8e-7).  Each
+// product of q.M^-1 q enters the float-float sum by itself, like those of every
+// other dot product, with a reciprocal that has no common error (rcp_newton):
+// 142 -> 144 us.
 constexpr int MV_RUN = 128;
 constexpr int MV_ZB = 2;
 constexpr int MV_NT = MV_RUN * MV_ZB;
@@ -207,6 +209,12 @@ enum { MV_REFERENCE = 0, MV_FUSED = 1, MV_DOTS = 2 };
 //   z.q_old = (z.r_old - z.r) / a_old,  z.r_old = z_old.r = z_old.r_old - a_old q_old.z_old.
 // So no error passes from one beta to the next but the rounding of the vectors.
 // alpha itself uses the fresh sigma.
+// The terms are of the size of z.r, whatever is left of it, so beta's error is
+// that of the sums: 2^-24 (1 + beta) over the root of their number of products
+// (1e-9 measured from 0.01M cells on), below beta's own rounding to float
+// unless a single step takes more than nine tenths of z.r away.  A beta below
+// CG_BETA_FLOOR is noise, which the next one's q.p_old would carry on: the
+// iteration starts anew from p = z.
 __device__ __forceinline__ void cg_scalars(CGState *st, double pq, double qmq, int slot) {
   const double sg = st->sigma;
   st->pAp = pq;
@@ -220,7 +228,8 @@ __device__ __forceinline__ void cg_scalars(CGState *st, double pq, double qmq, i
     const double zro = st->sgOld - ao * st->qzOld;
     qz -= bo * ((zro - sg) / ao + bo * st->pqOld);
   }
-  st->beta = fma(a * a, qmq, fma(-2.0 * a, qz, sg)) / sg;
+  const double b = fma(a * a, qmq, fma(-2.0 * a, qz, sg)) / sg;
+  st->beta = b < CG_BETA_FLOOR ? 0.0 : b;  // a NaN stays
   st->betaf = (float)st->beta;
   st->aOld = a;
   st->sgOld = sg;
@@ -259,12 +268,6 @@ __device__ __forceinline__ void mv_load(MVLoads &a, const float4 *__restrict__ p
   a.xp = __ldg(p + id + 1);
   a.yp = __ldg(p + id + sY);
   a.zp = __ldg(p + id + sZ);
-}
-
-__device__ __forceinline__ float rcp_1ulp(float v) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
 }
 
 // OFFD: the neighbour terms are present (applyMat skips them for a zero
@@ -352,13 +355,10 @@ k_cg_matvec(const float4 *__restrict__ p, const GT *__restrict__ g,
       ff_add(dot, pc.z * qq.z);
       ff_add(dot, pc.w * qq.w);
       if (MODE == MV_DOTS) {
-        // for beta only, whose own rounding to float is larger than the last
-        // bit of these reciprocals
-        const float ux = rcp_1ulp(cur.gg.x * cur.gg.x + c.diag) * qq.x;
-        const float uy = rcp_1ulp(cur.gg.y * cur.gg.y + c.diag) * qq.y;
-        const float uz = rcp_1ulp(cur.gg.z * cur.gg.z + c.diag) * qq.z;
-        const float uw = rcp_1ulp(cur.gg.w * cur.gg.w + c.diag) * qq.w;
-        ff_add(dotm, (ux * qq.x + uy * qq.y) + (uz * qq.z + uw * qq.w));
+        ff_add(dotm, (rcp_newton(cur.gg.x * cur.gg.x + c.diag) * qq.x) * qq.x);
+        ff_add(dotm, (rcp_newton(cur.gg.y * cur.gg.y + c.diag) * qq.y) * qq.y);
+        ff_add(dotm, (rcp_newton(cur.gg.z * cur.gg.z + c.diag) * qq.z) * qq.z);
+        ff_add(dotm, (rcp_newton(cur.gg.w * cur.gg.w + c.diag) * qq.w) * qq.w);
       }
       pm = pc;
       pc = cur.pp;
