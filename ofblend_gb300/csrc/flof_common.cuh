@@ -379,6 +379,25 @@ __device__ __forceinline__ float rcp_newton(float v) {
   return fabsf(e) < 0.5f ? __fmaf_rn(r, e, r) : r;
 }
 
+// a / b in float without the FP64 division (a long chain of dependent FP64
+// operations on a part with few FP64 lanes): the float quotient q, off by some
+// 2^-22, corrected by its remainder a - q b (Markstein, IBM J. Res. Dev. 34,
+// 1990, on divisions with fused multiply-adds).  The remainder is formed in
+// FP64 and the correction's own error is some 2^-45 of the result, so this is
+// the nearest float of a / b unless a / b lies within 2^-43 of the middle of two.
+// Operands or results outside 1e-30 .. 1e30 take the division.
+__device__ __forceinline__ float quotient(double a, double b) {
+  const float af = (float)a, bf = (float)b;
+  const float aa = fabsf(af), ab = fabsf(bf);
+  if (aa > 1e-30f && aa < 1e30f && ab > 1e-30f && ab < 1e30f) {
+    const float rc = __frcp_rn(bf);
+    const float q = af * rc;
+    if (fabsf(q) > 1e-30f && fabsf(q) < 1e30f)
+      return __fmaf_rn((float)fma(-(double)q, b, a), rc, q);
+  }
+  return (float)(a / b);
+}
+
 // ---- reductions -----------------------------------------------------------
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -118,21 +118,6 @@ __device__ __forceinline__ bool grid_gate(CGState *st, int limit, const HostPost
   return *ok_sh != 0;
 }
 
-// (float)(a / b) without the FP64 division (a chain of some twenty dependent
-// FP64 operations on a part with few FP64 lanes): the float quotient plus one
-// correction from its exact remainder.
-__device__ __forceinline__ float quotient(double a, double b) {
-  const float af = (float)a, bf = (float)b;
-  const float aa = fabsf(af), ab = fabsf(bf);
-  if (aa > 1e-30f && aa < 1e30f && ab > 1e-30f && ab < 1e30f) {
-    const float rc = __frcp_rn(bf);
-    const float q = af * rc;
-    if (fabsf(q) > 1e-30f && fabsf(q) < 1e30f)
-      return __fmaf_rn((float)fma(-(double)q, b, a), rc, q);
-  }
-  return (float)(a / b);
-}
-
 __device__ __forceinline__ void post_outcome(const HostPost &post, const CGState *st) {
   HostResult *h = post.hr;
   h->done = st->done;
