@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(TB_W, 3) k_conv_tc(TcArgs p) {
     const int last = issued - 1;
     if (!mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) ok = false;
   }
-  if (!ok) atomicExch(p.err, FLOF_DEV_ERR_TC_TIMEOUT);
+  if (!ok) *(volatile int *)p.err = FLOF_DEV_ERR_TC_TIMEOUT;
   ok = __syncthreads_and(ok);
   // a slice past this block's reduction (a parity class with fewer taps)
   // contributes zeros
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(TB_W, 2) k_dgrad_halo(HaloArgs p) {
     const int last = issued - 1;
     if (!mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) ok = false;
   }
-  if (!ok) atomicExch(p.err, FLOF_DEV_ERR_TC_TIMEOUT);
+  if (!ok) *(volatile int *)p.err = FLOF_DEV_ERR_TC_TIMEOUT;
   ok = __syncthreads_and(ok);
   // a slice whose chunks all fall off the grid contributes zeros
   const bool empty = ok && issued == 0;
@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(TB_W, 1) k_wgrad_halo(WgradArgs p) {
     const int last = issued - 1;
     if (!mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1)) ok = false;
   }
-  if (!ok) atomicExch(p.err, FLOF_DEV_ERR_TC_TIMEOUT);
+  if (!ok) *(volatile int *)p.err = FLOF_DEV_ERR_TC_TIMEOUT;
   ok = __syncthreads_and(ok);
   // a slice without a tile: zeros
   if (ok && producer) drain(issued <= p.drain, issued == 0);
