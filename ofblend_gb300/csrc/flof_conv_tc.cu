@@ -768,10 +768,10 @@ __global__ void __launch_bounds__(TB_W, 2) k_dgrad_halo(HaloArgs p) {
 // registers the kernel spilled and took 80 us).  The bias gradient is summed
 // in FP32 by the threads that stage dout, in the middle taps' block.
 // Bound by the latency of a tile's loads (the 288 columns leave room for one
-// block per SM): 48 -> 16 channels at 16^4 78 us (im2col 192; with the tap's
+// block per SM): 48 -> 16 channels at 16^4 67 us (im2col 193; with the tap's
 // shift on the input's side, one MMA of 32 columns per tap from a misaligned
-// start, 120), 96 -> 32 at 8^4 23 (43), 64 -> 64 at 4^4 9 (11), 32 -> 32 at 8^4
-// 14 (12).
+// start, 120), 96 -> 32 at 8^4 25 (43), 64 -> 64 at 4^4 12 (12), 32 -> 32 at 8^4
+// 14 (20).
 struct WgradArgs {
   const float *in, *dout;
   float *out;             // slices: 2 per blockIdx.z, of 81 cin + 1 rows of cout
@@ -1261,9 +1261,6 @@ void launch_halo(const HaloArgs &a0, const HaloPlan &pl, cudaStream_t s) {
 // channels, tiles per slice.  A block takes about 4 us of set-up and stores and
 // 1.2 us per tile, the sum of the slices 8 bytes per entry of a slice pair at 4
 // TB/s; the count with the lowest estimate wins.
-bool wgrad_halo_ok(int cin, int cout, int stride) {
-  return stride == 1 && cin % 16 == 0 && cout % 16 == 0;
-}
 struct WgradPlan {
   int nz, per, tiles, ncc, nco;
   int blocks() const { return 9 * ncc * nco; }
@@ -1284,6 +1281,31 @@ WgradPlan wgrad_halo_plan(int R, int cin, int cout) {
     if (us < best) best = us, pl.nz = z, pl.per = per;
   }
   return pl;
+}
+
+// Halo tiles or im2col, by what each is expected to take.  Fitted to both over
+// the four stride-1 layers' channels at extents 1 to 48 (halo against im2col, us,
+// a layer at a time):
+//   48 -> 16  8^4 13 / 19   16^4 67 / 193   48^4 4779 / 15127
+//   32 -> 32  2^4 7.0 / 5.4  8^4 14 / 20    18^4 290 / 266    24^4 661 / 909
+//   64 -> 64  3^4 10 / 8.4   8^4 28 / 37     9^4 72 / 46      12^4 147 / 141
+// Tiles are 8 wide and a plane is padded, so a tile is mostly empty at an extent
+// of 1 to 3 and half empty at 9; im2col packs its rows.  Where the
+// estimates choose the slower form they lose up to 1.4 us (64 -> 64 at 5^4).
+bool wgrad_halo_ok(int R, int cin, int cout, int stride) {
+  if (stride != 1 || cin % 16 != 0 || cout % 16 != 0) return false;
+  const WgradPlan pl = wgrad_halo_plan(R, cin, cout);
+  const int waves = (pl.blocks() * pl.nz + sm_count() - 1) / sm_count();
+  // a tile's loads, and the sums taken out every WG_DRAIN tiles
+  const double tile = cin / pl.ncc < 64 ? 1.6 : 1.9;
+  const double halo = 6.5 + waves * (tile * pl.per + 5.0 * ((pl.per - 1) / WG_DRAIN));
+  const long long M = 81LL * cin + 1, K = (long long)R * R * R * R;
+  const TcPlan tc = tc_plan_for<2, 0>(M, K, cout);
+  // a chunk takes longer as blocks share an SM's loads
+  const double share = (double)((M + TB_M - 1) / TB_M * tc.nz) / sm_count();
+  const double chunk = (1.25 + 0.009 * cout) * std::max(1.0, 0.8 * share);
+  const double sum = tc.nz > 1 ? 1.5 + (double)tc.nz * M * cout / 1.1e6 : 0.0;
+  return halo <= 4.0 + chunk * (tc.kslice / TB_K) + sum;
 }
 
 void launch_wgrad_halo(const WgradArgs &a, const WgradPlan &pl, cudaStream_t s) {
@@ -1318,7 +1340,7 @@ size_t net_tc_work(int rin, int rout, int cin, int cout, bool first) {
                                        : tc_plan_for<1, 1>(Vi, 81LL * cout, cin).nz;
     if (nz > 1) w = std::max(w, (size_t)nz * (size_t)Vi * cin);
   }
-  const int nw = wgrad_halo_ok(cin, cout, same ? 1 : 2)
+  const int nw = wgrad_halo_ok(rin, cin, cout, same ? 1 : 2)
                      ? 2 * wgrad_halo_plan(rin, cin, cout).nz
                      : tc_plan_for<2, 0>(81LL * cin + 1, Vo, cout).nz;
   return std::max(w, (size_t)nw * (81 * cin + 1) * cout);
@@ -1416,7 +1438,7 @@ void net_tc_conv_bwd_data(const float *dout, const uint16_t *wb, float *din, flo
 void net_tc_conv_bwd_weight(const float *in, const float *dout, float *grad, float *work, int rin,
                             int rout, int cin, int cout, int stride, int acc, int *err,
                             cudaStream_t s) {
-  if (wgrad_halo_ok(cin, cout, stride)) {
+  if (wgrad_halo_ok(rin, cin, cout, stride)) {
     const WgradPlan pl = wgrad_halo_plan(rin, cin, cout);
     WgradArgs a{};
     a.in = in;
