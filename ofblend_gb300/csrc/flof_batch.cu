@@ -1,14 +1,15 @@
 // flof_batch.cu -- many independent deformation solves of uneven grid sizes
-// on one GPU.  A solve at 24^3 x 16 cells launches kernels of a few
-// microseconds, far too small to fill 152 SMs, and spends much of its time
-// in host round trips (CG convergence checks, multistep decisions).  The
-// batch runs the solves concurrently: each worker context owns a CUDA stream,
-// a buffer pool and the PCG state, and one host thread drives it through the
-// same multiscale driver as the single call, so kernels of different solves
-// overlap on the GPU and one solve's host round trip hides behind another's
-// kernels.  Solves are handed out largest first from a shared counter, and
-// a budget of cells in flight keeps large solves, which fill the GPU alone,
-// from running side by side.
+// on one GPU.  A 24^3 x 16 solve is some seventy launches that fill a part of
+// the SMs, with a host round trip behind each of its PCGs and error metrics.
+// The batch runs the solves concurrently: each worker context owns a CUDA
+// stream, a buffer pool and the PCG state, and one host thread drives it
+// through the same multiscale driver as the single call, so kernels of
+// different solves overlap on the GPU and one solve's host round trip hides
+// behind another's kernels.  The small levels' resident PCGs run on a quarter of
+// the SMs each, four side by side; those above 1024 cells per SM take all SMs in
+// turn.  Solves are handed out largest first from a shared counter, and a
+// budget of cells in flight keeps large solves, which fill the GPU alone, from
+// running side by side.
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
@@ -38,11 +39,14 @@ flof_ctx *worker(flof_ctx *c, size_t q) {
   return c->workers[q];
 }
 
-// Cells of the solves in flight at once.  A solve of a few million cells
-// keeps the PCG kernels near the HBM roofline on its own (on GB300: 3.5M-cell
-// solves gain nothing from a second stream, 1M-cell solves 1.4x from several,
-// 0.2M-cell solves 2.8x from sixteen), so a larger solve runs alone and
-// smaller ones share the budget.
+// Cells of the solves in flight at once, so that a larger solve runs alone and
+// smaller ones share the budget.  Solves a second on GB300 (cgAccuracy 0.01, no
+// projection) with 1, 4 and 16 workers, and as chosen here:
+//   24^3 x 16, 48 pairs   802  1701  2310   2310
+//   30^3 x 24, 32         558   838   868    885
+//   36^3 x 32, 16         380   435   432    437
+//   40^4, 12              160   145   144    160
+//   48^3 x 32, 8          146   133   132    146
 constexpr long long kCellsInFlight = 4ll << 20;
 
 // Worker count when the caller leaves it open: enough streams that the

@@ -259,9 +259,6 @@ struct OFArgs {
   int solver = FLOF_SOLVER_PCG;
 };
 
-// opticalFlowDim<Grid4d<Real>,Grid4d<Vec4>,4> (optflow4d.cpp:361-553).
-// velIn (nullable) is the input velocity used in the rhs; the result goes
-// to velOut (may alias velIn).
 // PCG launch shapes for grid size d: the defaults, or (FLOF_OPT_AUTOTUNE)
 // the fastest of a few candidates timed once per size on scratch buffers.
 // The candidates give the same per-cell arithmetic; the grouping of the dot
@@ -338,11 +335,6 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
   return best;
 }
 
-// PCG iterations (GridCGOptflow4d::solve, optflow4d.cpp:304-326) from the
-// state the initialisation left.  Iterations are launched in chunks without
-// waiting; every kernel returns at once when the state says done.  After each
-// chunk the host reads the state (into c->st_h) and sizes the next chunk from
-// the observed reduction rate.
 // The ring of search directions: p and CG_RING - 1 more grids, or p alone where
 // those do not fit, so that a level that fits with one p still runs.
 void make_ring(flof_ctx *c, Dims4 d, float4 *p, CGRing &ring, DBuf *more) {
@@ -362,6 +354,11 @@ void make_ring(flof_ctx *c, Dims4 d, float4 *p, CGRing &ring, DBuf *more) {
   }
 }
 
+// PCG iterations (GridCGOptflow4d::solve, optflow4d.cpp:304-326) from the
+// state the initialisation left.  Iterations are launched in chunks without
+// waiting; every kernel returns at once when the state says done.  After each
+// chunk the host reads the state (into c->st_h) and sizes the next chunk from
+// the observed reduction rate.  A small level is one launch instead.
 // i1: the FP32 solve's target level set; the step kernel rebuilds the
 // preconditioner's gradient from it (null: it reads g).
 template <class GT>
@@ -619,6 +616,9 @@ void mixed_solve(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, cons
   if (resOut) *resOut = res;
 }
 
+// opticalFlowDim<Grid4d<Real>,Grid4d<Vec4>,4> (optflow4d.cpp:361-553).
+// velIn (nullable) is the input velocity used in the rhs; the result goes
+// to velOut (may alias velIn).
 void optical_flow_dim(flof_ctx *c, Dims4 d, float4 *velOut, const float4 *velIn,
                       const float *i0w, const float *i1, const OFArgs &a, int *itersOut,
                       float *resOut) {

@@ -156,7 +156,7 @@ struct CGRing {
 struct CGState {
   double sigma;     // z . r of the current iterate
   double alpha;     // sigma / (p . A p)
-  double beta;      // sigmaNew / sigma
+  double beta;      // the next sigma, as predicted, / sigma
   double acc;       // accuracy * max(r0)
   double resIni;    // max(r0)
   double pAp;

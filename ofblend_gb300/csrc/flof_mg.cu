@@ -839,10 +839,10 @@ void launch_mg_build(const float4 *g, Dims4 d, const MGLevelPtrs *L, int nl, con
                      const MGParams &mp, const CGState *st, cudaStream_t s) {
   if (nl <= 0) return;
   launch_pdl(k_mg_build1, grid_for(L[0].m.cells(), MT, 8), MT, s, g, d, L[0].m, L[0].G, L[0].cpl,
-            L[0].dinv, c.wSmooth, c.wEnergy, mp.lambda, st);
+             L[0].dinv, c.wSmooth, c.wEnergy, mp.lambda, st);
   for (int l = 1; l < nl; ++l)
     launch_pdl(k_mg_build, grid_for(L[l].m.cells(), MT, 8), MT, s, L[l - 1].G, L[l - 1].cpl,
-              L[l - 1].m, L[l].m, L[l].G, L[l].cpl, L[l].dinv, mp.lambda, st);
+               L[l - 1].m, L[l].m, L[l].G, L[l].cpl, L[l].dinv, mp.lambda, st);
 }
 
 void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0, float4 *z, Dims4 d,
@@ -859,7 +859,7 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
   }
   if (nl == 0) {
     launch_pdl(k_mg0_post, nb0, MT, s, b0, g, x0, z, d, bx, nint, c0, wS, mp.omega0, st, dpart,
-              init);
+               init);
     if (launches) *launches += nl_;  // the caller counts one
     return;
   }
@@ -868,7 +868,7 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
     const int tchunks = (L[0].m.t + RR_TP - 1) / RR_TP;
     const long long nblk = (long long)nbx * L[0].m.y * L[0].m.z * tchunks;
     launch_pdl(k_mg0_resid_restrict, (unsigned)nblk, RR_NT, s, b0, g, x0, L[0].b, d, L[0].m, nbx,
-              c0, wS, st);
+               c0, wS, st);
     ++nl_;
   }
   for (int l = 0; l + 1 < nl; ++l) {
@@ -877,19 +877,19 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
     launch_pdl(k_mgc_pre, nb, MT, s, L[l].b, L[l].dinv, L[l].x, n, mp.omegac, st);
     launch_pdl(k_mgc_resid, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].x, L[l].r, L[l].m, st);
     launch_pdl(k_mgc_restrict, grid_for(L[l + 1].m.cells(), MT, 8), MT, s, L[l].r, L[l + 1].b,
-              L[l].m, L[l + 1].m, st);
+               L[l].m, L[l + 1].m, st);
     nl_ += 3;
   }
   const MGLevelPtrs &B = L[nl - 1];
   launch_pdl(k_mgc_coarsest, 1, MG_COARSEST, s, B.b, B.G, B.cpl, B.dinv, B.x, B.m, mp.omegac,
-            mp.coarse_sweeps, st);
+             mp.coarse_sweeps, st);
   ++nl_;
   for (int l = nl - 2; l >= 0; --l) {
     const uint32_t n = (uint32_t)L[l].m.cells();
     const int nb = grid_for(n, MT, 8);
     launch_pdl(k_mgc_prolong, nb, MT, s, L[l].x, L[l + 1].x, L[l].m, L[l + 1].m, st);
     launch_pdl(k_mgc_post, nb, MT, s, L[l].b, L[l].G, L[l].cpl, L[l].dinv, L[l].x, L[l].r, L[l].m,
-              mp.omegac, st);
+               mp.omegac, st);
     // the post-smoothed iterate is in r; it becomes this level's x
     std::swap(L[l].x, L[l].r);
     nl_ += 2;
@@ -900,7 +900,7 @@ void launch_mg_vcycle(const float4 *b0, const float4 *g, float4 *x0, float4 *r0,
     const int tchunks = (d.t - 2 + MG_TT - 1) / MG_TT;
     launch_pdl(k_mg0_prolong, nb0, MT, s, x0, L[0].x, d, bx, nint, L[0].m, st);
     launch_pdl(k_mg0_post_tw, grid_for((long long)nxyz * tchunks, MT, 8), MT, s, b0, g, x0, z, d,
-              bxyz, nxyz, tchunks, c0, wS, mp.omega0, st, dpart, init);
+               bxyz, nxyz, tchunks, c0, wS, mp.omega0, st, dpart, init);
     nl_ += 2;
   }
   if (launches) *launches += nl_ - 1;  // the caller counts one
@@ -910,7 +910,7 @@ void launch_mgcg_update(float4 *x, float4 *r, const float4 *p, const float4 *q, 
                         CGState *st, float *fpart, int maxIter, cudaStream_t s) {
   const uint32_t nint = interior_n(d);
   launch_pdl(k_mgcg_update, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, r, p, q, d,
-            interior_box(d), nint, st, fpart, maxIter);
+             interior_box(d), nint, st, fpart, maxIter);
 }
 void launch_mgcg_update_pre(float4 *x, float4 *r, const float4 *p, const float4 *q,
                             const float4 *g, const float *i1, float4 *x0, Dims4 d,
@@ -920,11 +920,11 @@ void launch_mgcg_update_pre(float4 *x, float4 *r, const float4 *p, const float4 
   const int nb = grid_for(nint > 0 ? nint : 1, MT, 8);
   if (i1)
     launch_pdl(k_mgcg_update_pre<GradFromI1>, nb, MT, s, x, r, p, q,
-              GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, x0, d, interior_box(d), nint, c.diag,
-              mp.omega0, st, fpart, maxIter);
+               GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, x0, d, interior_box(d), nint, c.diag,
+               mp.omega0, st, fpart, maxIter);
   else
     launch_pdl(k_mgcg_update_pre<GradLoad>, nb, MT, s, x, r, p, q, GradLoad{g}, x0, d,
-              interior_box(d), nint, c.diag, mp.omega0, st, fpart, maxIter);
+               interior_box(d), nint, c.diag, mp.omega0, st, fpart, maxIter);
 }
 
 void launch_mg_judge(const float4 *x, const float4 *b, const float4 *g, float4 *r, Dims4 d,
@@ -932,14 +932,14 @@ void launch_mg_judge(const float4 *x, const float4 *b, const float4 *g, float4 *
                      cudaStream_t s) {
   const uint32_t nint = interior_n(d);
   launch_pdl(k_mg_judge, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, x, b, g, r, d, interior_box(d),
-            nint, c.diag, c.wSmooth, fpart, counter, rmax);
+             nint, c.diag, c.wSmooth, fpart, counter, rmax);
 }
 
 void launch_mgcg_direction(float4 *p, const float4 *z, Dims4 d, const CGState *st, int init,
                            cudaStream_t s) {
   const uint32_t nint = interior_n(d);
   launch_pdl(k_mgcg_direction, grid_for(nint > 0 ? nint : 1, MT, 8), MT, s, p, z, d, interior_box(d),
-            nint, st, init);
+             nint, st, init);
 }
 
 // ---------------------------------------------------------------------------

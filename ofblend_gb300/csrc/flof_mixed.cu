@@ -1,7 +1,7 @@
 // flof_mixed.cu -- the mixed-precision solve's own kernels.
 //
 // In mixed precision the PCG iterates on a matrix built from the image
-// gradient stored in BF16 (8 bytes per cell instead of 16, read by all three
+// gradient stored in BF16 (8 bytes per cell instead of 16, read by both
 // PCG kernels), with FP32 vectors and float-float dot products.  Mixed-
 // precision iterative refinement then restores the FP32 system: the
 // residual r = b - A x of the FP32 matrix is formed with FP64 row sums, the

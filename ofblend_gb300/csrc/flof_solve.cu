@@ -173,18 +173,18 @@ void launch_of_assemble_init(const float *i0w, const float *i1,
 // consecutive t planes, keeping p at t-1, t and t+1 in registers, so the -t
 // and +t terms cost no extra load, and loading the next plane's operands
 // while it computes the current one.  A work item is (run of MV_RUN cells of
-// the interior (x,y) plane, MV_ZB planes z, t chunk) with the (x,y) run fastest, so the
-// blocks resident at one time cover neighbouring z at the same t chunk and
-// the z-neighbour loads hit L2.  The grid is persistent (a fixed number of
+// the interior (x,y) plane, MV_ZB planes z, t chunk) with the (x,y) run
+// fastest, so the blocks resident at one time cover neighbouring z at the same
+// t chunk and the z-neighbour loads hit L2.  The grid is persistent (a fixed number of
 // blocks per SM); p.Ap is accumulated per thread in float-float and summed
 // in double by the last block to finish, in a fixed order.
 //
 // MV_DOTS (the plain PCG): the kernel also forms q.M^-1 q, from which its last
 // block predicts the next z.r, and so beta, before r is updated (cg_scalars).
 // The step kernel then has alpha and beta and updates r and p in one pass.
-// The extra sum costs 6 us of 148 at 64^4.  The loads need the 1024 threads per
-// SM that 64 registers allow: at 105 registers it takes 186 us.  Two z planes a block share their z neighbours
-// in L1 (148 -> 146 us at 64^4, 59 -> 57 at 48^4; four planes 150 and 61, rows of
+// The extra sum costs 8 us of 144 at 64^4.  The loads need the 1024 threads per
+// SM that 64 registers allow: at 105 registers it takes 186 us.  Two z planes a
+// block share their z neighbours in L1 (148 -> 146 us at 64^4, 59 -> 57 at 48^4; four planes 150 and 61, rows of
 // 256 cells 152 and 59), the fused rows take 146 -> 142 and 57 -> 56 and halve
 // the rounding (the 64^4 deformation against 64 bits 7.5e-7 -> 4.8e-7).  Each
 // product of q.M^-1 q enters the float-float sum by itself, like those of every
@@ -472,7 +472,8 @@ struct GradStored {
 };
 
 // r -= alpha q; z = M^-1 r; the next p = z + beta p; sigma' = z.r; max(r); and
-// in every CG_RING-th step x += the last CG_RING alpha p, added in order.
+// in every CG_RING-th step x += the sum of the last CG_RING alpha p, formed from
+// the newest to the oldest.
 //
 // Bound by HBM: q, r and p read, r and p written, i1 for g (84 bytes a cell),
 // and x.  Adding to x in every step reads and writes it each time (32 bytes);
