@@ -319,8 +319,8 @@ CGTune cg_tune(flof_ctx *c, Dims4 d, const OFConsts &k) {
     CGTune cand = best;
     cand.per_sm = ps;
     const float ms = time_it([&] {
-      for (int slot = 0; slot < CG_RING; ++slot)
-        launch_cg_step(x.v(), r.v(), q.v(), ring, slot, g.v(), nullptr, d, k, st, c->dpart,
+      for (int m = 0; m < CG_RING; ++m)  // past the first pass over the ring
+        launch_cg_step(x.v(), r.v(), q.v(), ring, CG_RING + m, g.v(), nullptr, d, k, st, c->dpart,
                        c->fpart, 1 << 30, c->stream, cand);
     });
     if (ms < bt) {
@@ -347,11 +347,7 @@ void make_ring(flof_ctx *c, Dims4 d, float4 *p, CGRing &ring, DBuf *more) {
     for (int m = 1; m < CG_RING; ++m) more[m].release();
     ring.n = 1;
   }
-  for (int m = 1; m < CG_RING; ++m) {
-    ring.p[m] = ring.n > 1 ? more[m].v() : p;
-    if (ring.n > 1)  // the border rows
-      CK(cudaMemsetAsync(ring.p[m], 0, vec_bytes(d), c->stream));
-  }
+  for (int m = 1; m < CG_RING; ++m) ring.p[m] = ring.n > 1 ? more[m].v() : p;
 }
 
 // PCG iterations (GridCGOptflow4d::solve, optflow4d.cpp:304-326) from the
@@ -391,7 +387,10 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
   }
   CGRing ring;
   DBuf more[CG_RING];
-  make_ring(c, d, p, ring, more);
+  if (maxIter > 0)
+    make_ring(c, d, p, ring, more);
+  else
+    ring.n = 1;  // no iteration
   int it = 0;
   int chunk = 4;
   for (;;) {
@@ -401,7 +400,7 @@ void pcg_loop(flof_ctx *c, Dims4 d, const OFConsts &k, const CGTune &tu, float4 
       KLP(c, KC_MATVEC, d.x, nint(d) * (32 + gb),
           launch_cg_matvec(ring.p[slot], g, q, d, k, c->st, c->dpart, slot, c->stream, tu));
       KLP(c, KC_STEP, d.x, nint(d) * (80 + gpc + (slot == ring.n - 1 ? 16 * (ring.n + 1) : 0)),
-          launch_cg_step(x, r, q, ring, slot, g, i1, d, k, c->st, c->dpart, c->fpart, maxIter,
+          launch_cg_step(x, r, q, ring, it + s, g, i1, d, k, c->st, c->dpart, c->fpart, maxIter,
                          c->stream, tu));
     }
     it += n;

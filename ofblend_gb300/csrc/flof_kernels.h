@@ -212,8 +212,9 @@ void launch_strict_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, 
 // One iteration of the plain PCG is launch_cg_matvec and launch_cg_step with
 // slot = iteration % ring.n.  The matvec reads ring.p[slot] and forms alpha and
 // beta; the step updates r, writes the next direction to the ring's next
-// buffer, and in the last slot adds the ring's directions to x.  launch_cg_flush
-// adds what is left when the solve ends in another slot.
+// buffer (whose border rows the first pass over the ring zeroes), and in the
+// last slot adds the ring's directions to x.  launch_cg_flush adds what is left
+// when the solve ends in another slot.
 // With i1 (the level's target level set, from which the assembly built g)
 // the step rebuilds g from it instead of reading g.  g in BF16: mixed
 // precision (the matrix g g^T + diag I is built from the rounded gradient).
@@ -221,10 +222,10 @@ void launch_cg_matvec(const float4 *p, const float4 *g, float4 *q, Dims4 d, OFCo
                       CGState *st, double *dpart, int slot, cudaStream_t s, const CGTune &tu);
 void launch_cg_matvec(const float4 *p, const BF4 *g, float4 *q, Dims4 d, OFConsts c, CGState *st,
                       double *dpart, int slot, cudaStream_t s, const CGTune &tu);
-void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int iter,
                     const float4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st,
                     double *dpart, float *fpart, int maxIter, cudaStream_t s, const CGTune &tu);
-void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int iter,
                     const BF4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st, double *dpart,
                     float *fpart, int maxIter, cudaStream_t s, const CGTune &tu);
 void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState *st,

@@ -494,6 +494,10 @@ struct GradStored {
 // NX: the directions that this step adds to x.  Where memory for a ring is
 // short there is one buffer, pin = pout, and every step adds its own (NX = 1);
 // a cell is read before it is written, by the same thread.
+// FILL: pout is used for the first time in this solve, and the step zeroes its
+// border rows too (an eighth of the cells at 64^4, 12 us; clearing the ring's
+// three buffers before the first iteration took 120 us, which a solve of one or
+// two iterations felt).
 __device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
   x.x = __fmaf_rn(a, p.x, x.x);
   x.y = __fmaf_rn(a, p.y, x.y);
@@ -501,14 +505,30 @@ __device__ __forceinline__ void axpy4(float4 &x, float a, const float4 p) {
   x.w = __fmaf_rn(a, p.w, x.w);
 }
 
-template <int NX, class GS>
+template <int NX, bool FILL, class GS>
 __global__ void __launch_bounds__(NT)
 k_cg_step(float4 *__restrict__ x, float4 *__restrict__ r, const float4 *__restrict__ q,
           CGRing ring, const float4 *pin, float4 *pout, GS gs, Dims4 d, BoxDecoder bx,
-          uint32_t nint, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter) {
+          BoxDecoder rows, uint32_t nint, OFConsts c, CGState *st, double *dpart, float *fpart,
+          int maxIter) {
   pdl_wait();
   pdl_launch_dependents();
   if (st->done) return;
+  if (FILL) {  // a warp per x row
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int lane = threadIdx.x & 31;
+    const uint32_t n = (uint32_t)d.y * d.z * d.t, warps = gridDim.x * (NT / 32);
+    for (uint32_t w = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); w < n; w += warps) {
+      int j, k, l, unused;
+      rows.decode(w, j, k, l, unused);
+      float4 *const row = pout + (idx_t)d.x * w;
+      if (j < 1 || j >= d.y - 1 || k < 1 || k >= d.z - 1 || l < 1 || l >= d.t - 1) {
+        for (int i = lane; i < d.x; i += 32) row[i] = zero;
+      } else if (lane < 2) {
+        row[lane ? d.x - 1 : 0] = zero;
+      }
+    }
+  }
   __shared__ double shd[NT / 32];
   __shared__ FF shff[NT / 32];
   __shared__ float shf[NT / 32];
@@ -642,40 +662,44 @@ int resident_per_sm(K kernel, int want) {
   return want < n ? want : n;
 }
 
-template <int NX, class GS>
+template <int NX, bool FILL, class GS>
 void step_launch(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs,
                  Dims4 d, OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter,
                  cudaStream_t s, const CGTune &tu) {
-  static const int occ = resident_per_sm(k_cg_step<NX, GS>, 1 << 30);
+  static const int occ = resident_per_sm(k_cg_step<NX, FILL, GS>, 1 << 30);
   const long long n = interior_count(d);
-  launch_pdl(k_cg_step<NX, GS>, grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ),
-             NT, s, x, r, q, ring, (const float4 *)ring.p[slot], ring.p[NX > 0 ? 0 : slot + 1], gs, d,
-             interior_decoder(d), (uint32_t)n, c, st, dpart, fpart, maxIter);
+  launch_pdl(k_cg_step<NX, FILL, GS>,
+             grid_for(n > 0 ? n : 1, NT, tu.per_sm < occ ? tu.per_sm : occ), NT, s, x, r, q, ring,
+             (const float4 *)ring.p[slot], ring.p[NX > 0 ? 0 : slot + 1], gs, d, interior_decoder(d),
+             make_decoder(d.y, d.z, d.t, 0, 0, 0, 0), (uint32_t)n, c, st, dpart, fpart, maxIter);
 }
 template <class GS>
-void step_any(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot, GS gs, Dims4 d,
+void step_any(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int iter, GS gs, Dims4 d,
               OFConsts c, CGState *st, double *dpart, float *fpart, int maxIter, cudaStream_t s,
               const CGTune &tu) {
+  const int slot = iter % ring.n;
   if (ring.n == 1)
-    step_launch<1>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_launch<1, false>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
   else if (slot == CG_RING - 1)
-    step_launch<CG_RING>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_launch<CG_RING, false>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+  else if (iter < CG_RING - 1)
+    step_launch<0, true>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
   else
-    step_launch<0>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_launch<0, false>(x, r, q, ring, slot, gs, d, c, st, dpart, fpart, maxIter, s, tu);
 }
-void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int iter,
                     const float4 *g, const float *i1, Dims4 d, OFConsts c, CGState *st,
                     double *dpart, float *fpart, int maxIter, cudaStream_t s, const CGTune &tu) {
   if (i1)
-    step_any(x, r, q, ring, slot, GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, d, c, st, dpart,
+    step_any(x, r, q, ring, iter, GradFromI1{i1, d.x, d.sz(), d.st(), c.dxf}, d, c, st, dpart,
              fpart, maxIter, s, tu);
   else
-    step_any(x, r, q, ring, slot, GradStored<float4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
+    step_any(x, r, q, ring, iter, GradStored<float4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
 }
-void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int slot,
+void launch_cg_step(float4 *x, float4 *r, const float4 *q, const CGRing &ring, int iter,
                     const BF4 *g, const float *, Dims4 d, OFConsts c, CGState *st, double *dpart,
                     float *fpart, int maxIter, cudaStream_t s, const CGTune &tu) {
-  step_any(x, r, q, ring, slot, GradStored<BF4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
+  step_any(x, r, q, ring, iter, GradStored<BF4>{g}, d, c, st, dpart, fpart, maxIter, s, tu);
 }
 void launch_cg_flush(float4 *x, const CGRing &ring, int count, Dims4 d, CGState *st,
                      cudaStream_t s) {

@@ -80,7 +80,7 @@ int main() {
     for (int it = 0; it < (k < 8 ? 6 : 2); ++it) {
       const double before = h.sigma;
       launch_cg_matvec(ring.p[it % CG_RING], g, q, d, c, st, dpart, it % CG_RING, 0, CGTune());
-      launch_cg_step(x, r, q, ring, it % CG_RING, g, i1, d, c, st, dpart, fpart, 1 << 30, 0, CGTune());
+      launch_cg_step(x, r, q, ring, it, g, i1, d, c, st, dpart, fpart, 1 << 30, 0, CGTune());
       OK(cudaMemcpy(&h, st, sizeof(h), cudaMemcpyDeviceToHost));
       const double want = h.sigma / before;
       // Four sums of 4 x cells products, together 5 (1 + beta) z.r, whose two or
